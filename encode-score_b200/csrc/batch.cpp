@@ -52,7 +52,6 @@ struct Picture {
     int source = 0, encode = -1;  // encode -1: the source's own picture
     int w = 0, h = 0, depth = 10;
     int tile_rows[kScales] = {64, 64, 64, 64, 64};  // c-value tile rows per scale
-    int tile_cols[kScales] = {64, 64, 64, 64, 64};  // c-value tile columns per scale
     float *cv_plane[kScales] = {};                   // optional: every computed c-value at its pixel (tests)
     es_cambi_params p{};
     int sw[kScales], sh[kScales];
@@ -185,6 +184,8 @@ void init_cambi(es_batch &b)
     std::vector<unsigned long long> n(P * kScales), k(P * kScales);
     std::vector<CvSlot> init(P * kScales);
     std::memset(init.data(), 0, sizeof(CvSlot) * init.size());
+    int tiles0 = 0;
+    for (auto &pic : b.pictures) tiles0 += cv_tiles(pic->w, pic->h);
     for (int i = 0; i < P; i++) {
         Picture &pic = *b.pictures[i];
         pic.sw[0] = pic.w;
@@ -194,6 +195,7 @@ void init_cambi(es_batch &b)
             pic.sh[s] = (pic.sh[s - 1] + 1) >> 1;
         }
         for (int s = 0; s < kScales; s++) {
+            if (!pic.tile_rows[s]) pic.tile_rows[s] = cv_default_tile_rows(pic.sw[s], pic.sh[s], tiles0);
             const size_t m = (size_t)pic.sw[s] * pic.sh[s];
             pic.words[s].reset(m);
             pic.lists[s].reset(m);
@@ -399,8 +401,7 @@ void record_cambi(es_batch &b, long f, uint32_t skip, cudaStream_t s)
             j.w = pic.sw[sc];
             j.h = pic.sh[sc];
             j.pad = pic.p.pad;
-            j.tile_cols = b.net ? kCvTX : pic.tile_cols[sc];  // the proposal maps 64-column tiles
-            j.tiles_x = (j.w + j.tile_cols - 1) / j.tile_cols;
+            j.tiles_x = (j.w + kCvTX - 1) / kCvTX;
             j.first_tile = tiles;
             j.slot = i * kScales + sc;
             j.plane = pic.cv_plane[sc];
@@ -692,10 +693,9 @@ int es_batch_create(const es_module *m, int n_sources, const es_batch_source *so
                 for (int sc = 0; sc < kScales; sc++) {
                     const int r = sources[i].cv_tile_rows[sc];
                     require(r == 0 || r == 16 || r == 32 || r == 64, "es_batch_create: c-value tile rows must be 0, 16, 32 or 64");
-                    pic->tile_rows[sc] = r ? r : 64;
+                    pic->tile_rows[sc] = r;  // 0: chosen once every picture is known
                     const int c = sources[i].cv_tile_cols[sc];
                     require(c == 0 || c == 64 || c == 128, "es_batch_create: c-value tile columns must be 0, 64 or 128");
-                    pic->tile_cols[sc] = c ? c : cv_default_tile_cols(sc);
                 }
                 b->pictures.push_back(std::move(pic));
             }

@@ -120,12 +120,12 @@ void queue_cambi(es_cambi *c, uint64_t img, int pitch, cudaStream_t caller)
         j.w = c->sw[sc];
         j.h = c->sh[sc];
         j.pad = p.pad;
-        j.tile_cols = c->tile_mass ? kCvTX : cv_default_tile_cols(sc);  // per-tile masses are counted on 64 x 64 tiles
-        j.tiles_x = (j.w + j.tile_cols - 1) / j.tile_cols;
+        j.tiles_x = (j.w + kCvTX - 1) / kCvTX;
         j.first_tile = tiles;
         j.slot = sc;
         j.plane = c->planes[sc];
-        tiles += j.tiles_x * ((j.h + kCvTY - 1) / kCvTY);
+        j.tile_rows = c->tile_mass ? kCvTY : cv_default_tile_rows(j.w, j.h, cv_tiles(c->w, c->h));  // per-tile masses are counted on 64 x 64 tiles
+        tiles += j.tiles_x * ((j.h + j.tile_rows - 1) / j.tile_rows);
     }
     cb.total_tiles = tiles;
     cb.max_pad = p.pad;

@@ -116,11 +116,11 @@ cudaError_t launch_decimate_mode(DecBatch &b, cudaStream_t s);
 constexpr unsigned kCvDigit0 = 0x3F000000u >> 21, kCvDigits = 64;
 struct CvSlot {
     unsigned long long sum_fx, count;  // positive c-values: sum in 2^-24 units, number
-    unsigned long long list_n;         // values appended to `list`
+    unsigned long long list_n;         // values in `list`
     unsigned long long n, k;           // pixels of the scale, top-k count
     unsigned long long remaining, above_fx, above_n;
     unsigned prefix, mask;             // radix select state
-    float *list;                       // positive c-values (capacity n)
+    float *list;                       // c-values, zeros among them (capacity n): every positive one is there once
     unsigned hist[2048];               // counts of the current radix digit
     unsigned long long dsum[1024];     // last round: sums (2^-24 units) of the values of each last digit
 };
@@ -133,7 +133,6 @@ struct CvJob {
     float *plane;   // optional: every computed c-value at its pixel
     int run_index;  // the entry of CvBatch::run that gates this job (with a run table)
     int tile_rows;  // rows of this job's tiles: 64 (0 means 64), 32 or 16; tiles are numbered row by row
-    int tile_cols;  // columns of this job's tiles: 64 (0 means 64) or 128 (tiles_x counts tiles of this width)
 };
 struct CvBatch {
     CvJob job[kMaxJobs];
@@ -153,13 +152,23 @@ struct CvBatch {
     int need_lo, need_span;  // set by the launcher: as Prep0Batch's
 };
 // Blocks of a tile-list launch.
-constexpr int kCvListBlocks = 148 * 4;
+constexpr int kCvListBlocks = 148 * 3;
 constexpr int kCvTX = 64, kCvTY = 64, kCvThreads = 256, kCvBins = 32;
-size_t cvalues_smem_bytes(int max_pad, int tile_cols);
-// The c-value tile width of a scale when nothing else asks for one: 64 columns (128-column tiles stage less margin per
-// output pixel, but two 512-thread blocks per SM measured slower than four 256-thread ones at every scale of a 4K
-// picture; the autotuner may still pick them).
-inline int cv_default_tile_cols(int /*scale*/) { return 64; }
+size_t cvalues_smem_bytes(int max_pad);
+// 64 x 64 c-value tiles of a w x h scale.
+inline int cv_tiles(int w, int h) { return ((w + kCvTX - 1) / kCvTX) * ((h + kCvTY - 1) / kCvTY); }
+// The tile rows of a w x h scale when nothing else asks for a height; tiles0: the launch's 64 x 64 tiles of scale 0, all
+// pictures. Short tiles cost more in all (the window margins are staged and counted again for fewer rows) but a block is
+// done sooner, which decides where the tiles do not fill the chip's 444 places or hold many ranks (several passes),
+// as the small scales' do. Measured, c-values of one picture, 64 rows everywhere / by this rule: 640x360 8-bit 55 / 24
+// us, 1920x1080 8-bit 96 / 57 us, 3840x2160 10-bit 190 / 108 us; 32 rows for scale 1 of a dense 4K picture instead of 64:
+// 260 against 247 us, 64 rows for scale 0 of the 1080p one instead of 32: 69 against 57 us.
+inline int cv_default_tile_rows(int w, int h, int tiles0)
+{
+    const int tiles = cv_tiles(w, h);
+    if (tiles0 >= 592) return tiles >= 148 ? 64 : tiles >= 74 ? 32 : 16;
+    return tiles >= 148 ? 32 : 16;
+}
 cudaError_t launch_cvalues(const CvBatch &b, cudaStream_t s);
 
 // ---- top-k pooling and score -------------------------------------------------------------------------------------

@@ -164,12 +164,12 @@ extern "C" int es_cambi_score_noalloc(uint64_t img, int pitch, int w, int h, int
             j.w = c.sw[k];
             j.h = c.sh[k];
             j.pad = p.pad;
-            j.tile_cols = cv_default_tile_cols(k);
-            j.tiles_x = (j.w + j.tile_cols - 1) / j.tile_cols;
+            j.tiles_x = (j.w + kCvTX - 1) / kCvTX;
             j.first_tile = tiles;
             j.slot = k;
             j.plane = nullptr;
-            tiles += j.tiles_x * ((j.h + kCvTY - 1) / kCvTY);
+            j.tile_rows = cv_default_tile_rows(j.w, j.h, cv_tiles(w, h));
+            tiles += j.tiles_x * ((j.h + j.tile_rows - 1) / j.tile_rows);
         }
         cb.total_tiles = tiles;
         cb.max_pad = p.pad;

@@ -523,7 +523,7 @@ AUTOTUNE_PATH = os.path.join(HERE, "autotune.json")
 
 def autotune_table(path: str = AUTOTUNE_PATH) -> dict:
     """{(w, h): {"rows": c-value tile rows per scale, "cols": tile columns per scale}} from the autotuner's table
-    (empty when there is none; columns 0 where the table has none, the library's default)."""
+    (empty when there is none; columns 0 where the table has none: they make no difference)."""
     import json
     try:
         with open(path) as f:
@@ -540,9 +540,9 @@ def autotune_table(path: str = AUTOTUNE_PATH) -> dict:
 def _tile_shape(entry) -> tuple:
     """(rows, cols) per scale from a tuning entry: a list of rows, or a dict with "rows" and optionally "cols"."""
     if entry is None:
-        return [64] * 5, [0] * 5
+        return [0] * 5, [0] * 5
     if isinstance(entry, dict):
-        return list(entry.get("rows", [64] * 5)), list(entry.get("cols", [0] * 5))
+        return list(entry.get("rows", [0] * 5)), list(entry.get("cols", [0] * 5))
     return list(entry), [0] * 5
 
 
@@ -551,7 +551,7 @@ class Batch:
     frame 14 on. ``sources`` is a list of (w, h, pd, n_encodes); pictures and encodes are numbered source by source.
     ``tuning``: None for the autotuned c-value tile shapes of autotune.json (by picture size; the library's defaults
     where absent), False for the defaults everywhere, or a dict {(w, h): rows per scale, or {"rows": [...], "cols":
-    [...]}} (cols 0: the library's default width)."""
+    [...]}} (rows 0: the library's choice; cols, 0, 64 or 128, make no difference)."""
 
     def __init__(self, module: Module, sources: list, use_graphs: bool = True, tuning=None):
         self.handle = ctypes.c_void_p()

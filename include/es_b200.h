@@ -309,10 +309,9 @@ typedef struct {
     int w, h;      /* common picture area of the source and its encodes (even) */
     int pd;        /* pipeline depth, 8 or 10 */
     int n_encodes; /* 1 to 16 */
-    int cv_tile_rows[5]; /* rows of the c-value tiles per scale: 64, 32 or 16 (0 = 64); an autotuner's choice. With
-                          * the learned proposal on, scales 0 and 1 use 64. */
-    int cv_tile_cols[5]; /* columns of the c-value tiles per scale: 64 or 128 (0 = 64);
-                          * an autotuner's choice. With the learned proposal on, every scale uses 64. */
+    int cv_tile_rows[5]; /* rows of the c-value tiles per scale: 64, 32 or 16 (0 = chosen by the scale's size); an
+                          * autotuner's choice. With the learned proposal on, scales 0 and 1 use 64. */
+    int cv_tile_cols[5]; /* 64, 128 or 0, which are the same: the c-value tiles are 64 columns wide */
 } es_batch_source;
 typedef struct {
     int use_graphs; /* replay steps from CUDA graphs once the rings are full (frame 14 on) */
