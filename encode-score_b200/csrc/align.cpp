@@ -1,6 +1,6 @@
 // es_thumbnails / es_offset_totals / es_find_offset: the offset search between a source and an encode that start at
 // different points (src/main.cpp:301-353 with its tiny_luma kernel, src/kernels.cu:502-520).
-#include <cstring>
+#include <atomic>
 #include <string>
 #include <vector>
 
@@ -18,6 +18,49 @@ void check_luma_view(const es_frame_view &v)
     require(v.shift >= 0 && v.shift < 16, "es_thumbnails: bad shift");
     require(v.ypitch >= v.bytes, "es_thumbnails: bad pitch");
 }
+
+// Device memory for one search's totals. A slot of the library's fixed array is taken where one is free (allocating and
+// freeing cost 0.7 ms a call, several times the search); its address is looked up in the current context every time, so
+// nothing is kept across contexts or device resets. Searches with more lags, or beside 8 others, allocate.
+class TotalsBuffer {
+    static std::atomic<unsigned> taken;  // bit per slot
+    int slot = -1;
+    DeviceBuffer<double> own;
+    cudaStream_t stream;
+
+public:
+    double *ptr = nullptr;
+    bool settled = false;  // the stream has been waited for since the buffer was used
+    TotalsBuffer(int lags, cudaStream_t s) : stream(s)
+    {
+        if (lags <= offset_totals_slot_lags()) {
+            unsigned t = taken.load(std::memory_order_relaxed);
+            for (int i = 0; i < offset_totals_slots() && slot < 0;) {
+                if (t & (1u << i)) i++;
+                else if (taken.compare_exchange_weak(t, t | (1u << i), std::memory_order_acquire)) slot = i;
+            }
+        }
+        if (slot >= 0) {
+            const cudaError_t e = offset_totals_slot(slot, &ptr);
+            if (e != cudaSuccess) release();
+            cuda_check(e, "finding the totals array");
+        } else {
+            own.reset(lags);
+            ptr = own.ptr;
+        }
+    }
+    ~TotalsBuffer()
+    {
+        if (!settled) cudaStreamSynchronize(stream);  // a failed call may have left work that writes the buffer
+        release();
+    }
+    void release()
+    {
+        if (slot >= 0) taken.fetch_and(~(1u << slot), std::memory_order_release);
+        slot = -1;
+    }
+};
+std::atomic<unsigned> TotalsBuffer::taken{0};
 
 }  // namespace
 
@@ -65,8 +108,7 @@ int es_offset_totals(uint64_t ref, int n_ref, uint64_t probe, int n_probe, uint6
         require(ref != 0 && probe != 0 && totals != 0, "es_offset_totals: NULL argument");
         require(n_probe > 0 && n_ref >= n_probe, "es_offset_totals: needs 1 <= n_probe <= n_ref");
         check_device();
-        cuda_check(launch_offset_totals((const float *)ref, (const float *)probe, n_probe, n_ref - n_probe + 1, (double *)totals,
-                                        (cudaStream_t)stream),
+        cuda_check(launch_offset_totals((const float *)ref, n_ref, (const float *)probe, n_probe, (double *)totals, (cudaStream_t)stream),
                    "offset totals");
     });
 }
@@ -82,11 +124,14 @@ int es_find_offset(uint64_t ref, const double *ref_times, int n_ref, uint64_t pr
         check_device();
         const cudaStream_t s = (cudaStream_t)stream;
         const int lags = n_ref - n_probe + 1;
-        DeviceBuffer<double> d_totals(lags);
         std::vector<double> totals(lags);
-        cuda_check(launch_offset_totals((const float *)ref, (const float *)probe, n_probe, lags, d_totals.ptr, s), "offset totals");
-        cuda_check(cudaMemcpyAsync(totals.data(), d_totals.ptr, lags * sizeof(double), cudaMemcpyDeviceToHost, s), "reading totals");
-        cuda_check(cudaStreamSynchronize(s), "offset totals");
+        {
+            TotalsBuffer d_totals(lags, s);
+            cuda_check(launch_offset_totals((const float *)ref, n_ref, (const float *)probe, n_probe, d_totals.ptr, s), "offset totals");
+            cuda_check(cudaMemcpyAsync(totals.data(), d_totals.ptr, lags * sizeof(double), cudaMemcpyDeviceToHost, s), "reading totals");
+            cuda_check(cudaStreamSynchronize(s), "offset totals");
+            d_totals.settled = true;
+        }
         // src/main.cpp:340-348: the first lag of least mean. The reference stops adding a lag's differences once its
         // partial total reaches the best lag's total; such a lag is not chosen there, nor here with its full total.
         double best = 1e30;

@@ -4,8 +4,8 @@
 // The reference (src/kernels.cu:502-520, src/main.cpp:301-353) launches tiny_luma once per decoded frame, copies
 // each 64 x 36 thumbnail to the host with a stream synchronisation, and searches the lags on the CPU. Here one launch
 // makes the thumbnails of a whole batch of frames (one block per cell and frame), each cell's sum is an exact integer
-// divided once, and the lags are searched on the device, one thread per lag, adding the differences in the same order
-// and arithmetic as the reference's loop so that the chosen lag is the same.
+// divided once, and the lags are searched on the device with totals that equal the reference's in-order double sums bit
+// for bit, so that the chosen lag is the same.
 #include "es_kernels.h"
 
 namespace es {
@@ -120,6 +120,94 @@ __global__ void __launch_bounds__(256) thumb_rows_kernel(const __grid_constant__
 // value the shifts cannot represent (an increment of 2^53 or more, an infinity or NaN) is added in order, one value at
 // a time, from shared memory. Adding zeros leaves s as it is, so a chunk of zeros and the padding of the last chunk
 // are skipped. The result equals the in-order double sum bit for bit.
+// Thumbnails of ordinary pictures need none of that: means of 8 code values or more have no bits below 2^-20, so every
+// difference is a whole number of those units below 2^30, and while the total stays below 2^53 of them every sum is
+// exact in any order. offset_check_kernel finds the frames with a value that is no whole number of units (or outside
+// [0, 1024), or NaN) and marks the lags that read them; offset_exact_kernel adds the differences of every lag as 64-bit
+// integers: a block takes 16 lags x 16 probe frames x 768 pixels, a thread one pixel at a time, 47 values in registers
+// for 256 differences (a float subtraction, a conversion and about one integer addition each). The loads bound it, 47
+// from L2 per 256 differences (conversions spread over other pipes changed nothing, sums in double were slower: 84
+// against 62 us); the in-order form issues about 40 instructions per difference and has one warp per lag. 483 lags of
+// 192 frames: 1027 us in order, 78 us for the three launches.
+constexpr double kFixed = 1048576.0;                     // units per code value
+constexpr unsigned long long kInexact = 1ull << 63;      // mark in a lag's integer sum
+constexpr int kExactMaxProbe = (1 << 23) / kThumbPixels;  // frames whose totals stay below 2^53 units
+constexpr int kExLags = 16, kExFrames = 16, kExThreads = 256, kExPixels = 768;
+static_assert(kThumbPixels % kExPixels == 0 && kExPixels % kExThreads == 0, "whole pixel chunks");
+
+__global__ void __launch_bounds__(kExThreads) offset_check_kernel(const float *ref, int n_ref, const float *probe, int n_probe, int lags,
+                                                                  unsigned long long *sums)
+{
+    const int f = blockIdx.x;
+    const float *v = f < n_ref ? ref + (size_t)f * kThumbPixels : probe + (size_t)(f - n_ref) * kThumbPixels;
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < kThumbPixels / kExThreads; i++) {
+        const float x = __ldg(v + i * kExThreads + threadIdx.x), u = __fmul_rn(x, (float)kFixed);
+        ok &= x >= 0.0f && x < 1024.0f && rintf(u) == u;
+    }
+    if (!__syncthreads_or(!ok)) return;
+    const int first = f < n_ref ? max(f - n_probe + 1, 0) : 0, last = f < n_ref ? min(f, lags - 1) : lags - 1;
+    for (int l = first + threadIdx.x; l <= last; l += kExThreads) atomicOr(sums + l, kInexact);
+}
+
+template <bool kWhole>
+__device__ __forceinline__ void exact_pixel(const float *r0, const float *p0, int n_frames, int n_lags, unsigned long long (&acc)[kExLags])
+{
+    float r[kExLags + kExFrames - 1], p[kExFrames];
+#pragma unroll
+    for (int j = 0; j < kExLags + kExFrames - 1; j++)
+        r[j] = kWhole || j < n_frames + n_lags - 1 ? __fmul_rn(__ldg(r0 + (size_t)j * kThumbPixels), (float)kFixed) : 0.0f;
+#pragma unroll
+    for (int i = 0; i < kExFrames; i++) p[i] = kWhole || i < n_frames ? __fmul_rn(__ldg(p0 + (size_t)i * kThumbPixels), (float)kFixed) : 0.0f;
+#pragma unroll
+    for (int l = 0; l < kExLags; l++) {
+#pragma unroll
+        for (int i = 0; i < kExFrames; i += 4) {
+            unsigned t = 0;  // four differences below 1023 2^20 + 2^20 each: below 2^32
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const unsigned d = __float2uint_rz(fabsf(__fsub_rn(r[l + i + k], p[i + k])));
+                if (kWhole || i + k < n_frames) t += d;
+            }
+            acc[l] += t;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kExThreads, 2) offset_exact_kernel(const float *ref, const float *probe, int n_probe, int lags,
+                                                                     unsigned long long *sums)
+{
+    __shared__ unsigned long long total[kExLags];
+    const int l0 = blockIdx.x * kExLags, i0 = blockIdx.y * kExFrames, lane = threadIdx.x & 31;
+    const int n_lags = min(kExLags, lags - l0), n_frames = min(kExFrames, n_probe - i0);
+    if (threadIdx.x < kExLags) total[threadIdx.x] = 0;
+    __syncthreads();
+    unsigned long long acc[kExLags];
+#pragma unroll
+    for (int l = 0; l < kExLags; l++) acc[l] = 0;
+    for (int c = 0; c < kExPixels; c += kExThreads) {
+        const int px = blockIdx.z * kExPixels + c + threadIdx.x;
+        const float *r0 = ref + (size_t)(l0 + i0) * kThumbPixels + px, *p0 = probe + (size_t)i0 * kThumbPixels + px;
+        if (n_lags == kExLags && n_frames == kExFrames) exact_pixel<true>(r0, p0, n_frames, n_lags, acc);
+        else exact_pixel<false>(r0, p0, n_frames, n_lags, acc);
+    }
+    // 16 sums over 32 lanes: each step halves the sums a lane holds and adds the other half lane's
+#pragma unroll
+    for (int n = kExLags / 2, off = 16; n >= 1; n >>= 1, off >>= 1) {
+        const bool upper = (lane & off) != 0;
+#pragma unroll
+        for (int k = 0; k < n; k++) {
+            const unsigned long long send = upper ? acc[k] : acc[k + n], keep = upper ? acc[k + n] : acc[k];
+            acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+    }
+    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+    if ((lane & 1) == 0) atomicAdd(&total[lane >> 1], acc[0]);
+    __syncthreads();
+    if ((int)threadIdx.x < n_lags) atomicAdd(sums + l0 + threadIdx.x, total[threadIdx.x]);
+}
+
 constexpr int kLaneVals = 16, kChunk = 32 * kLaneVals, kLagWarps = 4;
 
 struct ParityMap {
@@ -137,13 +225,23 @@ __device__ __forceinline__ ParityMap compose(const ParityMap &a, const ParityMap
     return r;
 }
 
+// With kSums, totals[] holds the exact kernels' integer sums: a lag they marked is added as above, any other becomes its
+// sum's double.
 template <bool kVec>
 __global__ void __launch_bounds__(32 * kLagWarps) offset_totals_kernel(const float *ref, const float *probe, int n_probe, int lags,
-                                                                      double *totals)
+                                                                      double *totals, int sums)
 {
     __shared__ __align__(16) double serial[kLagWarps][kChunk];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, l = blockIdx.x * kLagWarps + w;
     if (l >= lags) return;  // whole warps: one lag per warp
+    if (sums) {
+        const unsigned long long v = ((const unsigned long long *)totals)[l];
+        if (!(v & kInexact)) {
+            __syncwarp();
+            if (lane == 0) totals[l] = (double)v * (1.0 / kFixed);  // both exact
+            return;
+        }
+    }
     const float *r = ref + (size_t)l * kThumbPixels;
     const long long count = (long long)n_probe * kThumbPixels;
     const long long chunks = (count + kChunk - 1) / kChunk;
@@ -258,15 +356,48 @@ cudaError_t launch_thumbnails(const ThumbBatch &b, cudaStream_t s)
     return after_launch();
 }
 
-cudaError_t launch_offset_totals(const float *ref, const float *probe, int n_probe, int lags, double *totals, cudaStream_t s)
+cudaError_t launch_offset_totals(const float *ref, int n_ref, const float *probe, int n_probe, double *totals, cudaStream_t s)
 {
+    const int lags = n_ref - n_probe + 1;
     if (lags <= 0) return cudaSuccess;
     const bool vec = (((uintptr_t)ref | (uintptr_t)probe) & 15) == 0;  // rows of 2304 floats keep the alignment
+    const bool exact = n_probe <= kExactMaxProbe && (n_probe + kExFrames - 1) / kExFrames <= 65535;
+    if (exact) {
+        unsigned long long *sums = (unsigned long long *)totals;
+        cudaError_t e = cudaMemsetAsync(sums, 0, sizeof(double) * (size_t)lags, s);
+        if (e != cudaSuccess) return e;
+        {
+            LaunchTimer t("align_offset_check", s);
+            offset_check_kernel<<<n_ref + n_probe, kExThreads, 0, s>>>(ref, n_ref, probe, n_probe, lags, sums);
+        }
+        if ((e = after_launch()) != cudaSuccess) return e;
+        {
+            LaunchTimer t("align_offset_exact", s);
+            const dim3 grid((lags + kExLags - 1) / kExLags, (n_probe + kExFrames - 1) / kExFrames, kThumbPixels / kExPixels);
+            offset_exact_kernel<<<grid, kExThreads, 0, s>>>(ref, probe, n_probe, lags, sums);
+        }
+        if ((e = after_launch()) != cudaSuccess) return e;
+    }
     LaunchTimer t("align_offset_totals", s);
     const int blocks = (lags + kLagWarps - 1) / kLagWarps;
-    if (vec) offset_totals_kernel<true><<<blocks, 32 * kLagWarps, 0, s>>>(ref, probe, n_probe, lags, totals);
-    else offset_totals_kernel<false><<<blocks, 32 * kLagWarps, 0, s>>>(ref, probe, n_probe, lags, totals);
+    if (vec) offset_totals_kernel<true><<<blocks, 32 * kLagWarps, 0, s>>>(ref, probe, n_probe, lags, totals, exact);
+    else offset_totals_kernel<false><<<blocks, 32 * kLagWarps, 0, s>>>(ref, probe, n_probe, lags, totals, exact);
     return after_launch();
+}
+
+namespace {
+constexpr int kTotalsLags = 2048, kTotalsSlots = 8;
+static __device__ double g_totals[kTotalsSlots][kTotalsLags];
+}  // namespace
+
+int offset_totals_slots() { return kTotalsSlots; }
+int offset_totals_slot_lags() { return kTotalsLags; }
+cudaError_t offset_totals_slot(int slot, double **ptr)
+{
+    void *p = nullptr;
+    const cudaError_t e = cudaGetSymbolAddress(&p, g_totals);
+    *ptr = (double *)p + (size_t)slot * kTotalsLags;
+    return e;
 }
 
 }  // namespace es

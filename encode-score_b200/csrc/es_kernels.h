@@ -331,7 +331,12 @@ struct ThumbBatch {
     float *out;           // [frame][kThumbH][kThumbW]
 };
 cudaError_t launch_thumbnails(const ThumbBatch &b, cudaStream_t s);
-cudaError_t launch_offset_totals(const float *ref, const float *probe, int n_probe, int lags, double *totals, cudaStream_t s);
+cudaError_t launch_offset_totals(const float *ref, int n_ref, const float *probe, int n_probe, double *totals, cudaStream_t s);
+// Totals of a search of up to offset_totals_slot_lags() lags: slot 0 .. offset_totals_slots() - 1 of a fixed device array
+// of the CUDA context current on the calling thread.
+int offset_totals_slots();
+int offset_totals_slot_lags();
+cudaError_t offset_totals_slot(int slot, double **ptr);
 
 // ---- learned tile proposal -------------------------------------------------------------------------------------
 // A 4-layer network of valid 3 x 3 convolutions (2 -> 16 -> 16 -> 16 -> 1, ReLU after the first three) on 4 x 4

@@ -645,8 +645,9 @@ def offset_totals(ref: int, n_ref: int, probe: int, n_probe: int, totals: int, s
 def find_offset(ref: int, ref_times, probe: int, probe_times, stream: int = 0) -> tuple:
     """(offset, least mean difference) of the probe's thumbnails against the reference's (device arrays of
     len(times) thumbnails each); raises EsError with status ES_ERR_NO_MATCH when they match at no lag."""
-    rt = (ctypes.c_double * len(ref_times))(*ref_times)
-    pt = (ctypes.c_double * len(probe_times))(*probe_times)
+    import array
+    rt = (ctypes.c_double * len(ref_times)).from_buffer(array.array("d", ref_times))
+    pt = (ctypes.c_double * len(probe_times)).from_buffer(array.array("d", probe_times))
     off, best = ctypes.c_double(), ctypes.c_double()
     status = lib().es_find_offset(ref, rt, len(ref_times), probe, pt, len(probe_times), ctypes.c_void_p(stream),
                                   ctypes.byref(off), ctypes.byref(best))

@@ -185,3 +185,21 @@ def test_find_offset_keeps_the_first_of_tied_lags(cuda, module):
     off, best = es_b200.find_offset(d_ref.data_ptr(), [k / 25.0 for k in range(60)], d_probe.data_ptr(), [0.0] * 24)
     want_off, want_lag, want_best = align.find_offset(ref, [k / 25.0 for k in range(60)], probe, [0.0] * 24)
     assert want_lag == 7 and off == want_off and best == want_best
+
+
+@pytest.mark.parametrize("n_ref,n_probe,cell", [(24, 24, 900), (40, 24, 3600), (39, 33, 150), (33, 16, 7), (16, 16, 900), (18, 1, 3600)])
+def test_offset_totals_of_picture_means_bit_for_bit(cuda, module, n_ref, n_probe, cell):
+    """Means of `cell` pixels as thumbnails hold them (no bits below 2^-20 from 8 code values on): lags and probe frames
+    around the 16 x 16 the exact sums take at once, a reference frame of values below 8 (its lags are added in order),
+    and values from 0 to the largest."""
+    rng = np.random.default_rng(n_ref + cell)
+    ref = (rng.integers(8 * cell, 1023 * cell, (n_ref, 36, 64)) / cell).astype(np.float32)
+    probe = (rng.integers(8 * cell, 1023 * cell, (n_probe, 36, 64)) / cell).astype(np.float32)
+    ref[0, 0, 0], probe[0, 0, 0] = 0.0, 1023.0
+    if n_ref > 30:
+        ref[n_ref - 1, 5] = np.float32(1) / np.float32(3)
+    d_ref, d_probe = cuda.from_numpy(ref.ravel()).cuda(), cuda.from_numpy(probe.ravel()).cuda()
+    totals = cuda.full((n_ref - n_probe + 1,), -1.0, dtype=cuda.float64, device="cuda")
+    es_b200.offset_totals(d_ref.data_ptr(), n_ref, d_probe.data_ptr(), n_probe, totals.data_ptr())
+    want = align.lag_totals(ref, probe)
+    assert np.array_equal(totals.cpu().numpy().view(np.uint64), want.view(np.uint64))
