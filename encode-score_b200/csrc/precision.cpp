@@ -6,11 +6,11 @@
 
 namespace es {
 int precision_quantities();
-cudaError_t launch_precision_sat(const uint16_t *y, int w, int h, int up, long long *si, float *shi, float *slo, float *sp,
-                                 cudaStream_t s);
-cudaError_t launch_precision_blocks(const uint16_t *yr, const uint16_t *yd, int w, int h, int up, const long long *const si[2],
-                                    const float *const shi[2], const float *const slo[2], const float *const sp[2], long long *qi,
-                                    float *qc, float *qp, cudaStream_t s);
+size_t precision_band_words(int w, int h);
+cudaError_t launch_precision_sat(const uint16_t *const y[2], int w, int h, int up, unsigned *const band[2], float *const shi[2],
+                                 float *const slo[2], float *const sp[2], cudaStream_t s);
+cudaError_t launch_precision_blocks(const uint16_t *const y[2], int w, int h, int up, const float *const shi[2], const float *const slo[2],
+                                    const float *const sp[2], long long *qi, float *qc, float *qp, cudaStream_t s);
 cudaError_t launch_precision_windows(const long long *qi, const float *qc, const float *qp, int bw, int bh, int k, int mode,
                                      double *out, cudaStream_t s);
 }  // namespace es
@@ -19,7 +19,7 @@ using namespace es;
 
 struct es_windows {
     int w = 0, h = 0, bw = 0, bh = 0;
-    DeviceBuffer<long long> si[2];
+    DeviceBuffer<unsigned> band[2];
     DeviceBuffer<float> shi[2], slo[2], sp[2];
     DeviceBuffer<long long> qi;
     DeviceBuffer<float> qc, qp;
@@ -41,7 +41,7 @@ int es_windows_create(int w, int h, es_windows **out)
         p->bh = h / 16;
         const size_t n = (size_t)w * h, q = (size_t)p->bw * p->bh * precision_quantities();
         for (int i = 0; i < 2; i++) {
-            p->si[i].reset(n);
+            p->band[i].reset(precision_band_words(w, h));
             p->shi[i].reset(n);
             p->slo[i].reset(n);
             p->sp[i].reset(n);
@@ -60,13 +60,11 @@ int es_windows_compute(es_windows *p, uint64_t src, uint64_t enc, int up, void *
         require(up == 0 || up == 2, "es_windows_compute: up must be 0 (10-bit) or 2 (8-bit)");
         cudaStream_t s = (cudaStream_t)stream;
         const uint16_t *y[2] = {(const uint16_t *)src, (const uint16_t *)enc};
-        for (int i = 0; i < 2; i++)
-            cuda_check(launch_precision_sat(y[i], p->w, p->h, up, p->si[i].ptr, p->shi[i].ptr, p->slo[i].ptr, p->sp[i].ptr, s),
-                       "summed-area tables");
-        const long long *si[2] = {p->si[0].ptr, p->si[1].ptr};
-        const float *shi[2] = {p->shi[0].ptr, p->shi[1].ptr}, *slo[2] = {p->slo[0].ptr, p->slo[1].ptr}, *sp[2] = {p->sp[0].ptr, p->sp[1].ptr};
-        cuda_check(launch_precision_blocks(y[0], y[1], p->w, p->h, up, si, shi, slo, sp, p->qi.ptr, p->qc.ptr, p->qp.ptr, s),
-                   "block sums");
+        unsigned *const band[2] = {p->band[0].ptr, p->band[1].ptr};
+        float *const shi[2] = {p->shi[0].ptr, p->shi[1].ptr}, *const slo[2] = {p->slo[0].ptr, p->slo[1].ptr},
+              *const sp[2] = {p->sp[0].ptr, p->sp[1].ptr};
+        cuda_check(launch_precision_sat(y, p->w, p->h, up, band, shi, slo, sp, s), "summed-area tables");
+        cuda_check(launch_precision_blocks(y, p->w, p->h, up, shi, slo, sp, p->qi.ptr, p->qc.ptr, p->qp.ptr, s), "block sums");
         p->ready = true;
     });
 }

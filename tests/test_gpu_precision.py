@@ -36,3 +36,31 @@ def test_window_energies_in_three_arithmetics(cuda, module, w, h, depth):
         assert rel_c.max() <= 1e-5, (window, rel_c.max())
         assert rel_c.max() <= rel_p.max() + 1e-12
     win.close()
+
+
+@pytest.mark.parametrize("w,h", [(16, 16), (65, 33), (130, 63), (64, 96), (191, 32), (16, 16400)])
+def test_sizes_around_the_table_bands_and_chunks(cuda, module, w, h):
+    """The tables are scanned in bands of 32 rows and chunks of 64 columns, blocks of 16 x 16 read 25 entries a side, and
+    pictures of more than 16384 rows take another path: the exact form equals the oracle's, the compensated form stays
+    within 1e-5 of it."""
+    rng = np.random.default_rng(w + h)
+    yy, xx = np.mgrid[0:h, 0:w]
+    yr = np.clip(700 + 200 * np.sin(xx / 9 + yy / 23) + rng.normal(0, 20, (h, w)), 0, 1023).astype(np.uint16)
+    yd = np.clip(yr + rng.normal(0, 8, (h, w)), 0, 1023).astype(np.uint16)
+    win = es_b200.Windows(w, h)
+    r, d = to_dev(cuda, yr), to_dev(cuda, yd)
+    win.compute(r.data_ptr(), d.data_ptr(), 0)
+    for window in (16, 32):
+        n = (w // window) * (h // window)
+        if not n:
+            continue
+        want = precision.window_figures(yr, yd, 0, window)
+        outs = []
+        for mode in range(2):
+            o = zeros_dev(cuda, (n, 8), np.float64)
+            win.figures(window, mode, o.data_ptr())
+            outs.append(from_dev(o, np.float64))
+        assert np.array_equal(outs[0], want), window
+        scale = np.maximum(np.abs(want), 1e-3 * np.abs(want).max(axis=0, keepdims=True))
+        assert (np.abs(outs[1] - want) / scale).max() <= 1e-5
+    win.close()
