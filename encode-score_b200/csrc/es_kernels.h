@@ -377,19 +377,21 @@ inline size_t feature_map_size(int w, int h) { return (size_t)((w + 3) / 4) * ((
 // Features of n crops: crop i covers scale-0 pixels from (xy[2 i], xy[2 i + 1]) on, fw x fh feature pixels of 4 x 4.
 cudaError_t launch_net_features(const uint16_t *word, int w, int h, const int *xy, int n, int fw, int fh, float *out,
                                 cudaStream_t s);
-// Training on crops (NCHW float): forward of layer l (input n x ci x h x w, output n x co x (h - 2) x (w - 2), ReLU
-// for l < 3); backward of layer l (gradients of its weights and biases into grads and, for l > 0, the gradient of its
-// input times the ReLU mask of that input into gin); the tile loss of the last layer (n x 1 x 16a x 16b against
+// Training on crops (NCHW float, h even): forward of layer l (input n x ci x h x w, output n x co x (h - 2) x (w - 2),
+// ReLU for l < 3); backward of layer l (its weights' and biases' gradients in kNetGradBlocks parts of kNetParams floats
+// and, for l > 0, the gradient of its input times the ReLU mask of that input into gin); the tile loss of the last layer (n x 1 x 16a x 16b against
 // n x a x b labels: per-tile squared differences into loss_parts, the gradient of the last layer's output into gz);
-// and Adam (master weights, their bfloat16-rounded copy, moments).
+// and the gradients from every layer's parts, with Adam's step on them when lr > 0 (master weights, their
+// bfloat16-rounded copy, moments).
+constexpr int kNetGradBlocks = 148 * 2;
 cudaError_t launch_net_forward(int layer, const float *in, int n, int h, int w, const float *params, float *out,
                                cudaStream_t s);
 cudaError_t launch_net_backward(int layer, const float *gout, const float *in, int n, int h, int w, const float *params,
-                                float *gin, float *grads, cudaStream_t s);
+                                float *gin, float *parts, cudaStream_t s);
 cudaError_t launch_net_loss(const float *z, const float *labels, int n, int ta, int tb, float *gz, float *loss_parts,
                             cudaStream_t s);
-cudaError_t launch_net_adam(float *params, float *rounded, const float *grads, float *m, float *v, int count, float lr,
-                            float b1, float b2, float eps, int t, cudaStream_t s);
+cudaError_t launch_net_grads(const float *parts, float *params, float *rounded, float *grads, float *m, float *v, float lr, float b1,
+                             float b2, float eps, int t, cudaStream_t s);
 // The mma B fragments of layers 1 and 2 (kNetFrags words) from the bfloat16-rounded parameters.
 cudaError_t launch_net_pack(const float *rounded, uint32_t *frags, cudaStream_t s);
 

@@ -13,6 +13,7 @@ using namespace es;
 
 struct es_proposal_net {
     DeviceBuffer<float> params, rounded, grads, m, v;
+    DeviceBuffer<float> parts;  // the training blocks' shares of the gradients (allocated by the first step)
     DeviceBuffer<uint32_t> frags;
     bool frags_current = false;
     int t = 0;
@@ -66,6 +67,7 @@ void init_net(es_proposal_net &net, const float *host, uint64_t seed)
 
 void ensure_scratch(es_proposal_net &net, int n, int h, int w)
 {
+    if (!net.parts.ptr) net.parts.reset((size_t)kNetGradBlocks * kNetParams);
     if (n <= net.cap_n && h == net.cap_h && w == net.cap_w) return;
     net.cap_n = n;
     net.cap_h = h;
@@ -134,19 +136,19 @@ int es_proposal_net_train_step(es_proposal_net *net, const float *x, const float
         cuda_check(launch_net_forward(3, net->a3.ptr, n, h - 6, w - 6, P, net->z.ptr, s), "training forward");
         const int ta = (h - 8) / 16, tb = (w - 8) / 16;
         cuda_check(launch_net_loss(net->z.ptr, labels, n, ta, tb, net->gz.ptr, net->loss_parts.ptr, s), "training loss");
-        cuda_check(launch_net_backward(3, net->gz.ptr, net->a3.ptr, n, h - 6, w - 6, P, net->g3.ptr, net->grads.ptr, s), "training backward");
-        cuda_check(launch_net_backward(2, net->g3.ptr, net->a2.ptr, n, h - 4, w - 4, P, net->g2.ptr, net->grads.ptr, s), "training backward");
-        cuda_check(launch_net_backward(1, net->g2.ptr, net->a1.ptr, n, h - 2, w - 2, P, net->g1.ptr, net->grads.ptr, s), "training backward");
-        cuda_check(launch_net_backward(0, net->g1.ptr, x, n, h, w, P, nullptr, net->grads.ptr, s), "training backward");
-        if (grads)
-            cuda_check(cudaMemcpyAsync(grads, net->grads.ptr, sizeof(float) * kNetParams, cudaMemcpyDeviceToHost, s), "reading gradients");
+        cuda_check(launch_net_backward(3, net->gz.ptr, net->a3.ptr, n, h - 6, w - 6, P, net->g3.ptr, net->parts.ptr, s), "training backward");
+        cuda_check(launch_net_backward(2, net->g3.ptr, net->a2.ptr, n, h - 4, w - 4, P, net->g2.ptr, net->parts.ptr, s), "training backward");
+        cuda_check(launch_net_backward(1, net->g2.ptr, net->a1.ptr, n, h - 2, w - 2, P, net->g1.ptr, net->parts.ptr, s), "training backward");
+        cuda_check(launch_net_backward(0, net->g1.ptr, x, n, h, w, P, nullptr, net->parts.ptr, s), "training backward");
         if (lr > 0.0f) {
             net->t++;
-            cuda_check(launch_net_adam(net->params.ptr, net->rounded.ptr, net->grads.ptr, net->m.ptr, net->v.ptr, kNetParams, lr, 0.9f,
-                                       0.999f, 1e-8f, net->t, s),
-                       "training step");
             net->frags_current = false;
         }
+        cuda_check(launch_net_grads(net->parts.ptr, net->params.ptr, net->rounded.ptr, net->grads.ptr, net->m.ptr, net->v.ptr, lr, 0.9f, 0.999f,
+                                    1e-8f, net->t, s),
+                   "training step");
+        if (grads)
+            cuda_check(cudaMemcpyAsync(grads, net->grads.ptr, sizeof(float) * kNetParams, cudaMemcpyDeviceToHost, s), "reading gradients");
         if (loss) {
             const size_t tiles = (size_t)n * ta * tb;
             cuda_check(cudaMemcpyAsync(net->h_loss.ptr, net->loss_parts.ptr, sizeof(float) * tiles, cudaMemcpyDeviceToHost, s), "reading the loss");

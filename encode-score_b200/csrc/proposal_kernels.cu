@@ -121,107 +121,197 @@ __global__ void __launch_bounds__(256) feature_map_kernel(const __grid_constant_
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Training: valid 3 x 3 convolutions on NCHW float crops, weights rounded to bfloat16.
+// Training: valid 3 x 3 convolutions on NCHW float crops, weights rounded to bfloat16. What bounds them is the FP32 fused
+// multiply-adds (2.1 G per step of 32 crops of 72 x 72: 58 us at the FP32 rate) and, beside them, the shared-memory reads
+// of the weights: a thread makes two pixels, one above the other, of all 16 channels, so one 16-byte read of four weights
+// serves eight multiply-adds. Per step of 32 crops, before / now: forward 142 / 89 us, backward 1339 / 209 us.
 // ---------------------------------------------------------------------------------------------------------------
-template <int CI, int CO>
-__global__ void __launch_bounds__(256) conv_fwd_kernel(const float *in, int n, int h, int w, const float *P, int woff, int boff,
-                                                       bool relu, float *out)
+// acc[j][c] += v[j] w[c] for the N channels of one tap
+template <int N>
+__device__ __forceinline__ void tap_fma(float (&acc)[2][N], float v0, float v1, const float *w)
 {
-    __shared__ float W[CO * CI * 9], B[CO];
-    for (int i = threadIdx.x; i < CO * CI * 9; i += 256) W[i] = bf16r(P[woff + i]);
-    for (int i = threadIdx.x; i < CO; i += 256) B[i] = bf16r(P[boff + i]);
-    __syncthreads();
-    const int ho = h - 2, wo = w - 2;
-    const size_t plane = (size_t)ho * wo, total = plane * n;
-    for (size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x; idx < total; idx += (size_t)gridDim.x * 256) {
-        const int nn = (int)(idx / plane), r = (int)(idx - (size_t)nn * plane), y = r / wo, x = r - y * wo;
-        float acc[CO];
+    if constexpr (N % 4 == 0) {
 #pragma unroll
-        for (int co = 0; co < CO; co++) acc[co] = B[co];
-        for (int ci = 0; ci < CI; ci++) {
-            const float *src = in + ((size_t)(nn * CI + ci) * h + y) * w + x;
+        for (int c = 0; c < N; c += 4) {
+            const float4 q = *(const float4 *)(w + c);
+            const float wv[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-            for (int k = 0; k < 9; k++) {
-                const float v = src[(k / 3) * w + (k % 3)];
-#pragma unroll
-                for (int co = 0; co < CO; co++) acc[co] = __fmaf_rn(v, W[(co * CI + ci) * 9 + k], acc[co]);
+            for (int k = 0; k < 4; k++) {
+                acc[0][c + k] = __fmaf_rn(v0, wv[k], acc[0][c + k]);
+                acc[1][c + k] = __fmaf_rn(v1, wv[k], acc[1][c + k]);
             }
         }
+    } else {
 #pragma unroll
-        for (int co = 0; co < CO; co++)
-            out[((size_t)(nn * CO + co) * ho + y) * wo + x] = relu ? fmaxf(acc[co], 0.0f) : acc[co];
+        for (int c = 0; c < N; c++) {
+            acc[0][c] = __fmaf_rn(v0, w[c], acc[0][c]);
+            acc[1][c] = __fmaf_rn(v1, w[c], acc[1][c]);
+        }
     }
+}
+
+// A thread makes output pixels (y, x) and (y + 1, x), y even (crops have an even number of rows), of every channel.
+template <int CI, int CO>
+__global__ void __launch_bounds__(128) conv_fwd_kernel(const float *in, int n, int h, int w, const float *P, int woff, int boff,
+                                                       bool relu, float *out)
+{
+    __shared__ __align__(16) float W[CI * 9 * CO];  // [input channel][tap][output channel]
+    __shared__ float B[CO];
+    for (int i = threadIdx.x; i < CO * CI * 9; i += 128) W[(i % (CI * 9)) * CO + i / (CI * 9)] = bf16r(P[woff + i]);
+    for (int i = threadIdx.x; i < CO; i += 128) B[i] = bf16r(P[boff + i]);
+    __syncthreads();
+    const int ho = h - 2, wo = w - 2, pairs = ho / 2 * wo, idx = blockIdx.x * 128 + threadIdx.x;
+    if (idx >= pairs * n) return;
+    const int nn = idx / pairs, r = idx - nn * pairs, y = 2 * (r / wo), x = r % wo;
+    float acc[2][CO];
+#pragma unroll
+    for (int co = 0; co < CO; co++) acc[0][co] = acc[1][co] = B[co];
+    const float *src = in + ((size_t)nn * CI * h + y) * w + x;
+    for (int ci = 0; ci < CI; ci++, src += (size_t)h * w) {
+        float v[4][3];
+#pragma unroll
+        for (int k = 0; k < 12; k++) v[k / 3][k % 3] = __ldg(src + (k / 3) * w + k % 3);
+#pragma unroll
+        for (int k = 0; k < 9; k++) tap_fma<CO>(acc, v[k / 3][k % 3], v[k / 3 + 1][k % 3], W + (ci * 9 + k) * CO);
+    }
+#pragma unroll
+    for (int co = 0; co < CO; co++)
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+            out[((size_t)(nn * CO + co) * ho + y + j) * wo + x] = relu ? fmaxf(acc[j][co], 0.0f) : acc[j][co];
 }
 
 // gin = (full correlation of gout with the flipped kernel) x (in > 0): the gradient of the layer's input, through the
-// ReLU that produced it.
+// ReLU that produced it, two input pixels per thread as above.
 template <int CI, int CO>
-__global__ void __launch_bounds__(256) conv_bwd_data_kernel(const float *gout, const float *in, int n, int h, int w,
+__global__ void __launch_bounds__(128) conv_bwd_data_kernel(const float *gout, const float *in, int n, int h, int w,
                                                             const float *P, int woff, float *gin)
 {
-    __shared__ float W[CO * CI * 9];
-    for (int i = threadIdx.x; i < CO * CI * 9; i += 256) W[i] = bf16r(P[woff + i]);
-    __syncthreads();
-    const int ho = h - 2, wo = w - 2;
-    const size_t plane = (size_t)h * w, total = plane * n;
-    for (size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x; idx < total; idx += (size_t)gridDim.x * 256) {
-        const int nn = (int)(idx / plane), r = (int)(idx - (size_t)nn * plane), y = r / w, x = r - y * w;
-        float acc[CI];
-#pragma unroll
-        for (int ci = 0; ci < CI; ci++) acc[ci] = 0.0f;
-        for (int co = 0; co < CO; co++) {
-#pragma unroll
-            for (int k = 0; k < 9; k++) {
-                const int oy = y - k / 3, ox = x - k % 3;
-                if (oy < 0 || oy >= ho || ox < 0 || ox >= wo) continue;
-                const float g = gout[((size_t)(nn * CO + co) * ho + oy) * wo + ox];
-#pragma unroll
-                for (int ci = 0; ci < CI; ci++) acc[ci] = __fmaf_rn(g, W[(co * CI + ci) * 9 + k], acc[ci]);
-            }
-        }
-#pragma unroll
-        for (int ci = 0; ci < CI; ci++) {
-            const size_t at = ((size_t)(nn * CI + ci) * h + y) * w + x;
-            gin[at] = in[at] > 0.0f ? acc[ci] : 0.0f;
-        }
+    __shared__ __align__(16) float W[CO * 9 * CI];  // [output channel][tap][input channel]
+    for (int i = threadIdx.x; i < CO * CI * 9; i += 128) {
+        const int co = i / (CI * 9), r = i % (CI * 9);
+        W[(co * 9 + r % 9) * CI + r / 9] = bf16r(P[woff + i]);
     }
+    __syncthreads();
+    const int ho = h - 2, wo = w - 2, pairs = h / 2 * w, idx = blockIdx.x * 128 + threadIdx.x;
+    if (idx >= pairs * n) return;
+    const int nn = idx / pairs, r = idx - nn * pairs, y = 2 * (r / w), x = r % w;
+    float acc[2][CI];
+#pragma unroll
+    for (int ci = 0; ci < CI; ci++) acc[0][ci] = acc[1][ci] = 0.0f;
+    for (int co = 0; co < CO; co++) {
+        const float *src = gout + (size_t)(nn * CO + co) * ho * wo;
+        float g[4][3];  // gout rows y - 2 .. y + 1, columns x - 2 .. x; 0 outside
+#pragma unroll
+        for (int k = 0; k < 12; k++) {
+            const int oy = y - 2 + k / 3, ox = x - 2 + k % 3;
+            g[k / 3][k % 3] = (oy >= 0 && oy < ho && ox >= 0 && ox < wo) ? __ldg(src + oy * wo + ox) : 0.0f;
+        }
+#pragma unroll
+        for (int k = 0; k < 9; k++) tap_fma<CI>(acc, g[2 - k / 3][2 - k % 3], g[3 - k / 3][2 - k % 3], W + (co * 9 + k) * CI);
+    }
+#pragma unroll
+    for (int ci = 0; ci < CI; ci++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const size_t at = ((size_t)(nn * CI + ci) * h + y + j) * w + x;
+            gin[at] = in[at] > 0.0f ? acc[j][ci] : 0.0f;
+        }
 }
 
-// One block per (co, ci): the 9 weight gradients (and the bias gradient when ci == 0), summed in a fixed order.
+// Weight and bias gradients. A block takes tiles of 8 x 36 output pixels in turn: both planes' tiles are staged in shared
+// memory and a thread holds the 9 taps of one (output, input) channel pair, reading 4 pixels of the gradient and the 6
+// input values of a new row per 36 multiply-adds. Its sums go to its own row of `parts`; net_grads_kernel adds the rows
+// in a fixed order. (One block per pair over every pixel, the form before, left 16 to 256 blocks walking 139 thousand
+// pixels each: 335 us a layer on average, with the data gradients, against 52.)
+constexpr int kWgRows = 8, kWgCols = 36, kWgStride = 40;
 template <int CI, int CO>
 __global__ void __launch_bounds__(256) conv_bwd_weight_kernel(const float *gout, const float *in, int n, int h, int w,
-                                                              float *G, int woff, int boff)
+                                                              float *parts, int woff, int boff)
 {
-    __shared__ float part[8][10];
-    const int co = blockIdx.x / CI, ci = blockIdx.x % CI;
-    const int ho = h - 2, wo = w - 2;
-    const size_t plane = (size_t)ho * wo, total = plane * n;
+    // channel strides of 4 words more than a whole number of rows: neighbouring channels' 16-byte reads fall on
+    // different banks
+    constexpr int kIn = (kWgRows + 2) * kWgStride + 4, kG = kWgRows * kWgCols + 4;
+    constexpr int kPairs = CI * CO, kGroups = 256 / kPairs;
+    __shared__ __align__(16) float tin[CI * kIn];
+    __shared__ __align__(16) float tg[CO * kG];
+    __shared__ float red[kGroups > 1 ? 256 * 10 : 1];
+    const int tid = threadIdx.x, pair = tid % kPairs, group = tid / kPairs, co = pair / CI, ci = pair % CI;
+    const int ho = h - 2, wo = w - 2, ty = (ho + kWgRows - 1) / kWgRows, tx = (wo + kWgCols - 1) / kWgCols, tiles = n * ty * tx;
     float acc[10];
 #pragma unroll
     for (int k = 0; k < 10; k++) acc[k] = 0.0f;
-    for (size_t idx = threadIdx.x; idx < total; idx += 256) {
-        const int nn = (int)(idx / plane), r = (int)(idx - (size_t)nn * plane), y = r / wo, x = r - y * wo;
-        const float g = gout[((size_t)(nn * CO + co) * ho + y) * wo + x];
-        const float *src = in + ((size_t)(nn * CI + ci) * h + y) * w + x;
+    for (int t = blockIdx.x; t < tiles; t += kNetGradBlocks) {
+        const int nn = t / (ty * tx), r = t - nn * ty * tx, y0 = r / tx * kWgRows, x0 = r % tx * kWgCols;
+        __syncthreads();
+        for (int i = tid; i < CI * (kWgRows + 2) * kWgStride; i += 256) {
+            const int c = i / ((kWgRows + 2) * kWgStride), q = i % ((kWgRows + 2) * kWgStride), y = y0 + q / kWgStride, x = x0 + q % kWgStride;
+            tin[c * kIn + q] = (y < h && x < w) ? __ldg(in + ((size_t)(nn * CI + c) * h + y) * w + x) : 0.0f;
+        }
+        for (int i = tid; i < CO * kWgRows * kWgCols; i += 256) {
+            const int c = i / (kWgRows * kWgCols), q = i % (kWgRows * kWgCols), y = y0 + q / kWgCols, x = x0 + q % kWgCols;
+            tg[c * kG + q] = (y < ho && x < wo) ? __ldg(gout + ((size_t)(nn * CO + c) * ho + y) * wo + x) : 0.0f;
+        }
+        __syncthreads();
+        const float *a = tin + ci * kIn, *g = tg + co * kG;
+        auto row6 = [&](float (&v)[6], int y, int x) {
+            const float4 q = *(const float4 *)(a + y * kWgStride + x);
+            const float2 p = *(const float2 *)(a + y * kWgStride + x + 4);
+            v[0] = q.x;
+            v[1] = q.y;
+            v[2] = q.z;
+            v[3] = q.w;
+            v[4] = p.x;
+            v[5] = p.y;
+        };
+        auto add = [&](const float (&v0)[6], const float (&v1)[6], const float (&v2)[6], int y, int x) {
+            const float4 q = *(const float4 *)(g + y * kWgCols + x);
+            const float gv[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-        for (int k = 0; k < 9; k++) acc[k] = __fmaf_rn(g, src[(k / 3) * w + (k % 3)], acc[k]);
-        acc[9] += g;
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+            for (int k = 0; k < 3; k++)
 #pragma unroll
-    for (int k = 0; k < 10; k++) {
-        float v = acc[k];
+                for (int j = 0; j < 4; j++) {
+                    acc[k] = __fmaf_rn(gv[j], v0[j + k], acc[k]);
+                    acc[3 + k] = __fmaf_rn(gv[j], v1[j + k], acc[3 + k]);
+                    acc[6 + k] = __fmaf_rn(gv[j], v2[j + k], acc[6 + k]);
+                }
+            acc[9] += (gv[0] + gv[1]) + (gv[2] + gv[3]);
+        };
+        if (kGroups == 1) {
+            for (int x = 0; x < kWgCols; x += 4) {
+                float v[3][6];
+                row6(v[0], 0, x);
+                row6(v[1], 1, x);
 #pragma unroll
-        for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-        if (lane == 0) part[warp][k] = v;
+                for (int y = 0; y < kWgRows; y++) {
+                    row6(v[(y + 2) % 3], y + 2, x);
+                    add(v[y % 3], v[(y + 1) % 3], v[(y + 2) % 3], y, x);
+                }
+            }
+        } else {
+            for (int i = group; i < kWgRows * (kWgCols / 4); i += kGroups) {
+                const int y = i / (kWgCols / 4), x = 4 * (i % (kWgCols / 4));
+                float v[3][6];
+                row6(v[0], y, x);
+                row6(v[1], y + 1, x);
+                row6(v[2], y + 2, x);
+                add(v[0], v[1], v[2], y, x);
+            }
+        }
     }
-    __syncthreads();
-    if (threadIdx.x < 10) {
-        float s = 0.0f;
-        for (int k = 0; k < 8; k++) s += part[k][threadIdx.x];
-        if (threadIdx.x < 9) G[woff + (co * CI + ci) * 9 + threadIdx.x] = s;
-        else if (ci == 0) G[boff + co] = s;
+    float *part = parts + (size_t)blockIdx.x * kNetParams;
+    if (kGroups > 1) {
+#pragma unroll
+        for (int k = 0; k < 10; k++) red[tid * 10 + k] = acc[k];
+        __syncthreads();
+        if (group != 0) return;
+        for (int q = 1; q < kGroups; q++)
+#pragma unroll
+            for (int k = 0; k < 10; k++) acc[k] += red[(q * kPairs + pair) * 10 + k];
     }
+#pragma unroll
+    for (int k = 0; k < 9; k++) part[woff + (co * CI + ci) * 9 + k] = acc[k];
+    if (ci == 0) part[boff + co] = acc[9];
 }
 
 // One block per crop: the mean of each 16 x 16 block of z against its label; gz = d loss / d z with
@@ -252,12 +342,29 @@ __global__ void __launch_bounds__(256) net_loss_kernel(const float *z, const flo
     }
 }
 
-__global__ void net_adam_kernel(float *P, float *R, const float *G, float *M, float *V, int count, float lr, float b1, float b2,
-                                float eps, int t)
+// The gradients from the blocks' parts, 32 parameters per block in a fixed order (warp g adds blocks g q .. g q + q - 1,
+// the 8 warps' sums are added in turn), then, with lr > 0, Adam's step on them.
+__global__ void __launch_bounds__(256) net_grads_kernel(const float *parts, float *P, float *R, float *G, float *M, float *V, float lr,
+                                                        float b1, float b2, float eps, int t)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const float g = G[i];
+    constexpr int kPer = kNetGradBlocks / 8;
+    static_assert(kNetGradBlocks % 8 == 0, "whole shares per warp");
+    __shared__ float sum[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+    float a = 0.0f;
+    if (i < kNetParams) {
+        const float *p = parts + (size_t)warp * kPer * kNetParams + i;
+#pragma unroll 8
+        for (int k = 0; k < kPer; k++) a += __ldg(p + (size_t)k * kNetParams);
+    }
+    sum[warp][lane] = a;
+    __syncthreads();
+    if (warp != 0 || i >= kNetParams) return;
+    float g = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; k++) g += sum[k][lane];
+    G[i] = g;
+    if (!(lr > 0.0f)) return;
     const float m = b1 * M[i] + (1.0f - b1) * g, v = b2 * V[i] + (1.0f - b2) * g * g;
     M[i] = m;
     V[i] = v;
@@ -799,41 +906,41 @@ cudaError_t launch_net_features(const uint16_t *word, int w, int h, const int *x
 
 cudaError_t launch_net_forward(int layer, const float *in, int n, int h, int w, const float *params, float *out, cudaStream_t s)
 {
-    const size_t total = (size_t)(h - 2) * (w - 2) * n;
+    const size_t total = (size_t)(h - 2) / 2 * (w - 2) * n;
     if (!total) return cudaSuccess;
     LaunchTimer t("proposal_train_forward", s);
-    const unsigned g = grid_for(total);
+    const unsigned g = (unsigned)((total + 127) / 128);
     switch (layer) {
-    case 0: conv_fwd_kernel<2, 16><<<g, 256, 0, s>>>(in, n, h, w, params, net_w(0), net_b(0), true, out); break;
-    case 1: conv_fwd_kernel<16, 16><<<g, 256, 0, s>>>(in, n, h, w, params, net_w(1), net_b(1), true, out); break;
-    case 2: conv_fwd_kernel<16, 16><<<g, 256, 0, s>>>(in, n, h, w, params, net_w(2), net_b(2), true, out); break;
-    case 3: conv_fwd_kernel<16, 1><<<g, 256, 0, s>>>(in, n, h, w, params, net_w(3), net_b(3), false, out); break;
+    case 0: conv_fwd_kernel<2, 16><<<g, 128, 0, s>>>(in, n, h, w, params, net_w(0), net_b(0), true, out); break;
+    case 1: conv_fwd_kernel<16, 16><<<g, 128, 0, s>>>(in, n, h, w, params, net_w(1), net_b(1), true, out); break;
+    case 2: conv_fwd_kernel<16, 16><<<g, 128, 0, s>>>(in, n, h, w, params, net_w(2), net_b(2), true, out); break;
+    case 3: conv_fwd_kernel<16, 1><<<g, 128, 0, s>>>(in, n, h, w, params, net_w(3), net_b(3), false, out); break;
     default: return cudaErrorInvalidValue;
     }
     return after_launch();
 }
 
 cudaError_t launch_net_backward(int layer, const float *gout, const float *in, int n, int h, int w, const float *params,
-                                float *gin, float *grads, cudaStream_t s)
+                                float *gin, float *parts, cudaStream_t s)
 {
     LaunchTimer t("proposal_train_backward", s);
-    const unsigned g = grid_for((size_t)h * w * n);
+    const unsigned g = (unsigned)(((size_t)h / 2 * w * n + 127) / 128);
     switch (layer) {
-    case 0: conv_bwd_weight_kernel<2, 16><<<16 * 2, 256, 0, s>>>(gout, in, n, h, w, grads, net_w(0), net_b(0)); break;
+    case 0: conv_bwd_weight_kernel<2, 16><<<kNetGradBlocks, 256, 0, s>>>(gout, in, n, h, w, parts, net_w(0), net_b(0)); break;
     case 1:
-        conv_bwd_weight_kernel<16, 16><<<256, 256, 0, s>>>(gout, in, n, h, w, grads, net_w(1), net_b(1));
+        conv_bwd_weight_kernel<16, 16><<<kNetGradBlocks, 256, 0, s>>>(gout, in, n, h, w, parts, net_w(1), net_b(1));
         count_launch();
-        conv_bwd_data_kernel<16, 16><<<g, 256, 0, s>>>(gout, in, n, h, w, params, net_w(1), gin);
+        conv_bwd_data_kernel<16, 16><<<g, 128, 0, s>>>(gout, in, n, h, w, params, net_w(1), gin);
         break;
     case 2:
-        conv_bwd_weight_kernel<16, 16><<<256, 256, 0, s>>>(gout, in, n, h, w, grads, net_w(2), net_b(2));
+        conv_bwd_weight_kernel<16, 16><<<kNetGradBlocks, 256, 0, s>>>(gout, in, n, h, w, parts, net_w(2), net_b(2));
         count_launch();
-        conv_bwd_data_kernel<16, 16><<<g, 256, 0, s>>>(gout, in, n, h, w, params, net_w(2), gin);
+        conv_bwd_data_kernel<16, 16><<<g, 128, 0, s>>>(gout, in, n, h, w, params, net_w(2), gin);
         break;
     case 3:
-        conv_bwd_weight_kernel<16, 1><<<16, 256, 0, s>>>(gout, in, n, h, w, grads, net_w(3), net_b(3));
+        conv_bwd_weight_kernel<16, 1><<<kNetGradBlocks, 256, 0, s>>>(gout, in, n, h, w, parts, net_w(3), net_b(3));
         count_launch();
-        conv_bwd_data_kernel<16, 1><<<g, 256, 0, s>>>(gout, in, n, h, w, params, net_w(3), gin);
+        conv_bwd_data_kernel<16, 1><<<g, 128, 0, s>>>(gout, in, n, h, w, params, net_w(3), gin);
         break;
     default: return cudaErrorInvalidValue;
     }
@@ -848,11 +955,11 @@ cudaError_t launch_net_loss(const float *z, const float *labels, int n, int ta, 
     return after_launch();
 }
 
-cudaError_t launch_net_adam(float *params, float *rounded, const float *grads, float *m, float *v, int count, float lr, float b1,
-                            float b2, float eps, int t, cudaStream_t s)
+cudaError_t launch_net_grads(const float *parts, float *params, float *rounded, float *grads, float *m, float *v, float lr, float b1,
+                             float b2, float eps, int t, cudaStream_t s)
 {
     LaunchTimer tm("proposal_train_adam", s);
-    net_adam_kernel<<<(count + 255) / 256, 256, 0, s>>>(params, rounded, grads, m, v, count, lr, b1, b2, eps, t);
+    net_grads_kernel<<<(kNetParams + 31) / 32, 256, 0, s>>>(parts, params, rounded, grads, m, v, lr, b1, b2, eps, t);
     return after_launch();
 }
 

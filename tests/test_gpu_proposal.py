@@ -162,3 +162,26 @@ def test_tile_masses_sum_the_cvalues_of_each_tile(cuda, module):
         at += nx * ny
     assert at == n_tiles and got.sum() > 0
     c.close()
+
+
+@pytest.mark.parametrize("n,th,tw", [(1, 1, 1), (3, 1, 2), (2, 3, 1), (5, 2, 4)])
+def test_gradients_of_crops_around_the_weight_kernels_tiles(cuda, module, n, th, tw):
+    """The weight gradients come from tiles of 8 x 36 output pixels: crops smaller than one, a little larger, and not
+    square. Tolerance as above: FP32 sums of some thousand products against FP64."""
+    rng = np.random.default_rng(n + 10 * th + 100 * tw)
+    h, w = 8 + 16 * th, 8 + 16 * tw
+    x = rng.normal(0, 1, (n, 2, h, w)).astype(np.float32)
+    labels = rng.normal(0.5, 0.5, (n, th, tw)).astype(np.float32)
+    params = random_params(6)
+    net = es_b200.ProposalNet(proposal.flatten(params))
+    xd, ld = to_dev(cuda, x), to_dev(cuda, labels)
+    loss, grads = net.train_step(xd.data_ptr(), ld.data_ptr(), n, h, w, 0.0, want_grads=True)
+    net.close()
+    want_loss, want = proposal.loss_and_grads(x.astype(np.float64), labels.astype(np.float64), params)
+    assert abs(loss - want_loss) <= 1e-5 * abs(want_loss)
+    at = 0
+    for gw, gb in want:
+        for g in (gw, gb):
+            got = grads[at:at + g.size].reshape(g.shape)
+            assert np.abs(got - g).max() <= 1e-3 * np.abs(g).max() + 1e-9
+            at += g.size
