@@ -203,3 +203,29 @@ def test_offset_totals_of_picture_means_bit_for_bit(cuda, module, n_ref, n_probe
     es_b200.offset_totals(d_ref.data_ptr(), n_ref, d_probe.data_ptr(), n_probe, totals.data_ptr())
     want = align.lag_totals(ref, probe)
     assert np.array_equal(totals.cpu().numpy().view(np.uint64), want.view(np.uint64))
+
+
+@pytest.mark.parametrize("fmt", ["planar8", "planar16", "p010"])
+@pytest.mark.parametrize("x0,w,h", [(0, 512, 36), (3, 513, 40), (8, 575, 612), (5, 1000, 1157), (15, 1024, 71)])
+def test_thumbnails_of_crops_that_start_and_end_anywhere(cuda, module, fmt, x0, w, h):
+    """Crops from 512 columns on are read 8 samples at a time wherever they start and end, in bands of any height, and
+    samples beyond the depth are added as they are."""
+    rng = np.random.default_rng(w + h)
+    size = 1 if fmt == "planar8" else 2
+    pitch = (x0 + w + 31) // 16 * 16
+    depth, shift = (8, 0) if fmt == "planar8" else (10, 6 if fmt == "p010" else 0)
+    frames = rng.integers(0, 256 if size == 1 else 1024, (2, h + 3, pitch)).astype(np.uint32) << shift
+    if fmt == "planar16":
+        frames[1, h // 2, x0 + w // 2] = 65535
+    frames = frames.astype(np.uint8 if size == 1 else np.uint16)
+    d = cuda.from_numpy(frames.view(np.uint8 if size == 1 else np.int16)).cuda()
+    views = [es_b200.FrameView(d[k].data_ptr(), d[k].data_ptr(), d[k].data_ptr(), pitch * size, pitch * size, 0, size, shift, depth) for k in range(2)]
+    out = cuda.full((2, 36, 64), -1.0, dtype=cuda.float32, device="cuda")
+    es_b200.thumbnails(views, x0, 2, w, h, out.data_ptr())
+    got = out.cpu().numpy()
+    v = (frames.astype(np.int64) >> shift) << (10 - depth)
+    ys, xs = [2 + k * h // 36 for k in range(37)], [x0 + k * w // 64 for k in range(65)]
+    for k in range(2):
+        sums = np.add.reduceat(np.add.reduceat(v[k, :ys[-1], :xs[-1]], ys[:-1], axis=0), xs[:-1], axis=1)
+        n = np.outer(np.diff(ys), np.diff(xs))
+        assert np.array_equal(got[k], sums.astype(np.float32) / n.astype(np.float32)), k
