@@ -23,9 +23,87 @@ __device__ __forceinline__ unsigned sample_at(const void *plane, int pitch, int 
     return v >> f.shift;
 }
 
-// Thread i takes 4 consecutive 2 x 2 groups of one chroma row (2 rows x 8 luma columns, 4 samples of U and of V).
-// Planar frames whose rows and crop allow it are moved with 16- / 8-byte loads and stores; every other layout
-// (semi-planar, shifted samples such as P010, odd alignments) one sample at a time.
+// 8 samples from p as four words of two 16-bit samples: one load where the address allows, else four loads of two samples,
+// else one by one.
+__device__ __forceinline__ uint4 load8(const unsigned char *p, int bytes)
+{
+    const uintptr_t at = (uintptr_t)p;
+    if (bytes == 2) {
+        if ((at & 15) == 0) return __ldg((const uint4 *)p);
+        const unsigned *q = (const unsigned *)p;
+        if ((at & 3) == 0) return make_uint4(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3));
+        const uint16_t *r = (const uint16_t *)p;
+        auto two = [&](int k) { return (unsigned)__ldg(r + k) | ((unsigned)__ldg(r + k + 1) << 16); };
+        return make_uint4(two(0), two(2), two(4), two(6));
+    }
+    if ((at & 7) == 0) {
+        const uint2 q = __ldg((const uint2 *)p);
+        return make_uint4(__byte_perm(q.x, 0, 0x4140), __byte_perm(q.x, 0, 0x4342), __byte_perm(q.y, 0, 0x4140), __byte_perm(q.y, 0, 0x4342));
+    }
+    if ((at & 1) == 0) {
+        const uint16_t *r = (const uint16_t *)p;
+        auto two = [&](int k) { return __byte_perm((unsigned)__ldg(r + k), 0, 0x4140); };
+        return make_uint4(two(0), two(1), two(2), two(3));
+    }
+    auto two = [&](int k) { return (unsigned)__ldg(p + k) | ((unsigned)__ldg(p + k + 1) << 16); };
+    return make_uint4(two(0), two(2), two(4), two(6));
+}
+
+// 4 samples from p, likewise.
+__device__ __forceinline__ uint2 load4(const unsigned char *p, int bytes)
+{
+    const uintptr_t at = (uintptr_t)p;
+    if (bytes == 2) {
+        if ((at & 7) == 0) return __ldg((const uint2 *)p);
+        const uint16_t *r = (const uint16_t *)p;
+        auto two = [&](int k) { return (unsigned)__ldg(r + k) | ((unsigned)__ldg(r + k + 1) << 16); };
+        return make_uint2(two(0), two(2));
+    }
+    if ((at & 3) == 0) {
+        const unsigned q = __ldg((const unsigned *)p);
+        return make_uint2(__byte_perm(q, 0, 0x4140), __byte_perm(q, 0, 0x4342));
+    }
+    auto two = [&](int k) { return (unsigned)__ldg(p + k) | ((unsigned)__ldg(p + k + 1) << 16); };
+    return make_uint2(two(0), two(2));
+}
+
+// 8 (4) samples to p, which is 4-byte (2-byte) aligned at least: rows of even widths.
+__device__ __forceinline__ void store8(uint16_t *p, uint4 v)
+{
+    const uintptr_t at = (uintptr_t)p;
+    if ((at & 15) == 0) {
+        *(uint4 *)p = v;
+    } else if ((at & 7) == 0) {
+        *(uint2 *)p = make_uint2(v.x, v.y);
+        *(uint2 *)(p + 4) = make_uint2(v.z, v.w);
+    } else {
+        unsigned *q = (unsigned *)p;
+        q[0] = v.x;
+        q[1] = v.y;
+        q[2] = v.z;
+        q[3] = v.w;
+    }
+}
+__device__ __forceinline__ void store4(uint16_t *p, uint2 v)
+{
+    const uintptr_t at = (uintptr_t)p;
+    if ((at & 7) == 0) {
+        *(uint2 *)p = v;
+    } else if ((at & 3) == 0) {
+        ((unsigned *)p)[0] = v.x;
+        ((unsigned *)p)[1] = v.y;
+    } else {
+        p[0] = (uint16_t)v.x;
+        p[1] = (uint16_t)(v.x >> 16);
+        p[2] = (uint16_t)v.y;
+        p[3] = (uint16_t)(v.y >> 16);
+    }
+}
+
+// Thread i takes 4 consecutive 2 x 2 groups of one chroma row (2 rows x 8 luma columns, 4 samples of U and of V), planar
+// or semi-planar, with the widest loads and stores each address allows; the last columns of a chroma row that is no
+// multiple of 4 go one sample at a time. Bound by HBM: two 3840 x 2160 P010 frames took 40 us one
+// sample at a time, 20 us now.
 __global__ void __launch_bounds__(256) unpack_kernel(const __grid_constant__ UnpackBatch b)
 {
     const int j = find_job(b.njobs, (int)blockIdx.x, [&](int k) { return b.job[k].first_block; });
@@ -36,41 +114,31 @@ __global__ void __launch_bounds__(256) unpack_kernel(const __grid_constant__ Unp
     const int i = (blockIdx.x - J.first_block) * 256 + threadIdx.x;
     if (i >= qw * ch) return;
     const int cy = i / qw, cx0 = 4 * (i - cy * qw), up = J.pd - f.depth;
-    const bool full = cx0 + 4 <= cw && !f.semi && f.shift == 0 && (x0 & 7) == 0;
-    if (full && f.bytes == 2 && (f.ypitch & 15) == 0 && (f.cpitch & 7) == 0 && (((uintptr_t)f.y & 15) | ((uintptr_t)f.u & 7) | ((uintptr_t)f.v & 7)) == 0 &&
-        (J.w & 7) == 0) {
-        auto sh4 = [&](uint4 q) { return make_uint4(q.x << up, q.y << up, q.z << up, q.w << up); };  // samples < 2^10
+    if (cx0 + 4 <= cw) {
+        const unsigned mask = ((f.bytes == 1 ? 0xFFu : 0xFFFFu) >> f.shift) * 0x10001u;
+        auto put = [&](unsigned q) { return ((q >> f.shift) & mask) << up; };
+        uint4 y[2];
 #pragma unroll
-        for (int dy = 0; dy < 2; dy++) {
-            const uint4 q = __ldg((const uint4 *)((const unsigned char *)f.y + (size_t)(2 * cy + dy + y0) * f.ypitch) + (2 * cx0 + x0) / 8);
-            *(uint4 *)(J.y16 + (size_t)(2 * cy + dy) * J.w + 2 * cx0) = sh4(q);
-        }
+        for (int dy = 0; dy < 2; dy++)
+            y[dy] = load8((const unsigned char *)f.y + (size_t)(2 * cy + dy + y0) * f.ypitch + (size_t)(2 * cx0 + x0) * f.bytes, f.bytes);
         const size_t co = (size_t)(cy + y0 / 2) * f.cpitch;
-        const uint2 u = __ldg((const uint2 *)((const unsigned char *)f.u + co) + (cx0 + x0 / 2) / 4);
-        const uint2 v = __ldg((const uint2 *)((const unsigned char *)f.v + co) + (cx0 + x0 / 2) / 4);
-        *(uint2 *)(J.u16 + (size_t)cy * cw + cx0) = make_uint2(u.x << up, u.y << up);
-        *(uint2 *)(J.v16 + (size_t)cy * cw + cx0) = make_uint2(v.x << up, v.y << up);
+        uint2 u, v;
+        if (f.semi) {  // (U, V) pairs
+            const uint4 q = load8((const unsigned char *)f.u + co + (size_t)(2 * cx0 + x0) * f.bytes, f.bytes);
+            u = make_uint2(__byte_perm(q.x, q.y, 0x5410), __byte_perm(q.z, q.w, 0x5410));
+            v = make_uint2(__byte_perm(q.x, q.y, 0x7632), __byte_perm(q.z, q.w, 0x7632));
+        } else {
+            u = load4((const unsigned char *)f.u + co + (size_t)(cx0 + x0 / 2) * f.bytes, f.bytes);
+            v = load4((const unsigned char *)f.v + co + (size_t)(cx0 + x0 / 2) * f.bytes, f.bytes);
+        }
+#pragma unroll
+        for (int dy = 0; dy < 2; dy++)
+            store8(J.y16 + (size_t)(2 * cy + dy) * J.w + 2 * cx0, make_uint4(put(y[dy].x), put(y[dy].y), put(y[dy].z), put(y[dy].w)));
+        store4(J.u16 + (size_t)cy * cw + cx0, make_uint2(put(u.x), put(u.y)));
+        store4(J.v16 + (size_t)cy * cw + cx0, make_uint2(put(v.x), put(v.y)));
         return;
     }
-    if (full && f.bytes == 1 && (f.ypitch & 7) == 0 && (f.cpitch & 3) == 0 && (((uintptr_t)f.y & 7) | ((uintptr_t)f.u & 3) | ((uintptr_t)f.v & 3)) == 0 &&
-        (J.w & 7) == 0) {
-        auto widen2 = [&](unsigned q) {  // 4 bytes -> 4 16-bit samples, shifted
-            return make_uint2(__byte_perm(q, 0, 0x4140) << up, __byte_perm(q, 0, 0x4342) << up);
-        };
-#pragma unroll
-        for (int dy = 0; dy < 2; dy++) {
-            const uint2 q = __ldg((const uint2 *)((const unsigned char *)f.y + (size_t)(2 * cy + dy + y0) * f.ypitch) + (2 * cx0 + x0) / 8);
-            const uint2 lo = widen2(q.x), hi = widen2(q.y);
-            *(uint4 *)(J.y16 + (size_t)(2 * cy + dy) * J.w + 2 * cx0) = make_uint4(lo.x, lo.y, hi.x, hi.y);
-        }
-        const size_t co = (size_t)(cy + y0 / 2) * f.cpitch;
-        const unsigned u = __ldg((const unsigned *)((const unsigned char *)f.u + co) + (cx0 + x0 / 2) / 4);
-        const unsigned v = __ldg((const unsigned *)((const unsigned char *)f.v + co) + (cx0 + x0 / 2) / 4);
-        *(uint2 *)(J.u16 + (size_t)cy * cw + cx0) = widen2(u);
-        *(uint2 *)(J.v16 + (size_t)cy * cw + cx0) = widen2(v);
-        return;
-    }
-    for (int cx = cx0; cx < min(cx0 + 4, cw); cx++) {
+    for (int cx = cx0; cx < cw; cx++) {
 #pragma unroll
         for (int dy = 0; dy < 2; dy++) {
             const int y = 2 * cy + dy;
