@@ -390,6 +390,11 @@ void record_cambi(es_batch &b, long f, uint32_t skip, cudaStream_t s)
         }
     }
     pb.band = band;
+    const int nslots = (int)b.pictures.size() * kScales;
+    pb.slots = b.slots.ptr;
+    pb.nslots = nslots;
+    pb.slot_n = b.slot_n.ptr;
+    pb.slot_k = b.slot_k.ptr;
     cuda_check(launch_prep0(pb, s), "batch scales 0 and 1");
     CvBatch cb{};
     int tiles = 0;
@@ -426,26 +431,19 @@ void record_cambi(es_batch &b, long f, uint32_t skip, cudaStream_t s)
         ab = record_proposal_lists(b, run, cb, a);
         if (split) cuda_check(cudaEventRecord(b.join_aux.e, a), "event");
     }
-    const int nslots = (int)b.pictures.size() * kScales;
-    cuda_check(launch_slots_reset(b.slots.ptr, nslots, b.slot_n.ptr, b.slot_k.ptr, s), "batch reset");
-    for (int sc = 2; sc < kScales; sc++) {
-        DecBatch db{};
-        int blocks = 0;
-        for (int i : run) {
-            const Picture &pic = *b.pictures[i];
-            DecJob &dj = db.job[db.njobs++];
-            dj.src = pic.words[sc - 1].ptr;
-            dj.sw = pic.sw[sc - 1];
-            dj.sh = pic.sh[sc - 1];
-            dj.dst = pic.words[sc].ptr;
-            dj.w = pic.sw[sc];
-            dj.h = pic.sh[sc];
-            dj.first_block = blocks;
-            blocks += (dj.w * dj.h + 255) / 256;
+    DecBatch db{};
+    for (int i : run) {
+        const Picture &pic = *b.pictures[i];
+        DecJob &dj = db.job[db.njobs++];
+        dj.src = pic.words[1].ptr;
+        dj.sw = pic.sw[1];
+        for (int sc = 2; sc < kScales; sc++) {
+            dj.dst[sc - 2] = pic.words[sc].ptr;
+            dj.w[sc - 2] = pic.sw[sc];
+            dj.h[sc - 2] = pic.sh[sc];
         }
-        db.total_blocks = blocks;
-        cuda_check(launch_decimate_mode(db, s), "batch scales");
     }
+    cuda_check(launch_decimate_mode(db, s), "batch scales");
     if (!b.net) {
         cuda_check(launch_cvalues(cb, s), "batch c-values");
     } else {
@@ -459,11 +457,10 @@ void record_cambi(es_batch &b, long f, uint32_t skip, cudaStream_t s)
         j.first_slot = i * kScales;
         j.window = b.pictures[i]->p.window;
         j.score = b.scores.ptr + (size_t)i * (1 + kScales);
+        j.host = b.h_scores[f % 2].ptr + (size_t)i * (1 + kScales);
     }
     sb.slots = b.slots.ptr;
     cuda_check(launch_score(sb, s), "batch score");
-    cuda_check(cudaMemcpyAsync(b.h_scores[f % 2].ptr, b.scores.ptr, b.scores.bytes(), cudaMemcpyDeviceToHost, s),
-               "reading scores");
     if (b.net)
         cuda_check(cudaMemcpyAsync(b.h_stats[f % 2].ptr, b.stats.ptr, b.stats.bytes(), cudaMemcpyDeviceToHost, s), "reading proposal stats");
 }

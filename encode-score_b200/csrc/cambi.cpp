@@ -1,8 +1,8 @@
 // es_cambi: CAMBI of one plane per launch, the C-ABI form of class Cambi (src/cambi.hpp:9-21, src/cambi.cpp:31-184).
 //
-// launch() queues the fused scale-0 kernel on the caller's stream (it reads the caller's plane, which is then free to
-// be overwritten), then the scales, c-values, device-side top-k selection and score on the instance's own stream,
-// ending with one 48-byte copy of the score and per-scale pooled values to page-locked memory. finish() only waits.
+// launch() queues the fused kernel of scales 0 and 1 on the caller's stream (it reads the caller's plane, which is then
+// free to be overwritten), then the other scales, c-values, device-side top-k selection and score on the instance's own
+// stream; the score kernel writes the score and per-scale pooled values to page-locked memory. finish() only waits.
 #include <cstring>
 #include <vector>
 
@@ -92,25 +92,25 @@ void queue_cambi(es_cambi *c, uint64_t img, int pitch, cudaStream_t caller)
     pj.word1 = c->words[1].ptr;
     pj.w1 = c->sw[1];
     pj.h1 = c->sh[1];
+    pb.slots = c->slots.ptr;
+    pb.nslots = kScales;
+    pb.slot_n = c->slot_n.ptr;
+    pb.slot_k = c->slot_k.ptr;
     cuda_check(launch_prep0(pb, caller), "cambi scales 0 and 1");
     cuda_check(cudaEventRecord(c->copied.e, caller), "cambi event");
     cudaStream_t s = serial_streams() ? caller : c->stream.s;
     cuda_check(cudaStreamWaitEvent(s, c->copied.e, 0), "cambi event");
-    cuda_check(launch_slots_reset(c->slots.ptr, kScales, c->slot_n.ptr, c->slot_k.ptr, s), "cambi reset");
+    DecBatch db{};
+    db.njobs = 1;
+    DecJob &dj = db.job[0];
+    dj.src = c->words[1].ptr;
+    dj.sw = c->sw[1];
     for (int sc = 2; sc < kScales; sc++) {
-        DecBatch db{};
-        db.njobs = 1;
-        DecJob &dj = db.job[0];
-        dj.src = c->words[sc - 1].ptr;
-        dj.sw = c->sw[sc - 1];
-        dj.sh = c->sh[sc - 1];
-        dj.dst = c->words[sc].ptr;
-        dj.w = c->sw[sc];
-        dj.h = c->sh[sc];
-        dj.first_block = 0;
-        db.total_blocks = (dj.w * dj.h + 255) / 256;
-        cuda_check(launch_decimate_mode(db, s), "cambi scales");
+        dj.dst[sc - 2] = c->words[sc].ptr;
+        dj.w[sc - 2] = c->sw[sc];
+        dj.h[sc - 2] = c->sh[sc];
     }
+    cuda_check(launch_decimate_mode(db, s), "cambi scales");
     CvBatch cb{};
     cb.njobs = kScales;
     int tiles = 0;
@@ -150,10 +150,9 @@ void queue_cambi(es_cambi *c, uint64_t img, int pitch, cudaStream_t caller)
     sb.job[0].first_slot = 0;
     sb.job[0].window = p.window;
     sb.job[0].score = c->score.ptr;
+    sb.job[0].host = c->host.ptr;
     sb.slots = c->slots.ptr;
     cuda_check(launch_score(sb, s), "cambi score");
-    cuda_check(cudaMemcpyAsync(c->host.ptr, c->score.ptr, sizeof(double) * (1 + kScales), cudaMemcpyDeviceToHost, s),
-               "reading the score");
     cuda_check(cudaEventRecord(c->finished.e, s), "cambi event");
 }
 

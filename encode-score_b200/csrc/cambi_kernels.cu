@@ -7,11 +7,13 @@
 //  * prep0_kernel fuses the 8-to-10-bit conversion (or copy), the 7x7 flat-pixel count and the 3x3 mode filter of
 //    scale 0 in one pass over a shared-memory tile, and packs each pixel as value | mask << 15, so every later step
 //    reads one 16-bit word per pixel;
-//  * decimate_mode_kernel builds scales 1-4 the same way from the previous scale's words;
+//  * the same kernel makes scale 1 and clears the counters; decimate_mode_kernel builds scales 2-4 from scale 1's words;
 //  * the c-values themselves are in cvalues_kernels.cu;
-//  * select_hist_kernel / select_pick_kernel find the exact k-th largest value, and the sum above it, on the device
-//    when more than k values are positive (no host round trips; the first radix digit is counted by the c-value
-//    kernel), and score_kernel pools and weights the scales.
+//  * two launches of select_kernel and the score kernel find the exact k-th largest value, and the sum above it, on the
+//    device when more than k values are positive (no host round trips; the first radix digit is counted by the c-value
+//    kernel); the score kernel also pools and weights the scales and writes the score to the host's memory.
+// A picture is five launches after the last one's input is there. They were twelve and a copy: a launch takes 2.5 to 5 us
+// of host time and 3 to 5 us on the GPU here, as long as the work of most of them.
 #include "cambi_codes.h"
 #include "es_kernels.h"
 
@@ -76,6 +78,18 @@ __device__ __forceinline__ uint32_t mode3x2(uint32_t a, uint32_t b, uint32_t c)
 
 __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ Prep0Batch b)
 {
+    if ((int)blockIdx.x >= b.total_tiles) {  // the blocks after the tiles clear the counters, a slot each
+        const int i = blockIdx.x - b.total_tiles;
+        CvSlot &S = b.slots[i];
+        for (int k = threadIdx.x; k < 2048 / 4; k += 256) ((uint4 *)S.hist)[k] = make_uint4(0, 0, 0, 0);
+        if (threadIdx.x == 0) {
+            S.sum_fx = S.count = S.list_n = 0;
+            S.n = b.slot_n[i];
+            S.k = b.slot_k[i];
+            S.above_fx = S.above_n = 0;
+        }
+        return;
+    }
     __shared__ __align__(16) uint16_t buf[2][kP0R][kP0C];  // [0]: the staged plane; [1]: 8-bit planes at 10 bits
     __shared__ uint32_t flatbits[kP0FR][4];                // 3 words of bits and a zero word
     __shared__ uint16_t dw[kP0D][kP0D];                    // scale-0 words at even positions, for scale 1
@@ -320,91 +334,169 @@ __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ P
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Scales 1-4: src/kernels.cu:43-53 (decimate) and 488-500 (mode) on the decimated picture, mask decimated alongside.
-// A block of 256 threads makes a 64 x 16 tile: the decimated words of the tile and a 1-pixel margin (the even rows
-// and columns of the previous scale, 4-byte loads keeping the even half) are staged in shared memory; thread (c, g)
-// then makes column c of rows 4 g .. 4 g + 3 from 6 horizontal modes.
+// Scales 2-4: src/kernels.cu:43-53 (decimate) and 488-500 (mode) on the decimated picture, mask decimated alongside, all
+// three in one launch: a block of 256 threads makes a 64 x 32 tile of scale 2 and the 32 x 16 and 16 x 8 tiles of scales
+// 3 and 4 beneath it. A scale's 3 x 3 filter reads its decimated neighbours, so the tile grows by 2 words a side per
+// scale above; the block makes those margins itself (a word of scale 2 in 1.5 is made twice; the three scales are a
+// twelfth of scale 0). Bound by latency: one launch of 10 us for two 4K pictures instead of three of 9.5.
 // ---------------------------------------------------------------------------------------------------------------
-constexpr int kDTW = 64, kDTH = 16;
+constexpr int kDTW = 64, kDTH = 32;                        // scale-2 tile
+constexpr int kD2W = kDTW + 12, kD2H = kDTH + 12;          // scale 2's decimated words from (x - 6 - 1, y - 6 - 1), 1 more
+constexpr int kF2W = kD2W - 2, kF2H = kD2H - 2;            // scale 2 filtered, from (x - 6, y - 6)
+constexpr int kF3W = kDTW / 2 + 3, kF3H = kDTH / 2 + 3;    // scale 3 filtered, from (x / 2 - 2, y / 2 - 2)
+
+// The 3 x 3 mode filter of N rows of one column: d points at the column's word in the row above the first, rows `stride`
+// apart; (x, y) is the first row's place in a w x h picture. Columns and rows on the picture's edge keep their value in
+// their direction, and a word keeps its mask. put(i, word) gets row i's word.
+template <int N, typename Put>
+__device__ __forceinline__ void mode_column(const uint16_t *d, int stride, int x, int y, int w, int h, Put put)
+{
+    const bool edge = x == 0 || x == w - 1;
+    auto hm = [&](const uint16_t *r) -> uint16_t {
+        const uint16_t m = r[0] & 0x7FFF;
+        return edge ? m : mode3(r[-1] & 0x7FFF, m, r[1] & 0x7FFF);
+    };
+    uint16_t m0 = hm(d), m1 = hm(d + stride);
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const uint16_t c = d[(i + 1) * stride], m2 = hm(d + (i + 2) * stride);
+        const bool keep = y + i == 0 || y + i == h - 1;
+        put(i, (uint16_t)((keep ? c & 0x7FFF : mode3(m0, m1, m2)) | (c & kMaskBit)));
+        m0 = m1;
+        m1 = m2;
+    }
+}
 
 __global__ void __launch_bounds__(256) decimate_mode_kernel(const __grid_constant__ DecBatch b)
 {
-    __shared__ uint16_t d[kDTH + 2][kDTW + 2];
+    __shared__ uint16_t d2[kD2H][kD2W], f2[kF2H][kF2W], d3[kF3H + 2][kF3W + 2], f3[kF3H][kF3W], d4[kDTH / 4 + 2][kDTW / 4 + 2];
     const int j = find_job(b.njobs, (int)blockIdx.x, [&](int k) { return b.job[k].first_block; });
     const DecJob &J = b.job[j];
-    const int w = J.w, h = J.h, tiles_x = (w + kDTW - 1) / kDTW, t = blockIdx.x - J.first_block;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tiles_x = (J.w[0] + kDTW - 1) / kDTW, t = blockIdx.x - J.first_block;
     const int x0 = (t % tiles_x) * kDTW, y0 = (t / tiles_x) * kDTH;
-    for (int i = threadIdx.x; i < (kDTH + 2) * (kDTW + 2); i += 256) {
-        const int r = i / (kDTW + 2), c = i - r * (kDTW + 2), X = x0 - 1 + c, Y = y0 - 1 + r;
-        uint16_t v = 0;
-        if (X >= 0 && X < w && Y >= 0 && Y < h) {  // word (2 X, 2 Y) of the previous scale
-            const uint16_t *p = J.src + (size_t)(2 * Y) * J.sw + 2 * X;
-            // the low half of a 4-byte load, unless the word ends an odd-width row (the high half would be past it)
-            v = 2 * X + 1 < J.sw ? (uint16_t)(__ldg((const unsigned *)p) & 0xFFFFu) : *p;
+    for (int r = warp; r < kD2H; r += 8) {
+        const int Y = y0 - 7 + r;
+        const uint16_t *row = J.src + (size_t)(2 * Y) * J.sw;
+#pragma unroll
+        for (int c = lane; c < kD2W; c += 32) {
+            const int X = x0 - 7 + c;  // word (2 X, 2 Y) of scale 1
+            d2[r][c] = (X >= 0 && X < J.w[0] && Y >= 0 && Y < J.h[0]) ? __ldg(row + 2 * X) : (uint16_t)0;
         }
-        d[r][c] = v;
     }
     __syncthreads();
-    const int c = threadIdx.x & (kDTW - 1), r0 = (threadIdx.x >> 6) * 4, x = x0 + c;
-    if (x >= w) return;
-    auto val = [&](int r, int cc) -> uint16_t { return d[r][cc] & 0x7FFF; };
-    const bool edge_x = x == 0 || x == w - 1;
-    uint16_t hm[6];  // horizontal modes of tile rows r0 - 1 .. r0 + 4 (staged rows r0 .. r0 + 5)
-#pragma unroll
-    for (int k = 0; k < 6; k++)
-        hm[k] = edge_x ? val(r0 + k, c + 1) : mode3(val(r0 + k, c), val(r0 + k, c + 1), val(r0 + k, c + 2));
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int y = y0 + r0 + i;
-        if (y >= h) break;
-        const uint16_t word = d[r0 + i + 1][c + 1];
-        const uint16_t v = (y == 0 || y == h - 1) ? (uint16_t)(word & 0x7FFF) : mode3(hm[i], hm[i + 1], hm[i + 2]);
-        J.dst[(size_t)y * w + x] = (uint16_t)(v | (word & kMaskBit));
+    // scale 2: a thread per column and 14 rows. Its words at even positions are scale 3's decimated words: (X, Y) is
+    // f2[2 (Y - y0 / 2) + 6][2 (X - x0 / 2) + 6]
+    static_assert(kF2H == 3 * 14 && kF2W * 3 <= 256, "three threads per column");
+    if (tid < kF2W * 3) {
+        const int seg = tid / kF2W, c = tid - seg * kF2W, r0 = 14 * seg, X = x0 - 6 + c, Y = y0 - 6 + r0;
+        if (X >= 0 && X < J.w[0])
+            mode_column<14>(&d2[r0][c + 1], kD2W, X, Y, J.w[0], J.h[0], [&](int i, uint16_t v) {
+                f2[r0 + i][c] = v;
+                if (X >= x0 && X < x0 + kDTW && Y + i >= y0 && Y + i < y0 + kDTH && Y + i < J.h[0]) J.dst[0][(size_t)(Y + i) * J.w[0] + X] = v;
+            });
+    }
+    __syncthreads();
+    static_assert(2 * (kF3W + 1) < kF2W && 2 * (kF3H + 1) < kF2H, "scale 3's margins lie in scale 2's");
+    for (int r = warp; r < kF3H + 2; r += 8)
+        for (int c = lane; c < kF3W + 2; c += 32) d3[r][c] = f2[2 * r][2 * c];  // from (x / 2 - 3, y / 2 - 3)
+    __syncthreads();
+    static_assert(kF3H == 19 && kF3W * 7 <= 256, "seven threads per column of scale 3, 3 rows each");
+    if (tid < kF3W * 7) {
+        const int seg = tid / kF3W, c = tid - seg * kF3W, r0 = min(3 * seg, kF3H - 3), X = x0 / 2 - 2 + c, Y = y0 / 2 - 2 + r0;
+        if (X >= 0 && X < J.w[1])
+            mode_column<3>(&d3[r0][c + 1], kF3W + 2, X, Y, J.w[1], J.h[1], [&](int i, uint16_t v) {
+                const int r = r0 + i;
+                f3[r][c] = v;
+                if (c >= 2 && c < 2 + kDTW / 2 && r >= 2 && r < 2 + kDTH / 2 && Y + i < J.h[1]) J.dst[1][(size_t)(Y + i) * J.w[1] + X] = v;
+            });
+    }
+    __syncthreads();
+    for (int i = tid; i < (kDTH / 4 + 2) * (kDTW / 4 + 2); i += 256) {
+        const int r = i / (kDTW / 4 + 2), c = i - r * (kDTW / 4 + 2);
+        d4[r][c] = f3[2 * r][2 * c];  // from (x / 4 - 1, y / 4 - 1)
+    }
+    __syncthreads();
+    if (tid < (kDTW / 4) * (kDTH / 4)) {
+        const int r = tid / (kDTW / 4), c = tid % (kDTW / 4), X = x0 / 4 + c, Y = y0 / 4 + r;
+        if (X < J.w[2] && Y < J.h[2])
+            mode_column<1>(&d4[r][c + 1], kDTW / 4 + 2, X, Y, J.w[2], J.h[2], [&](int, uint16_t v) { J.dst[2][(size_t)Y * J.w[2] + X] = v; });
     }
 }
 
 // ---------------------------------------------------------------------------------------------------------------
 // Pooling: src/cambi.cpp:137-184 with the radix rounds on the device.
 // ---------------------------------------------------------------------------------------------------------------
-struct SlotInit {
-    unsigned long long n, k;
-};
-
-__global__ void slots_reset_kernel(CvSlot *slots, int nslots, const unsigned long long *n, const unsigned long long *k)
-{
-    const int s = blockIdx.x;
-    if (s >= nslots) return;
-    CvSlot &S = slots[s];
-    for (int i = threadIdx.x; i < 2048; i += blockDim.x) S.hist[i] = 0;
-    for (int i = threadIdx.x; i < 1024; i += blockDim.x) S.dsum[i] = 0;
-    if (threadIdx.x == 0) {
-        S.sum_fx = S.count = S.list_n = 0;
-        S.n = n[s];
-        S.k = k[s];
-        S.remaining = k[s];
-        S.above_fx = S.above_n = 0;
-        S.prefix = S.mask = 0;
-    }
-}
-
 // A positive c-value in units of 2^-24 (exact: c-values are multiples of 2^-24).
 __device__ __forceinline__ unsigned long long fx_of(unsigned bits) { return __float2ull_rn(__fmul_rn(__uint_as_float(bits), 16777216.0f)); }
 
-// One radix round over every slot whose positive count exceeds k (the first round's counts come from the c-value
-// kernel); block b takes the b-th share of each such slot's list. One block of kSelThreads per SM: each block merges
-// one shared histogram per slot into the slot's, so fewer, larger blocks mean fewer global atomics for the same reads.
-// The last round (last = 1) also sums, per digit, the values that match the prefix (they are equal when their digits
-// are), and the values whose prefix is greater than the selected one (all of them lie above the k-th value).
 constexpr int kSelThreads = 1024, kSelBlocks = 148;
 
-__global__ void __launch_bounds__(kSelThreads) select_hist_kernel(CvSlot *slots, int nslots, int shift, int width, int last)
+// The digit of the `remaining`-th largest value from the counts of nb = 2 kSelThreads digits, and the values above that
+// digit (called by a whole block; every block of a launch finds the same).
+struct Picked {
+    unsigned digit;
+    unsigned long long above;
+};
+__device__ Picked pick_digit(const unsigned *hist, unsigned long long remaining, unsigned long long (&warp_tot)[32], Picked &found)
 {
-    __shared__ unsigned hist[2048];
-    __shared__ unsigned long long dsum[1024];
-    const int nb = 1 << width;
-    for (int sl = 0; sl < nslots; sl++) {
-        CvSlot &S = slots[sl];
-        if (S.count <= S.k) continue;  // the same for the whole block
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int top = 2 * kSelThreads - 1 - 2 * tid;  // this thread: digits top and top - 1
+    const unsigned long long c0 = hist[top], c1 = hist[top - 1];
+    unsigned long long incl = c0 + c1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) warp_tot[warp] = incl;
+    __syncthreads();
+    unsigned long long before = incl - c0 - c1;
+    for (int k = 0; k < warp; k++) before += warp_tot[k];
+    if (before < remaining && before + c0 + c1 >= remaining) {
+        const bool second = before + c0 < remaining;
+        found.digit = (unsigned)(second ? top - 1 : top);
+        found.above = before + (second ? c0 : 0);
+    }
+    __syncthreads();
+    return found;
+}
+
+// A radix round over every slot whose positive count exceeds k: each block picks the digit of the round before (round 1:
+// the c-value kernel's counts, 11 bits; round 2: 11 bits), then counts the next one (round 1: 11 bits, round 2: 10) over
+// its share of the slot's list. One block of kSelThreads per SM: each merges one shared histogram per slot into the
+// slot's, so fewer, larger blocks mean fewer global atomics for the same reads. Round 2 also sums, per digit, the values
+// that match the prefix (they are equal when their digits are), and the values whose prefix is greater than the selected
+// one (all of them lie above the k-th value). What it writes of the state (block 0) is read by the next launch only.
+template <int kRound>
+__global__ void __launch_bounds__(kSelThreads) select_kernel(CvSlot *slots, int nslots)
+{
+    constexpr bool last = kRound == 2;
+    constexpr int shift = last ? 0 : 10, nb = last ? 1024 : 2048;
+    __shared__ unsigned hist[nb];
+    __shared__ unsigned long long dsum[last ? 1024 : 1];
+    __shared__ unsigned long long warp_tot[32];
+    __shared__ Picked found;
+    __shared__ int todo[kMaxJobs], ntodo;
+    if (threadIdx.x == 0) ntodo = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < nslots; i += kSelThreads)
+        if (slots[i].count > slots[i].k) todo[atomicAdd(&ntodo, 1)] = i;
+    __syncthreads();
+    for (int it = 0; it < ntodo; it++) {
+        CvSlot &S = slots[todo[it]];
+        const unsigned long long remaining = last ? S.remaining1 : S.k;
+        const Picked p = pick_digit(last ? S.hist1 : S.hist, remaining, warp_tot, found);
+        const unsigned prefix = last ? S.prefix1 | (p.digit << 10) : p.digit << 21, mask = last ? 0xFFFFFC00u : 0xFFE00000u;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            if (last) {
+                S.prefix2 = prefix;
+                S.remaining2 = remaining - p.above;
+            } else {
+                S.prefix1 = prefix;
+                S.remaining1 = remaining - p.above;
+            }
+        }
         for (int i = threadIdx.x; i < nb; i += kSelThreads) {
             hist[i] = 0;
             if (last) dsum[i] = 0;
@@ -412,7 +504,6 @@ __global__ void __launch_bounds__(kSelThreads) select_hist_kernel(CvSlot *slots,
         __syncthreads();
         const unsigned *v = (const unsigned *)S.list;
         const unsigned long long n = S.list_n, n4 = n / 4, stride = (unsigned long long)gridDim.x * kSelThreads;
-        const unsigned mask = S.mask, prefix = S.prefix;
         unsigned long long above_fx = 0, above_n = 0;
         // neighbouring c-values of the list are often equal (they come from the same tile), so each thread adds runs
         // of equal digits at once; 4 values per 16-byte load
@@ -474,103 +565,84 @@ __global__ void __launch_bounds__(kSelThreads) select_hist_kernel(CvSlot *slots,
         }
         __syncthreads();
         for (int i = threadIdx.x; i < nb; i += kSelThreads) {
-            if (hist[i]) atomicAdd(&S.hist[i], hist[i]);
+            if (hist[i]) atomicAdd(last ? &S.hist2[i] : &S.hist1[i], hist[i]);
             if (last && dsum[i]) atomicAdd(&S.dsum[i], dsum[i]);
         }
         __syncthreads();
     }
 }
 
-// Picks the digit of the k-th largest value from a round's counts; the last round then adds the values of the greater
-// digits to the sum and count above it.
-__global__ void __launch_bounds__(256) select_pick_kernel(CvSlot *slots, int shift, int width, int last)
+// A block per picture, a warp per scale: the last digit of a slot with more than k positive values, from round 2's counts,
+// and the sum above it (the counters of both rounds are left clear); then the scales' pooled values and the score, to
+// device memory and, where the job has a place, to the host's.
+__global__ void __launch_bounds__(32 * kScales) score_kernel(const __grid_constant__ ScoreBatch b)
 {
-    CvSlot &S = slots[blockIdx.x];
-    if (S.count <= S.k) return;
-    __shared__ unsigned long long part[256];
-    __shared__ int picked;
-    const int nb = 1 << width, per = nb / 256, t = threadIdx.x;
-    if (t == 0) picked = 0;
-    // thread t holds the digits nb - (t + 1) per .. nb - t per - 1, counted from the top
-    const int top = nb - t * per - 1;
-    unsigned long long mine = 0;
-    for (int d = 0; d < per; d++) mine += S.hist[top - d];
-    part[t] = mine;
-    __syncthreads();
-    // exclusive sum of the counts above this thread's digits (256 entries, a simple serial-per-thread scan)
-    unsigned long long above = 0;
-    for (int k = 0; k < t; k++) above += part[k];
-    const unsigned long long remaining = S.remaining;
-    __syncthreads();
-    if (above < remaining && above + mine >= remaining) {
+    __shared__ double part[kScales];
+    const ScoreJob &J = b.job[blockIdx.x];
+    const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
+    CvSlot &S = b.slots[J.first_slot + s];
+    const unsigned long long count = S.count, k = S.k;
+    double pooled;
+    if (count <= k) {
+        pooled = __ddiv_rn(__dmul_rn(__ull2double_rn(S.sum_fx), 1.0 / 16777216.0), __ull2double_rn(k));
+    } else {
+        const unsigned long long remaining = S.remaining2;
+        // lane l: digits 1023 - 32 l down to 992 - 32 l
+        const int top = 1023 - 32 * lane;
+        unsigned long long mine = 0, fx = 0;
+#pragma unroll 8
+        for (int d = 0; d < 32; d++) {
+            mine += S.hist2[top - d];
+            fx += S.dsum[top - d];
+        }
+        unsigned long long cincl = mine, fincl = fx;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long c = __shfl_up_sync(0xffffffffu, cincl, o), f = __shfl_up_sync(0xffffffffu, fincl, o);
+            if (lane >= o) {
+                cincl += c;
+                fincl += f;
+            }
+        }
+        unsigned long long above_n = cincl - mine, above_fx = fincl - fx;
+        const bool here = above_n < remaining && cincl >= remaining;
         int digit = top;
-        for (int d = 0; d < per; d++, digit--) {
-            const unsigned c = S.hist[digit];
-            if (above + c >= remaining || digit == 0) break;
-            above += c;
+        if (here) {
+            for (int d = 0; d < 31; d++, digit--) {
+                const unsigned c = S.hist2[digit];
+                if (above_n + c >= remaining) break;
+                above_n += c;
+                above_fx += S.dsum[digit];
+            }
         }
-        S.remaining = remaining - above;
-        S.prefix |= (unsigned)digit << shift;
-        S.mask |= (unsigned)(nb - 1) << shift;
-        picked = digit;
+        const unsigned who = __ballot_sync(0xffffffffu, here);
+        const int src = __ffs(who) - 1;
+        digit = __shfl_sync(0xffffffffu, digit, src);
+        above_n = __shfl_sync(0xffffffffu, above_n, src) + S.above_n;
+        above_fx = __shfl_sync(0xffffffffu, above_fx, src) + S.above_fx;
+        const unsigned kth = S.prefix2 | (unsigned)digit;
+        const double above = __dmul_rn(__ull2double_rn(above_fx), 1.0 / 16777216.0);
+        const double rest = __dmul_rn(__ull2double_rn(k - above_n), (double)__uint_as_float(kth));
+        pooled = __ddiv_rn(__dadd_rn(above, rest), __ull2double_rn(k));
+        __syncwarp();
+        for (int i = lane; i < 2048 / 4; i += 32) ((uint4 *)S.hist1)[i] = make_uint4(0, 0, 0, 0);
+        for (int i = lane; i < 1024 / 4; i += 32) ((uint4 *)S.hist2)[i] = make_uint4(0, 0, 0, 0);
+        for (int i = lane; i < 1024 / 2; i += 32) ((uint4 *)S.dsum)[i] = make_uint4(0, 0, 0, 0);
+    }
+    if (lane == 0) {
+        part[s] = pooled;
+        J.score[1 + s] = pooled;
+        if (J.host) J.host[1 + s] = pooled;
     }
     __syncthreads();
-    if (last) {
-        // the values of the digits above the picked one: their sums and counts, added to those of greater prefixes
-        const int D = picked;
-        unsigned long long fx = 0, cnt = 0;
-        for (int d = D + 1 + t; d < nb; d += 256) {
-            fx += S.dsum[d];
-            cnt += S.hist[d];
-        }
-        part[t] = fx;
-        __syncthreads();
-        for (int o = 128; o; o >>= 1) {
-            if (t < o) part[t] += part[t + o];
-            __syncthreads();
-        }
-        const unsigned long long fx_all = part[0];
-        __syncthreads();
-        part[t] = cnt;
-        __syncthreads();
-        for (int o = 128; o; o >>= 1) {
-            if (t < o) part[t] += part[t + o];
-            __syncthreads();
-        }
-        if (t == 0) {
-            S.above_fx += fx_all;
-            S.above_n += part[0];
-        }
-        __syncthreads();
-        for (int i = t; i < nb; i += 256) S.dsum[i] = 0;
-    }
-    for (int i = t; i < nb; i += 256) S.hist[i] = 0;
-}
-
-__global__ void score_kernel(const __grid_constant__ ScoreBatch b)
-{
-    const int j = threadIdx.x;
-    if (j >= b.njobs) return;
-    const ScoreJob &J = b.job[j];
-    const double kScaleWeight[kScales] = {16.0, 8.0, 4.0, 2.0, 1.0};
+    if (threadIdx.x != 0) return;
     double total = 0.0;
-    for (int s = 0; s < kScales; s++) {
-        const CvSlot &S = b.slots[J.first_slot + s];
-        const double k = __ull2double_rn(S.k);
-        double pooled;
-        if (S.count <= S.k) {
-            pooled = __ddiv_rn(__dmul_rn(__ull2double_rn(S.sum_fx), 1.0 / 16777216.0), k);
-        } else {
-            const double above = __dmul_rn(__ull2double_rn(S.above_fx), 1.0 / 16777216.0);
-            const double rest = __dmul_rn(__ull2double_rn(S.k - S.above_n), (double)__uint_as_float(S.prefix));
-            pooled = __ddiv_rn(__dadd_rn(above, rest), k);
-        }
-        total = __dadd_rn(total, __dmul_rn(pooled, kScaleWeight[s]));
-        J.score[1 + s] = pooled;
-    }
+    const double kScaleWeight[kScales] = {16.0, 8.0, 4.0, 2.0, 1.0};
+    for (int q = 0; q < kScales; q++) total = __dadd_rn(total, __dmul_rn(part[q], kScaleWeight[q]));
     const int odd = 2 * (J.window >> 1) + 1;
     const double score = __ddiv_rn(total, (double)(odd * odd));
     J.score[0] = score < 1000.0 ? score : 1000.0;
+    if (J.host) J.host[0] = J.score[0];
 }
 
 }  // namespace
@@ -598,7 +670,7 @@ cudaError_t launch_prep0(Prep0Batch &b, cudaStream_t s)
     b.need_lo = lo < 0 ? 0 : lo + b.band.band_base;
     b.need_span = !one_range ? -1 : lo < 0 ? -1 : hi - lo;
     LaunchTimer t("cambi_prep0", s);
-    prep0_kernel<<<b.total_tiles, 256, 0, s>>>(b);
+    prep0_kernel<<<b.total_tiles + b.nslots, 256, 0, s>>>(b);
     return after_launch();
 }
 
@@ -607,51 +679,33 @@ cudaError_t launch_decimate_mode(DecBatch &b, cudaStream_t s)
     int blocks = 0;
     for (int j = 0; j < b.njobs; j++) {
         b.job[j].first_block = blocks;
-        blocks += ((b.job[j].w + kDTW - 1) / kDTW) * ((b.job[j].h + kDTH - 1) / kDTH);
+        blocks += ((b.job[j].w[0] + kDTW - 1) / kDTW) * ((b.job[j].h[0] + kDTH - 1) / kDTH);
     }
-    b.total_blocks = blocks;
-    if (b.total_blocks <= 0) return cudaSuccess;
+    if (blocks <= 0) return cudaSuccess;
     LaunchTimer t("cambi_decimate_mode", s);
-    decimate_mode_kernel<<<b.total_blocks, 256, 0, s>>>(b);
-    return after_launch();
-}
-
-cudaError_t launch_slots_reset(CvSlot *slots, int nslots, const unsigned long long *n, const unsigned long long *k,
-                               cudaStream_t s)
-{
-    if (nslots <= 0) return cudaSuccess;
-    LaunchTimer t("cambi_reset", s);
-    slots_reset_kernel<<<nslots, 256, 0, s>>>(slots, nslots, n, k);
+    decimate_mode_kernel<<<blocks, 256, 0, s>>>(b);
     return after_launch();
 }
 
 cudaError_t launch_topk(CvSlot *slots, int nslots, cudaStream_t s)
 {
     if (nslots <= 0) return cudaSuccess;
-    static const int shifts[3] = {21, 10, 0}, widths[3] = {11, 11, 10};
-    for (int round = 0; round < 3; round++) {
-        const int last = round == 2;
-        if (round > 0) {  // the first round's counts were made by the c-value kernel
-            LaunchTimer t("cambi_select_hist", s);
-            select_hist_kernel<<<kSelBlocks, kSelThreads, 0, s>>>(slots, nslots, shifts[round], widths[round], last);
-        }
-        cudaError_t e = round > 0 ? after_launch() : cudaSuccess;
-        if (e != cudaSuccess) return e;
-        {
-            LaunchTimer t("cambi_select_pick", s);
-            select_pick_kernel<<<nslots, 256, 0, s>>>(slots, shifts[round], widths[round], last);
-        }
-        e = after_launch();
-        if (e != cudaSuccess) return e;
+    {
+        LaunchTimer t("cambi_select", s);
+        select_kernel<1><<<kSelBlocks, kSelThreads, 0, s>>>(slots, nslots);
     }
-    return cudaSuccess;
+    const cudaError_t e = after_launch();
+    if (e != cudaSuccess) return e;
+    LaunchTimer t("cambi_select", s);
+    select_kernel<2><<<kSelBlocks, kSelThreads, 0, s>>>(slots, nslots);
+    return after_launch();
 }
 
 cudaError_t launch_score(const ScoreBatch &b, cudaStream_t s)
 {
     if (b.njobs <= 0) return cudaSuccess;
     LaunchTimer t("cambi_score", s);
-    score_kernel<<<1, kScoreMaxJobs, 0, s>>>(b);
+    score_kernel<<<b.njobs, 32 * kScales, 0, s>>>(b);
     return after_launch();
 }
 

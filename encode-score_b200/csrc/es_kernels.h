@@ -69,6 +69,29 @@ struct Band {
     int weight[kDiffs];
 };
 
+// ---- counters of the c-values -------------------------------------------------------------------------------------
+// Per picture-scale counters in device memory. The c-values are exact multiples of 2^-24 (they are at least 0.5), so
+// their sum is kept exactly as an integer in those units; the order of additions does not matter.
+// The c-value kernel also counts the positive values by the top 11 bits of their floats (the first radix digit of the
+// top-k selection): at least 0.5 and below 2^13, so those digits lie in kCvDigit0 .. kCvDigit0 + 55.
+constexpr unsigned kCvDigit0 = 0x3F000000u >> 21, kCvDigits = 64;
+struct CvSlot {
+    unsigned long long sum_fx, count;  // positive c-values: sum in 2^-24 units, number
+    unsigned long long list_n;         // values in `list`
+    unsigned long long n, k;           // pixels of the scale, top-k count
+    unsigned long long above_fx, above_n;
+    unsigned long long remaining1, remaining2;  // radix select state after each round
+    unsigned prefix1, prefix2;
+    float *list;                       // c-values, zeros among them (capacity n): every positive one is there once
+    unsigned pad_[2];
+    alignas(16) unsigned hist[2048];   // counts of the first radix digit
+    // counts of the second and the last digit, and the sums (2^-24 units) of the values of each last digit: clear between
+    // launches (the score kernel clears what a selection used)
+    alignas(16) unsigned hist1[2048];
+    alignas(16) unsigned hist2[1024];
+    alignas(16) unsigned long long dsum[1024];
+};
+
 // ---- scales 0 and 1: preprocessing, zero-derivative mask and mode filter of one plane, then its first decimation --
 struct Prep0Job {
     const uint16_t *img;  // input plane, `pitch` pixels per row
@@ -90,41 +113,29 @@ struct Prep0Batch {
     Band band;               // the codes that need c-values, for the need flags
     int need_lo, need_span;  // set by the launcher: the needed values are need_lo .. need_lo + need_span when they
                              // form one range (need_span >= 0), else need_span = -1 and the band's bits decide
+    // optional: clears the counters of slots [0, nslots) and sets each slot's n and k
+    CvSlot *slots;
+    int nslots;
+    const unsigned long long *slot_n, *slot_k;
 };
 cudaError_t launch_prep0(Prep0Batch &b, cudaStream_t s);
 
-// ---- scales 1..4: decimation and mode filter ------------------------------------------------------------------------
+// ---- scales 2..4: decimation and mode filter ------------------------------------------------------------------------
 struct DecJob {
-    const uint16_t *src;  // previous scale's words, sw x sh
-    int sw, sh;
-    uint16_t *dst;        // this scale's words, w x h
-    int w, h;
-    int first_block;      // set by the launcher: the job's first 64 x 16 output tile
+    const uint16_t *src;  // scale 1's words, rows of sw
+    int sw;
+    uint16_t *dst[3];     // the words of scales 2, 3 and 4
+    int w[3], h[3];       // their sizes
+    int first_block;      // set by the launcher
 };
 constexpr int kDecMaxJobs = kMaxPictures;
 struct DecBatch {
     DecJob job[kDecMaxJobs];
-    int njobs, total_blocks;  // total_blocks: set by the launcher
+    int njobs;
 };
 cudaError_t launch_decimate_mode(DecBatch &b, cudaStream_t s);
 
 // ---- c-values --------------------------------------------------------------------------------------------------------
-// Per picture-scale counters in device memory. The c-values are exact multiples of 2^-24 (they are at least 0.5), so
-// their sum is kept exactly as an integer in those units; the order of additions does not matter.
-// The c-value kernel also counts the positive values by the top 11 bits of their floats (the first radix digit of the
-// top-k selection): at least 0.5 and below 2^13, so those digits lie in kCvDigit0 .. kCvDigit0 + 55.
-constexpr unsigned kCvDigit0 = 0x3F000000u >> 21, kCvDigits = 64;
-struct CvSlot {
-    unsigned long long sum_fx, count;  // positive c-values: sum in 2^-24 units, number
-    unsigned long long list_n;         // values in `list`
-    unsigned long long n, k;           // pixels of the scale, top-k count
-    unsigned long long remaining, above_fx, above_n;
-    unsigned prefix, mask;             // radix select state
-    float *list;                       // c-values, zeros among them (capacity n): every positive one is there once
-    unsigned hist[2048];               // counts of the current radix digit
-    unsigned long long dsum[1024];     // last round: sums (2^-24 units) of the values of each last digit
-};
-
 struct CvJob {
     const uint16_t *word;
     int w, h, pad;
@@ -172,23 +183,22 @@ inline int cv_default_tile_rows(int w, int h, int tiles0)
 cudaError_t launch_cvalues(const CvBatch &b, cudaStream_t s);
 
 // ---- top-k pooling and score -------------------------------------------------------------------------------------
-// Clears the counters of slots [0, nslots) and sets each slot's n and k.
-cudaError_t launch_slots_reset(CvSlot *slots, int nslots, const unsigned long long *n, const unsigned long long *k,
-                               cudaStream_t s);
 // The exact k-th largest c-value, and the sum and count of the values above it, of every slot whose positive count
-// exceeds k, after the c-value launches (which leave the first digit's counts in each slot): three radix rounds of 11,
-// 11 and 10 bits over the slots' lists, the last one also summing what lies above the selected value.
+// exceeds k, after the c-value launches (which leave the first digit's counts in each slot): radix rounds of 11, 11 and
+// 10 bits, the second and third over the slots' lists, the last one also summing what lies above the selected value. The
+// score kernel makes the last pick.
 cudaError_t launch_topk(CvSlot *slots, int nslots, cudaStream_t s);
 struct ScoreJob {
     int first_slot;  // kScales consecutive slots
     int window;
-    double *score;   // out
+    double *score;   // out: the score, then the pooled value of each scale
+    double *host;    // the same in page-locked host memory, or null
 };
 constexpr int kScoreMaxJobs = kMaxPictures;
 struct ScoreBatch {
     ScoreJob job[kScoreMaxJobs];
     int njobs;
-    const CvSlot *slots;
+    CvSlot *slots;
 };
 cudaError_t launch_score(const ScoreBatch &b, cudaStream_t s);
 

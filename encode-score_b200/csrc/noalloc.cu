@@ -20,24 +20,26 @@ namespace es {
 namespace {
 
 constexpr size_t kScratchBytes = (size_t)20 << 20;
+// What the array holds before the planes: pictures are refused by what 20 MiB leave beside it. (The counters have an
+// array of their own.)
+constexpr size_t kScratchHead = 82432;
 constexpr int kNoAllocMaxPad = 32;                                                  // windows up to 65
 constexpr int kLutEntries = (2 * kNoAllocMaxPad + 1) * (2 * kNoAllocMaxPad + 1) + 1;  // 4226
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
+static __device__ CvSlot g_slots[kScales];
 
 constexpr size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 struct Carve {
-    size_t slots, score, lut, words[kScales], lists[kScales], end;
+    size_t score, lut, words[kScales], lists[kScales], end;
     int sw[kScales], sh[kScales];
 };
 
 Carve carve(int w, int h)
 {
     Carve c{};
-    size_t at = 0;
-    c.slots = at;
-    at = align256(at + kScales * sizeof(CvSlot));
+    size_t at = kScratchHead;
     c.score = at;
     at = align256(at + (1 + kScales) * sizeof(double));
     c.lut = at;
@@ -78,24 +80,27 @@ __global__ void noalloc_setup_kernel(CvSlot *slots, float *lut, const __grid_con
         return;
     }
     CvSlot &S = slots[blockIdx.x];
-    for (int i = threadIdx.x; i < 2048; i += blockDim.x) S.hist[i] = 0;
-    for (int i = threadIdx.x; i < 1024; i += blockDim.x) S.dsum[i] = 0;
+    for (int i = threadIdx.x; i < 2048; i += blockDim.x) S.hist[i] = S.hist1[i] = 0;
+    for (int i = threadIdx.x; i < 1024; i += blockDim.x) {
+        S.hist2[i] = 0;
+        S.dsum[i] = 0;
+    }
     if (threadIdx.x == 0) {
         S.sum_fx = S.count = S.list_n = 0;
         S.n = st.n[blockIdx.x];
         S.k = st.k[blockIdx.x];
-        S.remaining = S.k;
         S.above_fx = S.above_n = 0;
-        S.prefix = S.mask = 0;
         S.list = st.list[blockIdx.x];
     }
 }
 
-// The array's device address in the CUDA context current on the calling thread.
-unsigned char *scratch_in_current_context()
+// The arrays' device addresses in the CUDA context current on the calling thread.
+unsigned char *scratch_in_current_context(CvSlot *&slots)
 {
-    void *p = nullptr;
+    void *p = nullptr, *q = nullptr;
     cuda_check(cudaGetSymbolAddress(&p, g_scratch), "finding the no-allocation scratch array");
+    cuda_check(cudaGetSymbolAddress(&q, g_slots), "finding the no-allocation counters");
+    slots = (CvSlot *)q;
     return (unsigned char *)p;
 }
 
@@ -119,9 +124,9 @@ extern "C" int es_cambi_score_noalloc(uint64_t img, int pitch, int w, int h, int
         const es_cambi_params p = derive_params(w, h);
         require(p.pad <= kNoAllocMaxPad, "es_cambi_score_noalloc: window wider than 65");
         require(p.band_size > 0 && p.band_size <= kMaxBand, "es_cambi_score_noalloc: band out of range");
-        unsigned char *base = scratch_in_current_context();
+        CvSlot *slots;
+        unsigned char *base = scratch_in_current_context(slots);
         cudaStream_t s = (cudaStream_t)stream;
-        CvSlot *slots = (CvSlot *)(base + c.slots);
         double *rec = (double *)(base + c.score);
 
         SlotSetup st{};
@@ -147,14 +152,16 @@ extern "C" int es_cambi_score_noalloc(uint64_t img, int pitch, int w, int h, int
         pj.w1 = c.sw[1];
         pj.h1 = c.sh[1];
         cuda_check(launch_prep0(pb, s), "cambi scales 0 and 1");
+        DecBatch db{};
+        db.njobs = 1;
+        db.job[0].src = (const uint16_t *)(base + c.words[1]);
+        db.job[0].sw = c.sw[1];
         for (int k = 2; k < kScales; k++) {
-            DecBatch db{};
-            db.njobs = 1;
-            db.job[0] = DecJob{(const uint16_t *)(base + c.words[k - 1]), c.sw[k - 1], c.sh[k - 1], (uint16_t *)(base + c.words[k]),
-                               c.sw[k], c.sh[k], 0};
-            db.total_blocks = (c.sw[k] * c.sh[k] + 255) / 256;
-            cuda_check(launch_decimate_mode(db, s), "cambi scales");
+            db.job[0].dst[k - 2] = (uint16_t *)(base + c.words[k]);
+            db.job[0].w[k - 2] = c.sw[k];
+            db.job[0].h[k - 2] = c.sh[k];
         }
+        cuda_check(launch_decimate_mode(db, s), "cambi scales");
         CvBatch cb{};
         cb.njobs = kScales;
         int tiles = 0;
