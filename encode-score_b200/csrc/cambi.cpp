@@ -167,11 +167,6 @@ void set_lists(es_cambi *c)
 
 }  // namespace
 
-void cambi_join(es_cambi *c, cudaStream_t stream)
-{
-    cuda_check(cudaStreamWaitEvent(stream, c->finished.e, 0), "cambi event");
-}
-
 extern "C" {
 
 int es_cambi_create_with(const es_module *m, int w, int h, int depth, const es_cambi_params *params, es_cambi **out)

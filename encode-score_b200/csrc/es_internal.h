@@ -136,10 +136,6 @@ unsigned long long topk_count(unsigned long long n, double topk);
 
 }  // namespace es
 
-// Makes `stream` wait until the work of the instance's last launch is done (used by es_frame so that one event on
-// the caller's stream marks the end of a whole frame step).
-void cambi_join(es_cambi *c, cudaStream_t stream);
-
 namespace es {
 // The figures of one encode in a collected frame step, as the device left them in page-locked memory.
 struct EncodeFigures {

@@ -326,9 +326,8 @@ struct CollectBatch {
 };
 constexpr int kCollectSums = 20;  // 18 double sums and 2 counts per block
 int collect_blocks(int windows);
-cudaError_t launch_collect(CollectBatch &b, cudaStream_t s);
-// the same in two parts: the structure threshold and mask (needs the window figures only), then the windows' bins and
-// sums (needs the lasting figures too)
+// The structure threshold and mask (needs the window figures only), then the windows' bins and sums (needs the lasting
+// figures too).
 cudaError_t launch_collect_threshold(CollectBatch &b, cudaStream_t s);
 cudaError_t launch_collect_sums(CollectBatch &b, cudaStream_t s);
 

@@ -983,12 +983,6 @@ cudaError_t launch_collect_sums(CollectBatch &b, cudaStream_t s)
     return after_launch();
 }
 
-cudaError_t launch_collect(CollectBatch &b, cudaStream_t s)
-{
-    const cudaError_t e = launch_collect_threshold(b, s);
-    return e != cudaSuccess ? e : launch_collect_sums(b, s);
-}
-
 // ---------------------------------------------------------------------------------------------------------------
 // The VMAF picture feed: src/kernels.cu:537-545 (to_picture), one launch for every plane of a step. A thread moves 8
 // samples of a row: one 16-byte load of the 16-bit values, and one 8-byte (8-bit picture) or 16-byte store where the
