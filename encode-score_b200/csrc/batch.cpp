@@ -37,8 +37,7 @@ struct Source {
     DeviceBuffer<float> stats[2], persist[2];
     DeviceBuffer<uint8_t> masks;
     DeviceBuffer<unsigned long long> sums[2];
-    DeviceBuffer<FrameFigures> figs[2];
-    DeviceBuffer<uint16_t> bins[2];
+    DeviceBuffer<unsigned> bin_n;
     DeviceBuffer<float> threshold;
     DeviceBuffer<double> partials;
     PinnedBuffer<unsigned long long> h_sums[2];
@@ -165,13 +164,15 @@ void init_source(Source &S, const es_batch_source &d)
         S.stats[i].reset(std::max<size_t>(1, win * kStats * S.nenc));
         S.persist[i].reset(std::max<size_t>(1, win * kPersist * S.nenc));
         S.sums[i].reset((size_t)3 * S.nenc + 3 * (S.nenc + 1));
-        S.figs[i].reset(S.nenc);
-        S.bins[i].reset(win * kBinArrays * S.nenc + 4 * (size_t)S.nenc);  // the arrays, then 2 counts per encode
+        cuda_check(cudaMemset(S.sums[i].ptr, 0, S.sums[i].bytes()), "clearing");
         S.h_sums[i].reset(S.sums[i].count);
         S.h_figs[i].reset(S.nenc);
-        S.h_bins[i].reset(S.bins[i].count);
+        S.h_bins[i].reset(win * kBinArrays * S.nenc + 4 * (size_t)S.nenc);  // the arrays, then 2 counts per encode
+        std::memset(S.h_bins[i].ptr, 0, S.h_bins[i].count * sizeof(uint16_t));
         std::memset(S.h_figs[i].ptr, 0, sizeof(FrameFigures) * S.nenc);
     }
+    S.bin_n.reset(2 * (size_t)S.nenc);
+    cuda_check(cudaMemset(S.bin_n.ptr, 0, S.bin_n.bytes()), "clearing");
     S.threshold.reset(1);
     S.partials.reset(std::max<size_t>(1, (size_t)S.nenc * collect_blocks(S.windows) * kCollectSums));
     S.masks.reset(std::max<size_t>(1, win * kEncRing));
@@ -477,7 +478,6 @@ void record_texture(es_batch &b, long f, cudaStream_t s, cudaStream_t s2)
     for (auto &sp : b.sources) {
         Source &S = *sp;
         const int up = 10 - S.pd;
-        cuda_check(cudaMemsetAsync(S.sums[at].ptr, 0, S.sums[at].bytes(), s), "clearing");
         PairSumsJob &pj = pb.job[pb.njobs++];
         pj.ry = S.src_plane(f);
         pj.ru = S.src_u.ptr;
@@ -496,10 +496,8 @@ void record_texture(es_batch &b, long f, cudaStream_t s, cudaStream_t s2)
 
         WindowJob &wj = wb.job[wb.njobs++];
         wj.yr = S.src_plane(f);
-        for (int e = 0; e < S.nenc; e++) {
-            wj.yd[e] = S.enc_plane(e, f);
-            wj.stats[e] = S.stats[at].ptr + (size_t)e * S.windows * kStats;
-        }
+        for (int e = 0; e < S.nenc; e++) wj.yd[e] = S.enc_plane(e, f);
+        wj.stats = S.stats[at].ptr;
         wj.nenc = S.nenc;
         wj.w = S.w;
         wj.h = S.h;
@@ -514,38 +512,35 @@ void record_texture(es_batch &b, long f, cudaStream_t s, cudaStream_t s2)
         qj.y_m7 = f >= 7 ? S.src_plane(f - 7) : nullptr;
         qj.y_c = f >= 6 ? S.src_plane(f - 6) : nullptr;
         qj.y_f = S.src_plane(f);
-        for (int e = 0; e < S.nenc; e++) {
-            qj.yd[e] = f >= 6 ? S.enc_plane(e, f - 6) : nullptr;
-            qj.out[e] = S.persist[at].ptr + (size_t)e * S.windows * kPersist;
-        }
+        for (int e = 0; e < S.nenc; e++) qj.yd[e] = f >= 6 ? S.enc_plane(e, f - 6) : nullptr;
+        qj.out = S.persist[at].ptr;
         qj.nenc = S.nenc;
         qj.w = S.w;
         qj.h = S.h;
         qj.up = up;
         qj.stats = texture ? 1 : 0;
 
-        if (S.windows > 0) {
-            CollectJob &cj = cb.job[cb.njobs++];
-            for (int e = 0; e < S.nenc; e++) {
-                cj.stats[e] = wj.stats[e];
-                cj.persist[e] = texture ? qj.out[e] : nullptr;
-                cj.fig[e] = S.figs[at].ptr + e;
-                cj.bins[e] = S.bins[at].ptr + (size_t)e * kBinArrays * S.windows;
-                cj.bin_n[e] = bin_counts(S.bins[at].ptr, S.windows, S.nenc) + 2 * e;
-            }
-            cj.centre_mask = S.masks.ptr + (size_t)((f + kEncRing - kRadius) % kEncRing) * S.windows;
-            cj.mask = S.masks.ptr + (size_t)(f % kEncRing) * S.windows;
-            cj.nenc = S.nenc;
-            cj.windows = S.windows;
-            cj.threshold = S.threshold.ptr;
-            cj.partials = S.partials.ptr;
-        }
+        CollectJob &cj = cb.job[cb.njobs++];  // (a picture of 16 x 16 has one window)
+        cj.stats = wj.stats;
+        cj.persist = texture ? qj.out : nullptr;
+        cj.host_fig = S.h_figs[at].ptr;
+        cj.host_bins = S.h_bins[at].ptr;
+        cj.bin_n = S.bin_n.ptr;
+        cj.host_bin_n = bin_counts(S.h_bins[at].ptr, S.windows, S.nenc);
+        cj.sums = S.sums[at].ptr;
+        cj.host_sums = S.h_sums[at].ptr;
+        cj.centre_mask = S.masks.ptr + (size_t)((f + kEncRing - kRadius) % kEncRing) * S.windows;
+        cj.mask = S.masks.ptr + (size_t)(f % kEncRing) * S.windows;
+        cj.nenc = S.nenc;
+        cj.windows = S.windows;
+        cj.threshold = S.threshold.ptr;
+        cj.partials = S.partials.ptr;
     }
     cuda_check(launch_pair_sums(pb, s), "batch squared errors and colors");
     cuda_check(launch_window_stats(wb, s), "batch window figures");
     // the structure threshold needs only the window figures, so on a stream of its own it runs beside the lasting
     // texture (one block, otherwise alone at the end of the chain)
-    const bool fork = cb.njobs && s2 != nullptr;
+    const bool fork = s2 != nullptr;
     if (fork) {
         cuda_check(cudaEventRecord(b.fork_thr.e, s), "event");
         cuda_check(cudaStreamWaitEvent(s2, b.fork_thr.e, 0), "event");
@@ -553,22 +548,9 @@ void record_texture(es_batch &b, long f, cudaStream_t s, cudaStream_t s2)
         cuda_check(cudaEventRecord(b.join_thr.e, s2), "event");
     }
     cuda_check(launch_persist(qb, s), "batch lasting texture");
-    if (cb.njobs) {
-        if (fork) cuda_check(cudaStreamWaitEvent(s, b.join_thr.e, 0), "event");
-        else cuda_check(launch_collect_threshold(cb, s), "batch structure threshold");
-        for (auto &sp : b.sources)
-            if (sp->windows > 0)
-                cuda_check(cudaMemsetAsync(bin_counts(sp->bins[at].ptr, sp->windows, sp->nenc), 0, 8 * (size_t)sp->nenc, s), "clearing");
-        cuda_check(launch_collect_sums(cb, s), "batch collecting figures");
-    }
-    for (auto &sp : b.sources) {
-        Source &S = *sp;
-        cuda_check(cudaMemcpyAsync(S.h_sums[at].ptr, S.sums[at].ptr, S.sums[at].bytes(), cudaMemcpyDeviceToHost, s), "reading figures");
-        if (S.windows > 0) {
-            cuda_check(cudaMemcpyAsync(S.h_figs[at].ptr, S.figs[at].ptr, S.figs[at].bytes(), cudaMemcpyDeviceToHost, s), "reading figures");
-            cuda_check(cudaMemcpyAsync(S.h_bins[at].ptr, S.bins[at].ptr, S.bins[at].bytes(), cudaMemcpyDeviceToHost, s), "reading figures");
-        }
-    }
+    if (fork) cuda_check(cudaStreamWaitEvent(s, b.join_thr.e, 0), "event");
+    else cuda_check(launch_collect_threshold(cb, s), "batch structure threshold");
+    cuda_check(launch_collect_sums(cb, s), "batch collecting figures");
 }
 
 // The whole step f on b.main: unpacking, then the CAMBI chain on main beside the texture chain on side.

@@ -249,7 +249,7 @@ constexpr int kMaxEncodes = 16;
 struct WindowJob {
     const uint16_t *yr;                 // source luma (pipeline depth)
     const uint16_t *yd[kMaxEncodes];    // encode luma
-    float *stats[kMaxEncodes];          // per encode: windows x 8
+    float *stats;                       // [nenc][windows][8]
     int nenc, w, h, up;
     int first_block;                    // set by the launcher
 };
@@ -270,7 +270,7 @@ struct PersistJob {
     uint16_t *e_new, *o_new;
     const uint16_t *y_m13, *y_m7, *y_c, *y_f;  // frames f-13, f-7, f-6 (= centre), f; nullptr = zero
     const uint16_t *yd[kMaxEncodes];           // encodes' luma at the centre frame
-    float *out[kMaxEncodes];                   // per encode: windows x 5
+    float *out;                                // [nenc][windows][5]
     int nenc, w, h, up;
     int stats;  // 0: only advance the running sums
     int first_block;  // set by the launcher
@@ -305,18 +305,23 @@ struct FrameFigures {
     float threshold;
     unsigned pad_;
 };
+// The last kernel writes the step's figures to page-locked host memory and leaves the sums and counts it copied clear
+// for the step after the next.
 struct CollectJob {
-    const float *stats[kMaxEncodes];    // windows x 8
-    const float *persist[kMaxEncodes];  // windows x 5, centre frame (nullptr: no lasting texture this frame)
-    const uint8_t *centre_mask;         // structure mask of the centre frame
-    uint8_t *mask;                      // out: structure mask of this frame
-    FrameFigures *fig[kMaxEncodes];
-    uint16_t *bins[kMaxEncodes];        // out: 6 arrays of up to `windows` bins (amount 0-2, matching 0-1, lasting),
-                                        // only those that count, from the start of each array in no fixed order
-    unsigned *bin_n[kMaxEncodes];       // out (cleared by the caller): [0] bins in each of the first five arrays
-                                        // (the structure windows), [1] in the lasting array
-    float *threshold;                   // scratch: the frame's structure threshold
-    double *partials;                   // scratch: [nenc][collect_blocks(windows)][kCollectSums]
+    const float *stats;            // [nenc][windows][8]
+    const float *persist;          // [nenc][windows][5], centre frame (nullptr: no lasting texture this frame)
+    const uint8_t *centre_mask;    // structure mask of the centre frame
+    uint8_t *mask;                 // out: structure mask of this frame
+    FrameFigures *host_fig;        // out (host): [nenc]
+    uint16_t *host_bins;           // out (host): [nenc] of 6 arrays of up to `windows` bins (amount 0-2, matching 0-1,
+                                   // lasting), only those that count, from the start of each array in no fixed order
+    unsigned *bin_n;               // scratch: [nenc][2], bins in each of the first five arrays (the structure windows)
+                                   // and in the lasting array
+    unsigned *host_bin_n;          // out (host): the same
+    unsigned long long *sums;      // PairSumsJob's sse [nenc][3], then color [nenc + 1][3]
+    unsigned long long *host_sums; // out (host): the same
+    float *threshold;              // scratch: the frame's structure threshold
+    double *partials;              // scratch: [nenc][collect_blocks(windows)][kCollectSums]
     int nenc, windows;
     int first_enc;  // set by the launcher: this job's encodes are grid rows first_enc .. first_enc + nenc - 1
 };

@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(256, 3) window_stats_kernel(const __grid_const
         }
         const long long cf = half_warp_sum((long long)fine_x), cm = half_warp_sum(mid_x);
         if (inside && (lane & 15) == 0) {
-            float *o = J.stats[p - 1] + ((size_t)wy * ww + wx) * 8;
+            float *o = J.stats + (((size_t)(p - 1) * wh + wy) * ww + wx) * 8;
             o[0] = exact_ratio((long long)src_f, 81.0);
             o[1] = exact_ratio((long long)src_m, 6561.0);
             o[2] = exact_ratio((long long)sf, 81.0);
@@ -547,7 +547,7 @@ __global__ void __launch_bounds__(256, 3) persist_kernel(const __grid_constant__
             continue;
         }
         if (inside && (lane & 15) == 0) {
-            float *o = J.out[p - 1] + ((size_t)wy * ww + wx) * 5;
+            float *o = J.out + (((size_t)(p - 1) * wh + wy) * ww + wx) * 5;
             o[0] = exact_ratio(own, 78732.0);
             o[1] = exact_ratio(sp, 78732.0);
             o[2] = exact_ratio(sab, 236196.0);
@@ -739,7 +739,7 @@ __global__ void __launch_bounds__(kCT) collect_threshold_kernel(const __grid_con
     __shared__ unsigned hist[2048];
     extern __shared__ float stage[];
     const CollectJob &J = B.job[blockIdx.x];
-    const float *st = J.stats[0];  // the source's oriented figures are the same in every encode's array
+    const float *st = J.stats;  // the source's oriented figures are the same in every encode's array
     const int n = J.windows;
     const float *v = st + 6;
     int stride = 8;
@@ -786,7 +786,7 @@ __global__ void __launch_bounds__(kCW) collect_windows_kernel(const __grid_const
     bool structure = false, lasting = false;
     if (i < n) {
         const float q = *J.threshold;
-        const float *s = J.stats[e] + (size_t)i * 8;
+        const float *s = J.stats + ((size_t)e * n + i) * 8;
         const bool m = s[6] >= q && s[6] > 0.0f;
         structure = m;
         const double er[3] = {(double)s[0], (double)s[1], (double)s[6]}, ed[3] = {(double)s[2], (double)s[3], (double)s[7]};
@@ -810,8 +810,8 @@ __global__ void __launch_bounds__(kCW) collect_windows_kernel(const __grid_const
             }
         }
         v[18] = m ? 1.0 : 0.0;
-        if (J.persist[e]) {
-            const float *ps = J.persist[e] + (size_t)i * 5;
+        if (J.persist) {
+            const float *ps = J.persist + ((size_t)e * n + i) * 5;
             const double agree = __ddiv_rn((double)ps[2], __dsqrt_rn(fmax(__dmul_rn((double)ps[3], (double)ps[4]), 1e-9)));
             if (J.centre_mask[i] && agree > 0.5 && ps[0] > 0.0f) {
                 v[16] = (double)ps[0];
@@ -822,15 +822,16 @@ __global__ void __launch_bounds__(kCW) collect_windows_kernel(const __grid_const
             }
         }
     }
-    // the bins that count, compacted (a histogram does not depend on their order): the five structure arrays share
-    // one position per window, the lasting array has its own; a warp reserves its places with one atomic each
+    // the bins that count, compacted (a histogram does not depend on their order), straight to the host's memory: the
+    // five structure arrays share one position per window, the lasting array has its own; a warp reserves its places with
+    // one atomic each
     {
-        uint16_t *bins = J.bins[e];
+        uint16_t *bins = J.host_bins + (size_t)e * 6 * n;
         const unsigned below = (1u << lane) - 1u;
         const unsigned sm = __ballot_sync(0xffffffffu, structure), lm = __ballot_sync(0xffffffffu, lasting);
         unsigned sb = 0, lb = 0;
-        if (sm && lane == 0) sb = atomicAdd(&J.bin_n[e][0], (unsigned)__popc(sm));
-        if (lm && lane == 0) lb = atomicAdd(&J.bin_n[e][1], (unsigned)__popc(lm));
+        if (sm && lane == 0) sb = atomicAdd(&J.bin_n[2 * e], (unsigned)__popc(sm));
+        if (lm && lane == 0) lb = atomicAdd(&J.bin_n[2 * e + 1], (unsigned)__popc(lm));
         sb = __shfl_sync(0xffffffffu, sb, 0);
         lb = __shfl_sync(0xffffffffu, lb, 0);
         if (structure) {
@@ -854,19 +855,33 @@ __global__ void __launch_bounds__(kCW) collect_windows_kernel(const __grid_const
 }
 
 // Warp k of an encode's block makes sum k: lane l adds the partials of blocks l, l + 32, ... in order, then a fixed
-// shuffle tree adds the 32 lane sums (the same order on every run).
+// shuffle tree adds the 32 lane sums (the same order on every run). The figures, the encode's squared errors and colors
+// (the first block: also the source's colors) and its bin counts go to the host's memory; the copied sums and counts are
+// cleared. (As three copies and two memory clears per source they cost the step 15 us of waiting on one another.)
 __global__ void __launch_bounds__(32 * kCollectSums) collect_final_kernel(const __grid_constant__ CollectBatch B)
 {
     int jb = 0;
     while (jb + 1 < B.njobs && (int)blockIdx.x >= B.job[jb + 1].first_enc) jb++;
     const CollectJob &J = B.job[jb];
     const int e = blockIdx.x - J.first_enc, k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto move = [&](unsigned long long *from, unsigned long long *to) {
+        *to = *from;
+        *from = 0;
+    };
+    const int t = threadIdx.x, c0 = 3 * J.nenc;  // the sums: squared errors, then the encodes' colors, then the source's
+    if (t < 3) move(J.sums + 3 * e + t, J.host_sums + 3 * e + t);
+    else if (t < 6) move(J.sums + c0 + 3 * e + t - 3, J.host_sums + c0 + 3 * e + t - 3);
+    else if (t < 9 && e == 0) move(J.sums + 2 * c0 + t - 6, J.host_sums + 2 * c0 + t - 6);
+    else if (t >= 32 && t < 34) {
+        J.host_bin_n[2 * e + t - 32] = J.bin_n[2 * e + t - 32];
+        J.bin_n[2 * e + t - 32] = 0;
+    }
     const int nblocks = collect_blocks_dev(J.windows);
     double s = 0.0;
     for (int b = lane; b < nblocks; b += 32) s += J.partials[((size_t)e * nblocks + b) * kCollectSums + k];
     s = warp_sum(s);
     if (lane != 0) return;
-    FrameFigures *f = J.fig[e];
+    FrameFigures *f = J.host_fig + e;
     if (k < 3) f->all_r[k] = s;
     else if (k < 6) f->all_d[k - 3] = s;
     else if (k < 9) f->st_r[k - 6] = s;
