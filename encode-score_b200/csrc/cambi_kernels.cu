@@ -33,27 +33,28 @@ __device__ __forceinline__ uint16_t mode3(uint16_t a, uint16_t b, uint16_t c)
 // Scales 0 and 1: src/kernels.cu:524-535 (from8), 14-40 (mask), 488-500 (mode), 43-53 (decimation), in one pass over a
 // 64 x 64 tile of scale 0 and the 32 x 32 tile of scale 1 beneath it.
 //
-// The plane is staged with its margins (16-byte loads for tiles inside the picture; an 8-bit plane becomes 10-bit
-// anti-dithered values in a second buffer). A warp per staged row packs the flat pixels into bit words by ballot. Each
-// warp then walks 8 rows of the tile, a lane taking two neighbouring columns as the two halves of 32-bit words: the 7
-// flat bits around each column come from one funnel shift and two popcounts and are summed over 7 rows as they go (both
-// counts in one register), and the 3 x 3 mode filter reads both columns' neighbours with 32-bit loads. The scale-0 words at even
-// positions, with a ring of them one step outside the tile (made on their own), then give the tile's scale-1 words
-// (decimation and mode filter of the decimated values) without another read of scale 0.
+//  1. The plane is staged with its margins, 8 pixels per load, coordinates clamped to the picture. An 8-bit plane becomes
+//     10-bit anti-dithered values in place: ((4 a + 4 b + 4 c + 4 d) >> 2) of a pixel and its right, lower and lower
+//     right neighbours is a + b + c + d, and on the last row and column the clamped copies give the reference's pairs.
+//  2. Flat pixels (equal to the right and lower neighbours; a clamped copy is equal) become bits, 8 per thread and step.
+//  3. The 7 x 7 counts of flat pixels are made 32 columns at a time in bit-sliced form: the counts of 7 columns as three
+//     bit planes (four full adders of three-input logic), then 7 rows of those as six planes, compared with mask_index.
+//  4. Each warp walks 8 rows of the tile, a lane taking two neighbouring columns as the two halves of 32-bit words: the
+//     3 x 3 mode filter reads both columns' neighbours with 32-bit loads.
+//  5. The scale-0 words at even positions, with a ring of them one step outside the tile (made on their own), give the
+//     tile's scale-1 words (decimation and mode filter of the decimated values) without another read of scale 0.
+// Bound by integer issue (11 thousand warp instructions a tile, the ALU pipe 71 % busy). With counts by population count
+// per pixel pair, flat bits by ballot and a longer mode filter it took 54 us for a 3840 x 2160 10-bit picture and 31 us
+// for a 1920 x 1080 8-bit one; now 40 and 22 us.
 // Staged region: columns x0-8 .. x0+71 (index x - (x0-8)), rows y0-5 .. y0+69 (index y - (y0-5)).
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int kP0T = 64;                 // scale-0 tile side
 constexpr int kP0C = 80, kP0R = 75;      // staged columns and rows
 constexpr int kP0X = 8, kP0Y = 5;        // staged index of x0, y0
-constexpr int kP0FR = 73, kP0FX = 5;     // flat rows y0-5 .. y0+67; bit i of a row is column x0-5+i
+constexpr int kP0FR = 74;                // rows of flat bits (staged rows 0 .. 73); bit i of a row is staged column i
+constexpr int kP0M = 66;                 // rows of mask bits: y0 - 2, y0 .. y0 + 63, y0 + 64
 constexpr int kP0D = 34;                 // scale-0 words (x0-2+2X, y0-2+2Y), X, Y in 0 .. 33
 
-// The mode of three values per 16-bit half (the smallest when all three differ), from SIMD minima and maxima only:
-// with two or three equal values the repeated one is the median, and it equals the largest unless the pair is the
-// two smallest, when it equals the smallest; with three different values the mode is the smallest. So the mode is
-// the median where the median equals the largest, else the smallest. The halves' differences are never negative, so
-// 32-bit subtraction keeps them apart, and "median below the largest" is a per-half nonzero test. (16-bit SIMD
-// compares, and two scalar modes, measured slower.)
 __device__ __forceinline__ uint32_t vmin_u16x2(uint32_t a, uint32_t b)
 {
     uint32_t r;
@@ -66,14 +67,59 @@ __device__ __forceinline__ uint32_t vmax_u16x2(uint32_t a, uint32_t b)
     asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
+// Bit 15 of each half, over the half.
+__device__ __forceinline__ uint32_t sign_x2(uint32_t a)
+{
+    uint32_t r;
+    asm("prmt.b32 %0, %1, 0, 0xBB99;" : "=r"(r) : "r"(a));
+    return r;
+}
+// The mode of three values below 2^15 per 16-bit half (the smallest when all three differ): with two or three equal
+// values the repeated one is the median, and it equals the largest unless the pair is the two smallest, when it equals
+// the smallest; with three different values the mode is the smallest. So the mode is the largest where the median equals
+// it, else the smallest. The halves' differences are never negative, so 32-bit subtraction keeps them apart.
 __device__ __forceinline__ uint32_t mode3x2(uint32_t a, uint32_t b, uint32_t c)
 {
     const uint32_t lo = vmin_u16x2(a, b), hi = vmax_u16x2(a, b);
     const uint32_t mn = vmin_u16x2(lo, c), mx = vmax_u16x2(hi, c), md = vmax_u16x2(lo, vmin_u16x2(hi, c));
-    const uint32_t d = mx - md;  // per half, never negative: no borrow between the halves
-    const uint32_t t = (((d & 0x7FFF7FFFu) + 0x7FFF7FFFu) | d) & 0x80008000u;  // bit 15 of a half: median below max
-    const uint32_t nz = t | (t - (t >> 15));
-    return mn + ((md - mn) & ~nz);
+    const uint32_t differ = sign_x2(mx - md + 0x7FFF7FFFu);
+    return (mx & ~differ) | (mn & differ);
+}
+
+// One full adder on 32 columns: a + b + c = sum + 2 carry.
+struct Planes3 {
+    uint32_t p0, p1, p2;
+};
+__device__ __forceinline__ void full_add(uint32_t a, uint32_t b, uint32_t c, uint32_t &sum, uint32_t &carry)
+{
+    sum = a ^ b ^ c;
+    carry = (a & b) | (a & c) | (b & c);
+}
+// The number of set bits among seven words, per column.
+__device__ __forceinline__ Planes3 count7(const uint32_t (&v)[7])
+{
+    uint32_t s0, s1, c0, c1, c2;
+    Planes3 r;
+    full_add(v[0], v[1], v[2], s0, c0);
+    full_add(v[3], v[4], v[5], s1, c1);
+    full_add(s0, s1, v[6], r.p0, c2);
+    full_add(c0, c1, c2, r.p1, r.p2);
+    return r;
+}
+
+// 8 pixels of row y (inside the picture) from column x, clamped to 0 .. w - 1.
+__device__ __forceinline__ uint4 plane8(const uint16_t *img, int pitch, int w, int y, int x, int align)
+{
+    const uint16_t *row = img + (size_t)y * pitch;
+    if (x >= 0 && x + 8 <= w && align < 2) {
+        if (align == 0) return __ldg((const uint4 *)(row + x));
+        const uint32_t *q = (const uint32_t *)(row + x);
+        return make_uint4(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3));
+    }
+    uint32_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = __ldg(row + min(max(x + k, 0), w - 1));
+    return make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
 }
 
 __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ Prep0Batch b)
@@ -90,9 +136,11 @@ __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ P
         }
         return;
     }
-    __shared__ __align__(16) uint16_t buf[2][kP0R][kP0C];  // [0]: the staged plane; [1]: 8-bit planes at 10 bits
-    __shared__ uint32_t flatbits[kP0FR][4];                // 3 words of bits and a zero word
-    __shared__ uint16_t dw[kP0D][kP0D];                    // scale-0 words at even positions, for scale 1
+    __shared__ __align__(16) uint16_t buf[kP0R][kP0C];     // the staged plane at 10 bits
+    __shared__ __align__(16) uint32_t flatbits[kP0FR][4];  // 80 bits a row, then zeros
+    __shared__ uint32_t seven[kP0FR][9];                   // flat pixels among 7 columns: 3 planes of 3 words
+    __shared__ uint32_t maskbits[kP0M][3];
+    __shared__ __align__(4) uint16_t dw[kP0D][kP0D + 2];   // scale-0 words at even positions, for scale 1: word X at X + 1
     __shared__ uint32_t needbits[32];
     const int j = find_job(b.njobs, (int)blockIdx.x, [&](int k) { return b.job[k].first_tile; });
     const Prep0Job &J = b.job[j];
@@ -109,74 +157,114 @@ __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ P
             if (lane == 0) needbits[warp + 8 * k] = m;
         }
     }
-    if (tid < kP0FR) flatbits[tid][3] = 0;
-    const bool inside = xs >= 0 && xs + kP0C <= w && ys >= 0 && ys + kP0R <= h && (J.pitch & 7) == 0 && (((uintptr_t)J.img) & 15) == 0;
-    if (inside) {
-        for (int i = tid; i < kP0R * (kP0C / 8); i += 256) {
-            const int r = i / (kP0C / 8), q = i - r * (kP0C / 8);
-            *(uint4 *)&buf[0][r][8 * q] = __ldg((const uint4 *)(J.img + (size_t)(ys + r) * J.pitch + xs) + q);
-        }
-    } else {
-        for (int i = tid; i < kP0R * kP0C; i += 256) {
-            const int r = i / kP0C, c = i - r * kP0C, x = xs + c, y = ys + r;
-            buf[0][r][c] = (x >= 0 && x < w && y >= 0 && y < h) ? J.img[(size_t)y * J.pitch + x] : (uint16_t)0;
-        }
+    const int align = (J.pitch & 7) == 0 && (((uintptr_t)J.img) & 15) == 0 ? 0 : (J.pitch & 1) == 0 && (((uintptr_t)J.img) & 3) == 0 ? 1 : 2;
+    constexpr int kQ = kP0C / 8;  // 8-pixel groups of a staged row
+    for (int i = tid; i < kP0R * kQ; i += 256) {
+        const int r = i / kQ, q = i - r * kQ;
+        *(uint4 *)&buf[r][8 * q] = plane8(J.img, J.pitch, w, min(max(ys + r, 0), h - 1), xs + 8 * q, align);
     }
+    if (tid < kP0FR) ((uint4 *)flatbits)[tid] = make_uint4(0, 0, 0, 0);
     __syncthreads();
-    // preprocessed values of x0-5 .. x0+68, y0-5 .. y0+68: an 8-bit plane at 10 bits, the mean of the 2 x 2 block to
-    // the lower right (pairs on the last row and column); a 10-bit plane as staged (0 outside the picture)
-    const int sel = J.depth == 8 ? 1 : 0;
-    if (sel) {
-        for (int i = tid; i < 74 * 74; i += 256) {
-            const int r = i / 74, c = 3 + (i - r * 74), x = xs + c, y = ys + r;
-            unsigned v = 0;
-            if (x >= 0 && x < w && y >= 0 && y < h) {
-                const unsigned a = (unsigned)buf[0][r][c] << 2;
-                if (x < w - 1 && y < h - 1)
-                    v = (a + ((unsigned)buf[0][r][c + 1] << 2) + ((unsigned)buf[0][r + 1][c] << 2) + ((unsigned)buf[0][r + 1][c + 1] << 2)) >> 2;
-                else if (y < h - 1) v = (a + ((unsigned)buf[0][r + 1][c] << 2)) >> 1;
-                else if (x < w - 1) v = (a + ((unsigned)buf[0][r][c + 1] << 2)) >> 1;
-                else v = a;
+    // the pixels right of a group of 8, as a group
+    auto right = [](uint4 v, uint32_t next) {
+        return make_uint4(__byte_perm(v.x, v.y, 0x5432), __byte_perm(v.y, v.z, 0x5432), __byte_perm(v.z, v.w, 0x5432),
+                          __byte_perm(v.w, next, 0x5432));
+    };
+    if (J.depth == 8) {
+        uint4 sum[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {  // rows 0 .. 73; the last staged row is only read
+            const int i = tid + 256 * k, r = i / kQ, q = i - r * kQ;
+            sum[k] = make_uint4(0, 0, 0, 0);
+            if (i < kP0FR * kQ) {
+                const uint4 a = *(const uint4 *)&buf[r][8 * q], c = *(const uint4 *)&buf[r + 1][8 * q];
+                // (the staged region's last column has no right neighbour and is not used)
+                const uint4 ar = right(a, q < kQ - 1 ? buf[r][8 * q + 8] : 0u), cr = right(c, q < kQ - 1 ? buf[r + 1][8 * q + 8] : 0u);
+                sum[k] = make_uint4(a.x + ar.x + c.x + cr.x, a.y + ar.y + c.y + cr.y, a.z + ar.z + c.z + cr.z, a.w + ar.w + c.w + cr.w);
             }
-            buf[1][r][c] = (uint16_t)v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const int i = tid + 256 * k, r = i / kQ, q = i - r * kQ;
+            if (i < kP0FR * kQ) *(uint4 *)&buf[r][8 * q] = sum[k];
         }
         __syncthreads();
     }
-    // flat: equal to the right and lower neighbours (the last column / row count as equal); nothing outside. A warp
-    // takes whole flat rows, 3 ballots of 32 columns each (73 columns used).
-    {
-        const bool interior = x0 >= 5 && x0 + kP0T + 4 < w && y0 >= 5 && y0 + kP0T + 4 < h;
-        for (int q = warp; q < kP0FR; q += 8) {
-            const uint16_t *row = buf[sel][q], *nxt = buf[sel][q + 1];
-            const int y = ys + q;
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                const int i = 32 * k + lane, c = i + (kP0X - kP0FX), x = x0 - kP0FX + i;
-                bool f = false;
-                if (k < 2 || i < kP0FR) {
-                    const uint16_t v = row[c];
-                    if (interior) f = v == row[c + 1] && v == nxt[c];
-                    else if (x >= 0 && x < w && y >= 0 && y < h)
-                        f = (x == w - 1 || v == row[c + 1]) && (y == h - 1 || v == nxt[c]);
-                }
-                const uint32_t word = __ballot_sync(0xffffffffu, f);
-                if (lane == k) flatbits[q][k] = word;
-            }
+    // flat bits: rows of the picture 0 .. h - 1 and columns 0 .. w - 1 only. (The values of an 8-bit plane's last staged
+    // row are not made; its flat row, 73, is not used.)
+    for (int i = tid; i < kP0FR * kQ; i += 256) {
+        const int r = i / kQ, q = i - r * kQ, x = xs + 8 * q, y = ys + r;
+        if (y < 0 || y >= h || x < 0 || x >= w) continue;  // groups start at multiples of 8
+        const uint4 a = *(const uint4 *)&buf[r][8 * q], ar = right(a, q < kQ - 1 ? buf[r][8 * q + 8] : 0u);
+        uint4 c = *(const uint4 *)&buf[r + 1][8 * q];
+        if (y == h - 1) c = a;  // (an 8-bit plane's values past the last row are sums of other copies)
+        // per half: 0 when flat; values are below 2^15, so adding 0x7FFF sets bit 15 for every other one
+        const uint32_t v[4] = {((a.x ^ ar.x) | (a.x ^ c.x)) + 0x7FFF7FFFu, ((a.y ^ ar.y) | (a.y ^ c.y)) + 0x7FFF7FFFu,
+                               ((a.z ^ ar.z) | (a.z ^ c.z)) + 0x7FFF7FFFu, ((a.w ^ ar.w) | (a.w ^ c.w)) + 0x7FFF7FFFu};
+        const uint32_t lo = ~__byte_perm(v[0], v[1], 0x7531) & 0x80808080u, hi = ~__byte_perm(v[2], v[3], 0x7531) & 0x80808080u;
+        uint32_t bits = (((lo >> 7) * 0x10204080u) >> 28) | ((((hi >> 7) * 0x10204080u) >> 28) << 4);  // byte k's bit to bit k
+        if (x + 8 >= w) {  // the last columns: column w - 1 has no right neighbour, nothing is flat past it
+            const int n = w - x;  // 1 .. 8
+            const uint32_t last = (n & 1) ? 0x0000FFFFu : 0xFFFF0000u, e = n <= 2 ? a.x ^ c.x : n <= 4 ? a.y ^ c.y : n <= 6 ? a.z ^ c.z : a.w ^ c.w;
+            bits = (bits & ((1u << (n - 1)) - 1u)) | ((e & last) == 0 ? 1u << (n - 1) : 0u);
         }
+        ((uint8_t *)flatbits[r])[q] = (uint8_t)bits;
+    }
+    __syncthreads();
+    // flat pixels among the 7 columns around each column
+    if (tid < kP0FR * 3) {
+        const int r = tid / 3, k = tid - 3 * r;
+        const uint32_t c = flatbits[r][k], l = k ? flatbits[r][k - 1] : 0u, n = flatbits[r][k + 1];
+        const uint32_t v[7] = {__funnelshift_l(l, c, 3), __funnelshift_l(l, c, 2), __funnelshift_l(l, c, 1), c,
+                               __funnelshift_r(c, n, 1), __funnelshift_r(c, n, 2), __funnelshift_r(c, n, 3)};
+        const Planes3 p = count7(v);
+        seven[r][k] = p.p0;
+        seven[r][3 + k] = p.p1;
+        seven[r][6 + k] = p.p2;
+    }
+    __syncthreads();
+    // the mask: more than mask_index of the 49
+    if (tid < kP0M * 3) {
+        const int m = tid / 3, k = tid - 3 * m, r0 = (m == 0 ? 0 : m == kP0M - 1 ? 66 : m + 1);  // flat rows y - 3 .. y + 3
+        Planes3 p[3];
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            uint32_t v[7];
+#pragma unroll
+            for (int i = 0; i < 7; i++) v[i] = seven[r0 + i][3 * q + k];
+            p[q] = count7(v);
+        }
+        // p[0] + 2 p[1] + 4 p[2], bit by bit
+        uint32_t bit[6], c1, c2, c3, c4, c5, s;
+        bit[0] = p[0].p0;
+        bit[1] = p[0].p1 ^ p[1].p0;
+        c1 = p[0].p1 & p[1].p0;
+        full_add(p[0].p2, p[1].p1, p[2].p0, s, c2);
+        bit[2] = s ^ c1;
+        c3 = s & c1;
+        full_add(p[1].p2, p[2].p1, c2, s, c4);
+        bit[3] = s ^ c3;
+        c5 = s & c3;
+        full_add(p[2].p2, c4, c5, bit[4], bit[5]);
+        uint32_t more = J.mask_index < 0 ? 0xFFFFFFFFu : 0u, equal = J.mask_index < 0 || J.mask_index > 63 ? 0u : 0xFFFFFFFFu;
+#pragma unroll
+        for (int q = 5; q >= 0; q--) {
+            const uint32_t limit = (J.mask_index >> q) & 1 ? 0xFFFFFFFFu : 0u;
+            more |= equal & bit[q] & ~limit;
+            equal &= ~(bit[q] ^ limit);
+        }
+        maskbits[m][k] = more;
     }
     __syncthreads();
 
     // the walk: warp g makes rows y0 + 8 g .. + 7, lane l columns x0 + 2 l and + 1
     const int x = x0 + 2 * lane, g = warp;
-    const int kw = (2 * lane + 2) >> 5, sh = (2 * lane + 2) & 31;  // flat bit of column x - 3
-    auto h7 = [&](int q) -> uint32_t {  // flat counts of the 7 columns around x and x + 1 in flat row q, as halves
-        const uint32_t bits = __funnelshift_r(flatbits[q][kw], flatbits[q][kw + 1], sh);
-        return (uint32_t)__popc(bits & 0x7Fu) | ((uint32_t)__popc((bits >> 1) & 0x7Fu) << 16);
-    };
+    const int mw = (kP0X + 2 * lane) >> 5, ms = (kP0X + 2 * lane) & 31;  // the mask bit of column x
     // columns x and x + 1 at a picture edge keep their own value in the horizontal mode
     const uint32_t edge = ((x == 0 || x == w - 1) ? 0x0000FFFFu : 0u) | ((x + 1 == w - 1) ? 0xFFFF0000u : 0u);
     const int c = x - xs;  // staged column of x (even)
-    auto pair = [&](int r, int cc) -> uint32_t { return *(const uint32_t *)&buf[sel][r][cc]; };
+    auto pair = [&](int r, int cc) -> uint32_t { return *(const uint32_t *)&buf[r][cc]; };
     auto hmode = [&](int y) -> uint32_t {  // horizontal modes of x and x + 1 in picture row y
         const int r = y - ys;
         const uint32_t l2 = pair(r, c - 2), m2 = pair(r, c), r2 = pair(r, c + 2);
@@ -184,19 +272,9 @@ __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ P
         return (m2 & edge) | (mode3x2(left, m2, right) & ~edge);
     };
     const bool feat = J.feat != nullptr;  // the same for the whole block
-    // mask bit 15 of each half where the count exceeds mask_index: counts <= 49 and 0x7FFF - mask_index added per
-    // half reach bit 15 exactly then, without a carry into the other half
-    const uint32_t idx2 = (0x7FFFu - (uint32_t)J.mask_index) * 0x10001u;
     const bool vec_store = (w & 1) == 0 && (((uintptr_t)J.word) & 3) == 0;
     const bool need_range = b.need_span >= 0;
     const int yb = y0 + 8 * g;
-    uint32_t hv[14];  // h7 of flat rows yb-3 .. yb+10 (flat row index y - (y0-5))
-    uint32_t cnt = 0;
-#pragma unroll
-    for (int q = 0; q < 6; q++) {
-        hv[q] = h7(yb - 3 - ys + q);
-        cnt += hv[q];
-    }
     uint32_t m0 = hmode(yb - 1), m1 = hmode(yb);
     // features of this lane's two columns over the current 4 rows, as 16-bit pairs (a pair holds 2 rows of sums of
     // values below 2^15, then it is folded into fsum; counts up to 4)
@@ -209,12 +287,11 @@ __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ P
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int y = yb + i;
-        hv[i + 6] = h7(y + 3 - ys);
-        cnt += hv[i + 6];
         const uint32_t m2 = hmode(y + 1);
         uint32_t v2 = mode3x2(m0, m1, m2);
         if (y == 0 || y == h - 1) v2 = pair(y - ys, c);  // (the same for the whole warp)
-        const uint32_t mk = (cnt + idx2) & 0x80008000u;
+        const uint32_t mb = maskbits[8 * g + i + 1][mw] >> ms;
+        const uint32_t mk = ((mb << 15) & 0x8000u) | ((mb << 30) & 0x80000000u);
         const uint32_t word2 = v2 | mk;
         if (y < h) {
             if (vec_store && x + 1 < w) {
@@ -223,7 +300,7 @@ __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ P
                 if (x < w) J.word[(size_t)y * w + x] = (uint16_t)word2;
                 if (x + 1 < w) J.word[(size_t)y * w + x + 1] = (uint16_t)(word2 >> 16);
             }
-            if ((i & 1) == 0 && x < w) dw[4 * g + i / 2 + 1][lane + 1] = (uint16_t)word2;
+            if ((i & 1) == 0 && x < w) dw[4 * g + i / 2 + 1][lane + 2] = (uint16_t)word2;
             if (feat) {
                 const uint32_t ok = (x + 1 < w) ? 0xFFFFFFFFu : (x < w ? 0x0000FFFFu : 0u);
                 const uint32_t mm = (mk >> 15) & ok & 0x10001u;
@@ -249,7 +326,6 @@ __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ P
                 need |= hit != 0;
             }
         }
-        cnt -= hv[i];
         m0 = m1;
         m1 = m2;
         if (feat && (i & 3) == 3) {
@@ -290,44 +366,47 @@ __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ P
         }
         const int px = x0 - 2 + 2 * X, py = y0 - 2 + 2 * Y;
         if (px >= 0 && px < w && py >= 0 && py < h) {
-            const int bi = px - (x0 - kP0FX) - 3, bw = bi >> 5, bs = bi & 31;
-            int n = 0;
-#pragma unroll
-            for (int dy = -3; dy <= 3; dy++)
-                n += __popc(__funnelshift_r(flatbits[py + dy - ys][bw], flatbits[py + dy - ys][bw + 1], bs) & 0x7Fu);
-            const int pc = px - xs;
+            const int pc = px - xs, m = Y == 0 ? 0 : Y == kP0D - 1 ? kP0M - 1 : 2 * Y - 1;  // mask row of y0 - 2 + 2 Y
+            const bool masked = (maskbits[m][pc >> 5] >> (pc & 31)) & 1u;
             auto hm1 = [&](int yy) -> uint16_t {
-                const uint16_t *row = buf[sel][yy - ys];
+                const uint16_t *row = buf[yy - ys];
                 return (px == 0 || px == w - 1) ? row[pc] : (uint16_t)(mode3x2(row[pc - 1], row[pc], row[pc + 1]) & 0xFFFFu);
             };
-            const uint16_t v = (py == 0 || py == h - 1) ? buf[sel][py - ys][pc]
+            const uint16_t v = (py == 0 || py == h - 1) ? buf[py - ys][pc]
                                                         : (uint16_t)(mode3x2(hm1(py - 1), hm1(py), hm1(py + 1)) & 0xFFFFu);
-            dw[Y][X] = (uint16_t)(v | (n > J.mask_index ? kMaskBit : 0));
+            dw[Y][X + 1] = (uint16_t)(v | (masked ? kMaskBit : 0));
         }
     }
     __syncthreads();
     // scale 1: the decimated words dw, mode-filtered (rows and columns at the picture's edges keep their value); thread
-    // (cx, q) makes column cx of rows 4 q .. 4 q + 3 of the 32 x 32 tile
+    // (p, q) makes columns 2 p and 2 p + 1 of rows 2 q and 2 q + 1 of the 32 x 32 tile
     {
-        const int w1 = J.w1, h1 = J.h1, X0 = x0 >> 1, Y0 = y0 >> 1;
-        const int cx = tid & 31, q = tid >> 5, X1 = X0 + cx;
+        const int w1 = J.w1, h1 = J.h1, p = tid & 15, q = tid >> 4, X1 = (x0 >> 1) + 2 * p, Y0 = (y0 >> 1) + 2 * q;
         if (X1 < w1) {
-            const int X = cx + 1;
-            const bool edge1 = X1 == 0 || X1 == w1 - 1;
-            auto val = [&](int Y, int XX) -> uint32_t { return dw[Y][XX] & 0x7FFFu; };
-            uint32_t hm[6];  // rows Y0 + 4 q - 1 .. + 4 (dw rows 4 q .. 4 q + 5)
+            const uint32_t edge1 = ((X1 == 0 || X1 == w1 - 1) ? 0x0000FFFFu : 0u) | ((X1 + 1 == w1 - 1) ? 0xFFFF0000u : 0u);
+            auto pair1 = [&](int Y, int X) -> uint32_t { return *(const uint32_t *)&dw[Y][X] & 0x7FFF7FFFu; };
+            uint32_t hm[4];  // rows Y0 - 1 .. Y0 + 2 (dw rows 2 q .. 2 q + 3; rows outside the picture are not used)
 #pragma unroll
-            for (int k = 0; k < 6; k++) {
-                const int Y = 4 * q + k, Yp = Y0 + Y - 1;
-                hm[k] = (Yp < 0 || Yp >= h1) ? 0u : edge1 ? val(Y, X) : (mode3x2(val(Y, X - 1), val(Y, X), val(Y, X + 1)) & 0xFFFFu);
+            for (int k = 0; k < 4; k++) {
+                const uint32_t l2 = pair1(2 * q + k, 2 * p), m2 = pair1(2 * q + k, 2 * p + 2), r2 = pair1(2 * q + k, 2 * p + 4);
+                const uint32_t v = mode3x2(__byte_perm(l2, m2, 0x5432), m2, __byte_perm(m2, r2, 0x5432));
+                hm[k] = (m2 & edge1) | (v & ~edge1);
             }
+            const bool vec1 = (w1 & 1) == 0 && (((uintptr_t)J.word1) & 3) == 0;
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int Y1 = Y0 + 4 * q + i;
+            for (int i = 0; i < 2; i++) {
+                const int Y1 = Y0 + i;
                 if (Y1 >= h1) break;
-                const uint16_t word = dw[4 * q + i + 1][X];
-                const uint32_t v = (Y1 == 0 || Y1 == h1 - 1) ? (uint32_t)(word & 0x7FFFu) : (mode3x2(hm[i], hm[i + 1], hm[i + 2]) & 0xFFFFu);
-                J.word1[(size_t)Y1 * w1 + X1] = (uint16_t)(v | (word & kMaskBit));
+                const uint32_t word = *(const uint32_t *)&dw[2 * q + i + 1][2 * p + 2];
+                const uint32_t v = (Y1 == 0 || Y1 == h1 - 1) ? word & 0x7FFF7FFFu : mode3x2(hm[i], hm[i + 1], hm[i + 2]);
+                const uint32_t out = v | (word & 0x80008000u);
+                uint16_t *dst = J.word1 + (size_t)Y1 * w1 + X1;
+                if (vec1) {
+                    *(uint32_t *)dst = out;
+                } else {
+                    dst[0] = (uint16_t)out;
+                    if (X1 + 1 < w1) dst[1] = (uint16_t)(out >> 16);
+                }
             }
         }
     }
