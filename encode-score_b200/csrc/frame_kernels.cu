@@ -8,6 +8,8 @@
 // source's luma over the even and odd frame offsets (mid detail is linear in luma), so a frame step reads a few
 // 16-bit planes once for all encodes; and the per-frame reduction (structure threshold as an exact order statistic,
 // masks, sums, histogram bins) runs on the device.
+#include <type_traits>
+
 #include "es_kernels.h"
 
 namespace es {
@@ -176,71 +178,57 @@ __device__ __forceinline__ float oriented_of(long long jxx, long long jyy, long 
 // ---------------------------------------------------------------------------------------------------------------
 // Window statistics of one source frame against every encode: src/kernels.cu:346-428, exact.
 //
-// A block of 256 threads takes a 64 x 64 tile (4 x 4 windows) of every picture in turn. Per picture: the 72 x 72 region
-// (4-pixel margin, coordinates clamped) is staged in shared memory with 8-byte loads; each thread then builds the
-// horizontal 3- and 9-sums of 8 columns of a region row from two 16-byte reads; then thread (c, g) walks tile column c
-// down rows 16 g .. 16 g + 15 (one window's column) with running vertical sums, so the 3 x 3 and 9 x 9 sums of a pixel
-// cost a few additions. The 16 lanes of a window reduce its sums with shuffles.
+// A block of 128 threads takes a 64 x 64 tile (4 x 4 windows) of every picture in turn. Per picture: the 72 x 72 region
+// (4-pixel margin, coordinates clamped) is copied in asynchronously while the picture before is summed; the horizontal 3-
+// and 9-sums of 8 columns of a region row are made from two 16-byte reads, two columns to a word (no sum leaves 16 bits);
+// then thread (c, g) walks tile columns 2 c and 2 c + 1 down rows 16 g .. 16 g + 15 (two columns of one window) with
+// running vertical sums, the 3 x 3 sums two to a word. The 8 lanes of a window reduce its sums with shuffles.
+// Bound by integer issue. With one column per thread and one sum per word it took 121 us for a 3840 x 2160 source and
+// three encodes and 247 us for 16 uneven pairs; now 88 and 171 us. (The dot-product form of add_half pays for the 9 x 9
+// sums; used for the fine details and gradients too it made 102 and 203 us of these.)
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int kWT = 64;             // tile side
 constexpr int kWR = kWT + 2 * kM;   // region side, 72
 constexpr int kWS = 72;             // row stride of the region planes (144 bytes, a multiple of 16)
+constexpr int kWThreads = 128;
 
-struct WinSmem {
-    uint16_t y[kWR][kWS];   // y[r][j]: pixel (x0 - 4 + j, y0 - 4 + r), coordinates clamped
+using Region = uint16_t[kWR][kWS];  // [r][j]: pixel (x0 - 4 + j, y0 - 4 + r) of a plane, coordinates clamped
+
+struct WinSums {
     uint16_t h3[kWR][kWS];  // h3[r][k]: 3-sum of row r centred at x0 - 1 + k, k < 66
     uint16_t h9[kWR][kWT];  // h9[r][c]: 9-sum of row r centred at x0 + c
 };
 
-// h3 and h9 of every region row: item (r, s) covers columns 8 s .. 8 s + 7 from y[r][8 s .. 8 s + 15].
-__device__ __forceinline__ void window_horizontal_sums(WinSmem &sm)
+// h3 and h9 of every region row: item (r, s) covers columns 8 s .. 8 s + 7 from y[r][8 s .. 8 s + 15]; the sums are
+// shifted left by `up`. Pairs of neighbouring columns: p[k] holds columns 2 k and 2 k + 1, the pair one column on is one
+// byte permutation, and a pair of 9-sums is three pairs of 3-sums three columns apart.
+__device__ __forceinline__ void window_horizontal_sums(WinSums &sm, const Region &y, int up)
 {
-    for (int i = threadIdx.x; i < kWR * 8; i += 256) {
+    for (int i = threadIdx.x; i < kWR * 8; i += kWThreads) {
         const int r = i >> 3, c0 = 8 * (i & 7);
-        const uint4 a = *(const uint4 *)&sm.y[r][c0], b = *(const uint4 *)&sm.y[r][c0 + 8];
-        const unsigned wv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        int v[16];
+        const uint4 a = *(const uint4 *)&y[r][c0], b = *(const uint4 *)&y[r][c0 + 8];
+        const unsigned p[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        auto next = [](unsigned lo, unsigned hi) { return __byte_perm(lo, hi, 0x5432); };
+        unsigned t[7];  // t[k]: 3-sums from columns 2 k and 2 k + 1 on
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            v[2 * k] = (int)(wv[k] & 0xFFFFu);
-            v[2 * k + 1] = (int)(wv[k] >> 16);
-        }
-        int s9 = 0;
+        for (int k = 0; k < 7; k++) t[k] = p[k] + next(p[k], p[k + 1]) + p[k + 1];
+        unsigned h9[4];
 #pragma unroll
-        for (int k = 0; k < 9; k++) s9 += v[k];
-        int h9[8], h3[10];
-        h9[0] = s9;
-#pragma unroll
-        for (int k = 1; k < 8; k++) {
-            s9 += v[k + 8] - v[k - 1];
-            h9[k] = s9;
-        }
-#pragma unroll
-        for (int k = 0; k < 10; k++) h3[k] = v[k + 2] + v[k + 3] + v[k + 4];
-        *(uint4 *)&sm.h9[r][c0] = make_uint4(h9[0] | (h9[1] << 16), h9[2] | (h9[3] << 16), h9[4] | (h9[5] << 16), h9[6] | (h9[7] << 16));
-        *(uint4 *)&sm.h3[r][c0] = make_uint4(h3[0] | (h3[1] << 16), h3[2] | (h3[3] << 16), h3[4] | (h3[5] << 16), h3[6] | (h3[7] << 16));
-        if (c0 == 56) *(uint32_t *)&sm.h3[r][64] = h3[8] | (h3[9] << 16);
+        for (int k = 0; k < 4; k++) h9[k] = (t[k] + next(t[k + 1], t[k + 2]) + t[k + 3]) << up;
+        *(uint4 *)&sm.h9[r][c0] = make_uint4(h9[0], h9[1], h9[2], h9[3]);
+        *(uint4 *)&sm.h3[r][c0] = make_uint4(t[1] << up, t[2] << up, t[3] << up, t[4] << up);
+        if (c0 == 56) *(unsigned *)&sm.h3[r][64] = t[5] << up;
     }
 }
 
+// The sum over the 8 lanes of a window.
 template <typename T>
-__device__ __forceinline__ T half_warp_sum(T v)
+__device__ __forceinline__ T window_sum(T v)
 {
 #pragma unroll
-    for (int o = 8; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    for (int o = 4; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-
-// Dynamic shared memory: the region planes, then the source's fine and mid numerators of each thread's 16 rows, kept
-// for the encodes' cross products (|fine| <= 9 x 1023 fits 16 bits) in shared memory so that three blocks fit an SM's
-// registers, and two buffers of raw region values: the next picture's region is copied in (cp.async) while the
-// current one is summed.
-struct WinStatsSmem {
-    WinSmem sm;
-    int mr[kWin][256];
-    int16_t fr[kWin][256];
-    uint16_t raw[2][kWR][kWS];  // raw[b][r][j]: pixel (x0 - 4 + j, y0 - 4 + r) of a picture, coordinates clamped, unshifted
-};
 
 __device__ __forceinline__ void cp_async8(void *dst_smem, const void *src)
 {
@@ -253,16 +241,16 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // Queues the copy of `src`'s region at tile (x0, y0) into raw (unshifted; rows clamped): 8-byte asynchronous copies
 // where the columns lie inside the picture and the rows are 8-byte aligned, else plain loads and stores now. Every
 // thread commits one group of copies (possibly empty).
-__device__ __forceinline__ void stage_raw_async(uint16_t (*raw)[kWS], const uint16_t *src, int w, int h, int x0, int y0)
+__device__ __forceinline__ void stage_raw_async(Region &raw, const uint16_t *src, int w, int h, int x0, int y0)
 {
     if (x0 >= kM && x0 + kWT + kM <= w && (w & 3) == 0 && ((uintptr_t)src & 7) == 0) {
-        for (int i = threadIdx.x; i < kWR * 18; i += 256) {
+        for (int i = threadIdx.x; i < kWR * 18; i += kWThreads) {
             const int r = i / 18, q = i - r * 18;
             const int y = min(max(y0 - kM + r, 0), h - 1);
             cp_async8(&raw[r][4 * q], src + (size_t)y * w + (x0 - kM) + 4 * q);
         }
     } else {
-        for (int i = threadIdx.x; i < kWR * kWR; i += 256) {
+        for (int i = threadIdx.x; i < kWR * kWR; i += kWThreads) {
             const int r = i / kWR, j = i - r * kWR;
             const int x = min(max(x0 - kM + j, 0), w - 1), y = min(max(y0 - kM + r, 0), h - 1);
             raw[r][j] = src[(size_t)y * w + x];
@@ -271,44 +259,85 @@ __device__ __forceinline__ void stage_raw_async(uint16_t (*raw)[kWS], const uint
     cp_async_commit();
 }
 
-// window_horizontal_sums over a raw buffer, the sums shifted left by `up` (the values at the pipeline's depth).
-__device__ __forceinline__ void window_horizontal_sums_raw(WinSmem &sm, const uint16_t (*raw)[kWS], int up)
+// c + K times half `Hi` of a pair of unsigned 16-bit values: one instruction, beside the pipe of the additions and shifts.
+template <int K, int Hi>
+__device__ __forceinline__ int add_half(unsigned pair, int c)
 {
-    for (int i = threadIdx.x; i < kWR * 8; i += 256) {
-        const int r = i >> 3, c0 = 8 * (i & 7);
-        const uint4 a = *(const uint4 *)&raw[r][c0], b = *(const uint4 *)&raw[r][c0 + 8];
-        const unsigned wv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        int v[16];
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            v[2 * k] = (int)(wv[k] & 0xFFFFu);
-            v[2 * k + 1] = (int)(wv[k] >> 16);
-        }
-        int s9 = 0;
-#pragma unroll
-        for (int k = 0; k < 9; k++) s9 += v[k];
-        int h9[8], h3[10];
-        h9[0] = s9 << up;
-#pragma unroll
-        for (int k = 1; k < 8; k++) {
-            s9 += v[k + 8] - v[k - 1];
-            h9[k] = s9 << up;
-        }
-#pragma unroll
-        for (int k = 0; k < 10; k++) h3[k] = (v[k + 2] + v[k + 3] + v[k + 4]) << up;
-        *(uint4 *)&sm.h9[r][c0] = make_uint4(h9[0] | (h9[1] << 16), h9[2] | (h9[3] << 16), h9[4] | (h9[5] << 16), h9[6] | (h9[7] << 16));
-        *(uint4 *)&sm.h3[r][c0] = make_uint4(h3[0] | (h3[1] << 16), h3[2] | (h3[3] << 16), h3[4] | (h3[5] << 16), h3[6] | (h3[7] << 16));
-        if (c0 == 56) *(uint32_t *)&sm.h3[r][64] = h3[8] | (h3[9] << 16);
-    }
+    static_assert(K >= -128 && K < 128, "a signed byte");
+    int d;
+    asm("dp2a.lo.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(pair), "r"((K & 0xFF) << 8 * Hi), "r"(c));
+    return d;
 }
 
-__global__ void __launch_bounds__(256, 3) window_stats_kernel(const __grid_constant__ WindowBatch B)
+// Vertical running sums of two neighbouring columns (tile columns c, c + 1, c even) down a window's 16 rows: start at row
+// r0 - 1's successor state, then next() once per row.
+struct ColumnPair {
+    const WinSums &sm;
+    int c, row;            // tile row the sums are at
+    unsigned a1, a2, b1, b2;  // h3 words (columns left of and at c; right of c and of c + 1) of rows row, row + 1
+    unsigned l, r;            // 3 x 3 sums left of the pair's columns, right of them
+    int n9[2];                // minus the 9 x 9 sums
+    __device__ __forceinline__ unsigned h3(int t, int k) const { return *(const unsigned *)&sm.h3[t + kM][c + 2 * k]; }
+    __device__ __forceinline__ unsigned h9(int t) const { return *(const unsigned *)&sm.h9[t + kM][c]; }
+    __device__ __forceinline__ unsigned centre() const { return __byte_perm(l, r, 0x5432); }
+    __device__ __forceinline__ ColumnPair(const WinSums &s, int c_, int r0) : sm(s), c(c_), row(r0)
+    {
+        a1 = h3(r0, 0);
+        b1 = h3(r0, 1);
+        a2 = h3(r0 + 1, 0);
+        b2 = h3(r0 + 1, 1);
+        l = h3(r0 - 1, 0) + a1 + a2;
+        r = h3(r0 - 1, 1) + b1 + b2;
+        n9[0] = n9[1] = 0;
+#pragma unroll
+        for (int k = -4; k <= 4; k++) add9<-1>(h9(r0 + k));
+    }
+    // the 3 x 3 sums of the row above the current one
+    __device__ __forceinline__ unsigned centre_above() const
+    {
+        const unsigned a = h3(row - 2, 0) + h3(row - 1, 0) + a1, b = h3(row - 2, 1) + h3(row - 1, 1) + b1;
+        return __byte_perm(a, b, 0x5432);
+    }
+    // the 3 x 3 sums on to the next row (first half), the 9 x 9 sums (second half)
+    __device__ __forceinline__ void next3()
+    {
+        const unsigned a3 = h3(row + 2, 0), b3 = h3(row + 2, 1);
+        l = a1 + a2 + a3;
+        r = b1 + b2 + b3;
+        a1 = a2;
+        a2 = a3;
+        b1 = b2;
+        b2 = b3;
+    }
+    __device__ __forceinline__ void next9()
+    {
+        add9<-1>(h9(row + 5));
+        add9<1>(h9(row - 4));
+        row++;
+    }
+    template <int K>
+    __device__ __forceinline__ void add9(unsigned v)
+    {
+        n9[0] = add_half<K, 0>(v, n9[0]);
+        n9[1] = add_half<K, 1>(v, n9[1]);
+    }
+    // mid-detail numerator 9 S3 - S9 of the pair's column k
+    template <int Hi>
+    __device__ __forceinline__ int mid(unsigned here) const
+    {
+        return add_half<9, Hi>(here, n9[Hi]);
+    }
+};
+
+struct WinStatsSmem {
+    WinSums sm;
+    Region raw[2];  // the next picture's region is copied in while the current one is summed
+};
+
+__global__ void __launch_bounds__(kWThreads, 4) window_stats_kernel(const __grid_constant__ WindowBatch B)
 {
     extern __shared__ __align__(16) unsigned char win_dyn[];
     WinStatsSmem &ws = *(WinStatsSmem *)win_dyn;
-    WinSmem &sm = ws.sm;
-    auto &fr_s = ws.fr;
-    auto &mr_s = ws.mr;
     const int jb = find_job(B.njobs, (int)blockIdx.x, [&](int k) { return B.job[k].first_block; });
     const WindowJob &J = B.job[jb];
     const int bid = blockIdx.x - J.first_block;
@@ -316,78 +345,71 @@ __global__ void __launch_bounds__(256, 3) window_stats_kernel(const __grid_const
     const int tiles_x = (ww + 3) / 4;
     const int x0 = (bid % tiles_x) * kWT, y0 = (bid / tiles_x) * kWT;
     const int tid = threadIdx.x, lane = tid & 31;
-    const int c = tid & (kWT - 1), r0 = (tid >> 6) * kWin;  // tile column, first tile row
+    const int c = 2 * lane, r0 = (tid >> 5) * kWin;  // tile columns c and c + 1, first tile row
     const int wx = (x0 + c) / kWin, wy = (y0 + r0) / kWin;
     const bool inside = wx < ww && wy < wh;
-    const int x = x0 + c;
-    const bool gx_on = x > 0 && x < w - 1;
+    const int x = x0 + c, up = J.up;
+    const bool gx_on[2] = {x > 0 && x < w - 1, x + 1 < w - 1};
     unsigned long long src_f = 0, src_m = 0, src_xx = 0, src_yy = 0;
     long long src_xy = 0;
-    const int up = J.up;
-    stage_raw_async(ws.raw[0], J.yr, w, h, x0, y0);
-    for (int p = 0; p <= J.nenc; p++) {
-        const uint16_t(*raw)[kWS] = ws.raw[p & 1];
-        __syncthreads();  // the walk of picture p - 1 is done with the buffer picture p + 1 goes to
-        if (p < J.nenc) {
-            stage_raw_async(ws.raw[(p + 1) & 1], J.yd[p], w, h, x0, y0);
-            cp_async_wait<1>();  // picture p's copies are in; p + 1's may still be in flight
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-        window_horizontal_sums_raw(sm, raw, up);
-        __syncthreads();
-        // tile row t is region row t + 4; h3 column c + 1 is centred at x, c and c + 2 at x -+ 1
-        auto h3c = [&](int t) { return (int)sm.h3[t + kM][c + 1]; };
-        auto h3l = [&](int t) { return (int)sm.h3[t + kM][c]; };
-        auto h3r = [&](int t) { return (int)sm.h3[t + kM][c + 2]; };
-        auto h9c = [&](int t) { return (int)sm.h9[t + kM][c]; };
-        int s3_prev = h3c(r0 - 2) + h3c(r0 - 1) + h3c(r0);      // S3 at row r0 - 1
-        int s3 = s3_prev - h3c(r0 - 2) + h3c(r0 + 1);            // S3 at row r0
-        int s3l = h3l(r0 - 1) + h3l(r0) + h3l(r0 + 1), s3r = h3r(r0 - 1) + h3r(r0) + h3r(r0 + 1);
-        int s9 = 0;
-#pragma unroll
-        for (int k = -4; k <= 4; k++) s9 += h9c(r0 + k);
+    unsigned fr[kWin] = {};  // the source's fine numerators of the thread's pixels (|f| <= 9 x 1023: 16 bits each)
+    int mr[kWin][2] = {};    // and its mid numerators, for the encodes' cross products
+    auto walk = [&](auto first, const Region &raw, int p) {
+        constexpr bool kFirst = decltype(first)::value;
+        ColumnPair s(ws.sm, c, r0);
+        unsigned above = s.centre_above(), here = s.centre();
         unsigned fine_sq = 0, jxx = 0, jyy = 0;
-        int jxy = 0, fine_x = 0;
+        int jxy[2] = {0, 0}, fine_x[2] = {0, 0};  // 16 products each stay below 2^31
         unsigned long long mid_sq = 0;
         long long mid_x = 0;
 #pragma unroll
         for (int i = 0; i < kWin; i++) {
-            const int t = r0 + i, y = y0 + t;
-            const int s3_next = s3 - h3c(t - 1) + h3c(t + 2);
-            const int f = 9 * ((int)raw[t + kM][c + kM] << up) - s3, m = 9 * s3 - s9;
-            const int gx = gx_on ? s3r - s3l : 0;
-            const int gy = (y > 0 && y < h - 1) ? s3_next - s3_prev : 0;
-            if (p == 0) {
-                fr_s[i][tid] = (int16_t)f;
-                mr_s[i][tid] = m;
-            } else {
-                fine_x += f * (int)fr_s[i][tid];
-                mid_x += (long long)m * mr_s[i][tid];
-            }
-            fine_sq += (unsigned)(f * f);
-            mid_sq += (unsigned long long)((long long)m * m);
-            jxx += (unsigned)(gx * gx);
-            jyy += (unsigned)(gy * gy);
-            jxy += gx * gy;
-            if (i + 1 < kWin) {
-                s3_prev = s3;
-                s3 = s3_next;
-                s3l += h3l(t + 2) - h3l(t - 1);
-                s3r += h3r(t + 2) - h3r(t - 1);
-                s9 += h9c(t + 5) - h9c(t - 4);
-            }
+            const int y = y0 + r0 + i;
+            const bool gy_on = y > 0 && y < h - 1;
+            const unsigned v = *(const unsigned *)&raw[r0 + i + kM][c + kM] << up, left = s.l, right = s.r;
+            s.next3();  // the next row's 3 x 3 sums, for the vertical gradient
+            const unsigned below = s.centre();
+            // differences of pairs, 0x8000 added to each half so that nothing is borrowed between them
+            const unsigned dx = right + 0x80008000u - left, dy = below + 0x80008000u - above;
+            unsigned f16[2];
+            auto column = [&](auto which) {
+                constexpr int k = decltype(which)::value;
+                auto half = [&](unsigned q) { return (int)(k ? q >> 16 : q & 0xFFFFu); };
+                const int s3 = half(here), f = 9 * half(v) - s3, m = 9 * s3 + s.n9[k];
+                const int gx = gx_on[k] ? half(dx) - 0x8000 : 0, gy = gy_on ? half(dy) - 0x8000 : 0;
+                f16[k] = (unsigned)f;
+                if (kFirst) {
+                    mr[i][k] = m;
+                } else {
+                    fine_x[k] += f * (k ? (int)fr[i] >> 16 : (int)(short)fr[i]);
+                    mid_x += (long long)m * mr[i][k];
+                }
+                fine_sq += (unsigned)(f * f);
+                mid_sq += (unsigned long long)((long long)m * m);
+                jxx += (unsigned)(gx * gx);
+                jyy += (unsigned)(gy * gy);
+                jxy[k] += gx * gy;
+            };
+            column(std::integral_constant<int, 0>{});
+            column(std::integral_constant<int, 1>{});
+            if (kFirst) fr[i] = __byte_perm(f16[0], f16[1], 0x5410);
+            above = here;
+            here = below;
+            if (i + 1 < kWin) s.next9();
         }
-        const unsigned long long sf = half_warp_sum((unsigned long long)fine_sq), sm2 = half_warp_sum(mid_sq),
-                                 sxx = half_warp_sum((unsigned long long)jxx), syy = half_warp_sum((unsigned long long)jyy);
-        const long long sxy = half_warp_sum((long long)jxy);
-        if (p == 0) {
-            src_f = sf; src_m = sm2; src_xx = sxx; src_yy = syy; src_xy = sxy;
-            continue;
+        const unsigned long long sf = window_sum((unsigned long long)fine_sq), sm2 = window_sum(mid_sq),
+                                 sxx = window_sum((unsigned long long)jxx), syy = window_sum((unsigned long long)jyy);
+        const long long sxy = window_sum((long long)jxy[0] + jxy[1]);
+        if (kFirst) {
+            src_f = sf;
+            src_m = sm2;
+            src_xx = sxx;
+            src_yy = syy;
+            src_xy = sxy;
+            return;
         }
-        const long long cf = half_warp_sum((long long)fine_x), cm = half_warp_sum(mid_x);
-        if (inside && (lane & 15) == 0) {
+        const long long cf = window_sum((long long)fine_x[0] + fine_x[1]), cm = window_sum(mid_x);
+        if (inside && (lane & 7) == 0) {
             float *o = J.stats + (((size_t)(p - 1) * wh + wy) * ww + wx) * 8;
             o[0] = exact_ratio((long long)src_f, 81.0);
             o[1] = exact_ratio((long long)src_m, 6561.0);
@@ -398,156 +420,161 @@ __global__ void __launch_bounds__(256, 3) window_stats_kernel(const __grid_const
             o[6] = oriented_of((long long)src_xx, (long long)src_yy, src_xy);
             o[7] = oriented_of((long long)sxx, (long long)syy, sxy);
         }
+    };
+    stage_raw_async(ws.raw[0], J.yr, w, h, x0, y0);
+    for (int p = 0; p <= J.nenc; p++) {
+        const Region &raw = ws.raw[p & 1];
+        __syncthreads();  // the walk of picture p - 1 is done with the buffer picture p + 1 goes to
+        if (p < J.nenc) {
+            stage_raw_async(ws.raw[(p + 1) & 1], J.yd[p], w, h, x0, y0);
+            cp_async_wait<1>();  // picture p's copies are in; p + 1's may still be in flight
+        } else {
+            cp_async_wait<0>();
+        }
+        __syncthreads();
+        window_horizontal_sums(ws.sm, raw, up);
+        __syncthreads();
+        if (p == 0) walk(std::true_type{}, raw, p);
+        else walk(std::false_type{}, raw, p);
     }
 }
 
 // ---------------------------------------------------------------------------------------------------------------
 // Lasting texture: src/kernels.cu:435-451, exact, from running luma sums (see PersistJob).
 //
-// A block of 256 threads takes a 64 x 64 tile (4 x 4 windows): it advances the running sums E and O over the tile and
-// its 4-pixel margin (coordinates clamped, so the margins repeat the edges) and writes them for the tile's own pixels;
-// then, as in window_stats, the horizontal 3- and 9-sums of E, of O and of each picture are built in shared memory and
-// thread (c, g) walks tile column c down window row g with running vertical sums of the mid-detail numerators.
+// advance_kernel moves the running sums E and O on by a frame, 8 pixels per thread with 16-byte accesses: a pass over six
+// planes in and two out, bound by memory. persist_kernel then treats E, O, the centre frame and the encodes' pictures as
+// window_stats treats its pictures: regions copied in asynchronously, horizontal sums, and thread (c, g) walks tile
+// columns 2 c and 2 c + 1 down window row g with running vertical sums of the mid-detail numerators. When each tile
+// advanced its own region of the sums first, the scattered 8-byte loads of that part alone took 59 of 98 us for a 3840 x
+// 2160 pair at 20 % of the memory's rate. One kernel with a column per thread took 82 us for that pair, 107 us with three
+// encodes and 317 us for 16 uneven pairs; the two now take 78, 104 and 296 us, of which 26, 26 and 93 us advance.
 // ---------------------------------------------------------------------------------------------------------------
-// mid-detail numerators 9 S3 - S9 of the 16 rows from tile row r0 at tile column c, from the horizontal sums
-__device__ __forceinline__ void window_mids(const WinSmem &sm, int c, int r0, int (&m)[kWin])
+struct AdvanceJob {
+    const uint16_t *e_old, *o_old, *y_m13, *y_m7, *y_c, *y_f;
+    uint16_t *e_new, *o_new;
+    size_t n;
+    int up, first_block;
+};
+struct AdvanceBatch {
+    AdvanceJob job[kMaxSources];
+    int njobs;
+};
+constexpr int kAdvThreads = 256;
+constexpr int kAdvPixels = 8 * kAdvThreads;  // per block
+
+__global__ void __launch_bounds__(kAdvThreads) advance_kernel(const __grid_constant__ AdvanceBatch B)
 {
-    auto h3c = [&](int t) { return (int)sm.h3[t + kM][c + 1]; };
-    auto h9c = [&](int t) { return (int)sm.h9[t + kM][c]; };
-    int s3 = h3c(r0 - 1) + h3c(r0) + h3c(r0 + 1);
-    int s9 = 0;
-#pragma unroll
-    for (int k = -4; k <= 4; k++) s9 += h9c(r0 + k);
+    const int jb = find_job(B.njobs, (int)blockIdx.x, [&](int k) { return B.job[k].first_block; });
+    const AdvanceJob &J = B.job[jb];
+    const size_t at = (size_t)(blockIdx.x - J.first_block) * kAdvPixels + 8 * threadIdx.x;
+    if (at >= J.n) return;
+    const int up = J.up;
+    // E(c) = O(c-1) - y(c) + y(c+6), O(c) = E(c-1) - y(c-7) + y(c-1); a missing frame is 0
+    uintptr_t align = (uintptr_t)J.e_old | (uintptr_t)J.o_old | (uintptr_t)J.e_new | (uintptr_t)J.o_new;
+    align |= (uintptr_t)J.y_m13 | (uintptr_t)J.y_m7 | (uintptr_t)J.y_c | (uintptr_t)J.y_f;
+    if (at + 8 <= J.n && (align & 15) == 0) {
+        auto load = [&](const uint16_t *p) { return p ? __ldg((const uint4 *)(p + at)) : make_uint4(0, 0, 0, 0); };
+        const uint4 a = load(J.o_old), b = load(J.y_c), c = load(J.y_f), d = load(J.e_old), e = load(J.y_m13), f = load(J.y_m7);
+        // no element leaves 0 .. 65535 (the leaving frame is part of the old sum), so 32-bit arithmetic on the pairs
+        // carries and borrows nothing between the halves
+        *(uint4 *)(J.e_new + at) = make_uint4(a.x - (b.x << up) + (c.x << up), a.y - (b.y << up) + (c.y << up),
+                                              a.z - (b.z << up) + (c.z << up), a.w - (b.w << up) + (c.w << up));
+        *(uint4 *)(J.o_new + at) = make_uint4(d.x - (e.x << up) + (f.x << up), d.y - (e.y << up) + (f.y << up),
+                                              d.z - (e.z << up) + (f.z << up), d.w - (e.w << up) + (f.w << up));
+        return;
+    }
+    const size_t end = J.n < at + 8 ? J.n : at + 8;
+    for (size_t k = at; k < end; k++) {
+        auto value = [&](const uint16_t *p) { return p ? (int)(p[k] << up) : 0; };
+        J.e_new[k] = (uint16_t)((int)J.o_old[k] - value(J.y_c) + value(J.y_f));
+        J.o_new[k] = (uint16_t)((int)J.e_old[k] - value(J.y_m13) + value(J.y_m7));
+    }
+}
+
+// put(i, k, m): the mid-detail numerator 9 S3 - S9 of row r0 + i, column c + k, from the horizontal sums
+template <typename Put>
+__device__ __forceinline__ void window_mids(const WinSums &sm, int c, int r0, Put put)
+{
+    ColumnPair s(sm, c, r0);
 #pragma unroll
     for (int i = 0; i < kWin; i++) {
-        const int t = r0 + i;
-        m[i] = 9 * s3 - s9;
+        const unsigned here = s.centre();
+        put(i, 0, s.mid<0>(here));
+        put(i, 1, s.mid<1>(here));
         if (i + 1 < kWin) {
-            s3 += h3c(t + 2) - h3c(t - 1);
-            s9 += h9c(t + 5) - h9c(t - 4);
+            s.next3();
+            s.next9();
         }
     }
 }
 
-// Dynamic shared memory of persist_kernel: the region planes, the odd running sums of the region, and two buffers of
-// raw picture regions (the pictures' regions are copied in asynchronously, the first one while the sums advance).
+// Dynamic shared memory of persist_kernel: the region's horizontal sums and two buffers of raw regions.
 struct PersistSmem {
-    WinSmem sm;
-    uint16_t o_reg[kWR][kWS];
-    uint16_t raw[2][kWR][kWS];
+    WinSums sm;
+    Region raw[2];
 };
 
-__global__ void __launch_bounds__(256, 3) persist_kernel(const __grid_constant__ PersistBatch B)
+__global__ void __launch_bounds__(kWThreads, 4) persist_kernel(const __grid_constant__ PersistBatch B)
 {
     extern __shared__ __align__(16) unsigned char persist_dyn[];
     PersistSmem &ps = *(PersistSmem *)persist_dyn;
-    WinSmem &sm = ps.sm;
-    auto &o_reg = ps.o_reg;
     const int jb = find_job(B.njobs, (int)blockIdx.x, [&](int k) { return B.job[k].first_block; });
     const PersistJob &J = B.job[jb];
     const int bid = blockIdx.x - J.first_block;
     const int w = J.w, h = J.h, ww = w / kWin, wh = h / kWin;
-    const int tiles_x = (w + kWT - 1) / kWT;
+    const int tiles_x = (ww + 3) / 4;
     const int x0 = (bid % tiles_x) * kWT, y0 = (bid / tiles_x) * kWT;
     const int tid = threadIdx.x, lane = tid & 31;
-    if (J.stats) stage_raw_async(ps.raw[0], J.y_c, w, h, x0, y0);  // the centre frame's region, while the sums advance
-    // advance the running sums over the region: E(c) = O(c-1) - y(c) + y(c+6), O(c) = E(c-1) - y(c-7) + y(c-1)
-    const uint16_t *pl[4] = {J.y_m13, J.y_m7, J.y_c, J.y_f};
-    uintptr_t align = (uintptr_t)J.e_old | (uintptr_t)J.o_old | (uintptr_t)J.e_new | (uintptr_t)J.o_new;
-    for (int k = 0; k < 4; k++) align |= (uintptr_t)pl[k];
-    if (x0 >= kM && x0 + kWT + kM <= w && (w & 3) == 0 && (align & 7) == 0) {
-        // interior columns: 18 groups of 4 pixels per region row, packed 16-bit arithmetic (no element leaves 0..65535)
-        for (int i = tid; i < kWR * 18; i += 256) {
-            const int r = i / 18, q = i - r * 18, yu = y0 - kM + r, y = min(max(yu, 0), h - 1);
-            const size_t k = (size_t)y * w + (x0 - kM) + 4 * q;
-            uint2 v[4];
-#pragma unroll
-            for (int n = 0; n < 4; n++) {
-                v[n] = pl[n] ? __ldg((const uint2 *)(pl[n] + k)) : make_uint2(0, 0);
-                v[n].x <<= J.up;
-                v[n].y <<= J.up;
-            }
-            const uint2 oo = __ldg((const uint2 *)(J.o_old + k)), eo = __ldg((const uint2 *)(J.e_old + k));
-            // no element leaves 0 .. 65535 (the leaving frame is part of the old sum), so 32-bit arithmetic on the
-            // pairs carries and borrows nothing between the halves
-            const uint2 e = make_uint2(oo.x - v[2].x + v[3].x, oo.y - v[2].y + v[3].y);
-            const uint2 o = make_uint2(eo.x - v[0].x + v[1].x, eo.y - v[0].y + v[1].y);
-            *(uint2 *)&sm.y[r][4 * q] = e;
-            *(uint2 *)&o_reg[r][4 * q] = o;
-            if (r >= kM && r < kM + kWT && yu < h && q >= 1 && q <= 16) {
-                *(uint2 *)(J.e_new + k) = e;
-                *(uint2 *)(J.o_new + k) = o;
-            }
-        }
-    } else {
-        for (int i = tid; i < kWR * kWR; i += 256) {
-            const int r = i / kWR, cc = i - r * kWR;
-            const int xi = x0 - kM + cc, yi = y0 - kM + r;
-            const int x = min(max(xi, 0), w - 1), y = min(max(yi, 0), h - 1);
-            const size_t k = (size_t)y * w + x;
-            int yv[4];
-#pragma unroll
-            for (int n = 0; n < 4; n++) yv[n] = pl[n] ? (int)(pl[n][k] << J.up) : 0;
-            const int e = (int)J.o_old[k] - yv[2] + yv[3];
-            const int o = (int)J.e_old[k] - yv[0] + yv[1];
-            sm.y[r][cc] = (uint16_t)e;
-            o_reg[r][cc] = (uint16_t)o;
-            if (xi >= x0 && xi < x0 + kWT && yi >= y0 && yi < y0 + kWT && xi < w && yi < h) {
-                J.e_new[k] = (uint16_t)e;
-                J.o_new[k] = (uint16_t)o;
-            }
-        }
-    }
-    if (!J.stats) return;
-    const int c = tid & (kWT - 1), r0 = (tid >> 6) * kWin;
+    const int c = 2 * lane, r0 = (tid >> 5) * kWin;
     const int wx = (x0 + c) / kWin, wy = (y0 + r0) / kWin;
     const bool inside = wx < ww && wy < wh;
-    int a[kWin], bb[kWin], t[kWin];
-    __syncthreads();
-    window_horizontal_sums(sm);
-    __syncthreads();
-    window_mids(sm, c, r0, a);  // A x 486 = mid x 81 of E
-    __syncthreads();
-    for (int i = tid; i < kWR * kWS / 8; i += 256) ((uint4 *)&sm.y[0][0])[i] = ((const uint4 *)&o_reg[0][0])[i];
-    __syncthreads();
-    window_horizontal_sums(sm);
-    __syncthreads();
-    window_mids(sm, c, r0, bb);  // B x 486
-    long long sab = 0, saa = 0, sbb = 0;
-#pragma unroll
-    for (int i = 0; i < kWin; i++) {
-        t[i] = a[i] + bb[i];  // T x 972
-        sab += (long long)a[i] * bb[i];
-        saa += (long long)a[i] * a[i];
-        sbb += (long long)bb[i] * bb[i];
-    }
-    sab = half_warp_sum(sab);
-    saa = half_warp_sum(saa);
-    sbb = half_warp_sum(sbb);
-    long long own = 0;
-    for (int p = 0; p <= J.nenc; p++) {
-        __syncthreads();  // picture p - 1's sums are read, and its buffer is the one picture p + 1 goes to
-        if (p < J.nenc) {
-            stage_raw_async(ps.raw[(p + 1) & 1], J.yd[p], w, h, x0, y0);
+    // pictures in turn: E, O, the centre frame, the encodes at the centre frame
+    const int last = J.nenc + 2;
+    auto stage = [&](int p) {
+        const uint16_t *src = p == 0 ? J.e_new : p == 1 ? J.o_new : p == 2 ? J.y_c : J.yd[p - 3];
+        stage_raw_async(ps.raw[p & 1], src, w, h, x0, y0);
+    };
+    auto sums = [&](int p) {  // horizontal sums of picture p; picture p + 1's copies go on meanwhile
+        __syncthreads();      // the sums of picture p - 1 are read, and its buffer takes picture p + 1
+        if (p < last) {
+            stage(p + 1);
             cp_async_wait<1>();
         } else {
             cp_async_wait<0>();
         }
         __syncthreads();
-        window_horizontal_sums_raw(sm, ps.raw[p & 1], J.up);
+        window_horizontal_sums(ps.sm, ps.raw[p & 1], p < 2 ? 0 : J.up);
         __syncthreads();
-        int m[kWin];
-        window_mids(sm, c, r0, m);
+    };
+    int t[kWin][2] = {};  // A x 486 = mid x 81 of E, then T = A + B, x 972
+    stage(0);
+    sums(0);
+    window_mids(ps.sm, c, r0, [&](int i, int k, int m) { t[i][k] = m; });
+    long long sab = 0, saa = 0, sbb = 0;
+    sums(1);
+    window_mids(ps.sm, c, r0, [&](int i, int k, int m) {  // B x 486
+        const int a = t[i][k];
+        t[i][k] = a + m;
+        sab += (long long)a * m;
+        saa += (long long)a * a;
+        sbb += (long long)m * m;
+    });
+    sab = window_sum(sab);
+    saa = window_sum(saa);
+    sbb = window_sum(sbb);
+    long long own = 0;
+    for (int p = 2; p <= last; p++) {
+        sums(p);
         long long sp = 0;
-#pragma unroll
-        for (int i = 0; i < kWin; i++) sp += (long long)m[i] * t[i];
-        sp = half_warp_sum(sp);
-        if (p == 0) {
+        window_mids(ps.sm, c, r0, [&](int i, int k, int m) { sp += (long long)m * t[i][k]; });
+        sp = window_sum(sp);
+        if (p == 2) {
             own = sp;
             continue;
         }
-        if (inside && (lane & 15) == 0) {
-            float *o = J.out + (((size_t)(p - 1) * wh + wy) * ww + wx) * 5;
+        if (inside && (lane & 7) == 0) {
+            float *o = J.out + (((size_t)(p - 3) * wh + wy) * ww + wx) * 5;
             o[0] = exact_ratio(own, 78732.0);
             o[1] = exact_ratio(sp, 78732.0);
             o[2] = exact_ratio(sab, 236196.0);
@@ -919,23 +946,31 @@ cudaError_t launch_window_stats(WindowBatch &b, cudaStream_t s)
                                                (int)sizeof(WinStatsSmem));
     if (e != cudaSuccess) return e;
     LaunchTimer t("window_stats", s);
-    window_stats_kernel<<<blocks, 256, sizeof(WinStatsSmem), s>>>(b);
+    window_stats_kernel<<<blocks, kWThreads, sizeof(WinStatsSmem), s>>>(b);
     return after_launch();
 }
 
 cudaError_t launch_persist(PersistBatch &b, cudaStream_t s)
 {
+    AdvanceBatch ab{};
+    size_t advance = 0;
     int blocks = 0;
     for (int j = 0; j < b.njobs; j++) {
         PersistJob &J = b.job[j];
+        const size_t n = (size_t)J.w * J.h;
+        ab.job[ab.njobs++] = AdvanceJob{J.e_old, J.o_old, J.y_m13, J.y_m7, J.y_c, J.y_f, J.e_new, J.o_new, n, J.up, (int)advance};
+        advance += (n + kAdvPixels - 1) / kAdvPixels;
         J.first_block = blocks;
-        blocks += ((J.w + kWT - 1) / kWT) * ((J.h + kWT - 1) / kWT);
+        if (J.stats) blocks += ((J.w / kWin + 3) / 4) * ((J.h / kWin + 3) / 4);
     }
-    if (blocks == 0) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(persist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PersistSmem));
-    if (e != cudaSuccess) return e;
+    if (advance == 0) return cudaSuccess;
     LaunchTimer t("persist_stats", s);
-    persist_kernel<<<blocks, 256, sizeof(PersistSmem), s>>>(b);
+    advance_kernel<<<(unsigned)advance, kAdvThreads, 0, s>>>(ab);
+    cudaError_t e = after_launch();
+    if (e != cudaSuccess || blocks == 0) return e;
+    e = cudaFuncSetAttribute(persist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PersistSmem));
+    if (e != cudaSuccess) return e;
+    persist_kernel<<<blocks, kWThreads, sizeof(PersistSmem), s>>>(b);
     return after_launch();
 }
 
