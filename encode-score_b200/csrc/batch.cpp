@@ -56,6 +56,7 @@ struct Picture {
     int sw[kScales], sh[kScales];
     DeviceBuffer<uint16_t> words[kScales];
     DeviceBuffer<float> lists[kScales];
+    DeviceBuffer<unsigned> strips;  // Prep0Job::strips
 };
 }  // namespace
 
@@ -65,6 +66,7 @@ struct es_batch {
     int max_pad = 0;
     DeviceBuffer<CvSlot> slots;  // pictures x kScales
     DeviceBuffer<unsigned long long> slot_n, slot_k;
+    DeviceBuffer<unsigned> busy;  // CvBatch::busy
     DeviceBuffer<float> lut;
     DeviceBuffer<double> scores;  // pictures x (1 + kScales): score, then pooled per scale
     PinnedBuffer<double> h_scores[2];
@@ -179,6 +181,11 @@ void init_source(Source &S, const es_batch_source &d)
     cuda_check(cudaMemset(S.masks.ptr, 0, S.masks.bytes()), "clearing");
 }
 
+int scale_tiles(const Picture &pic, int s)
+{
+    return ((pic.sw[s] + kCvTX - 1) / kCvTX) * ((pic.sh[s] + pic.tile_rows[s] - 1) / pic.tile_rows[s]);
+}
+
 void init_cambi(es_batch &b)
 {
     const int P = (int)b.pictures.size();
@@ -186,6 +193,7 @@ void init_cambi(es_batch &b)
     std::vector<CvSlot> init(P * kScales);
     std::memset(init.data(), 0, sizeof(CvSlot) * init.size());
     int tiles0 = 0;
+    size_t tiles = 0;
     for (auto &pic : b.pictures) tiles0 += cv_tiles(pic->w, pic->h);
     for (int i = 0; i < P; i++) {
         Picture &pic = *b.pictures[i];
@@ -197,6 +205,7 @@ void init_cambi(es_batch &b)
         }
         for (int s = 0; s < kScales; s++) {
             if (!pic.tile_rows[s]) pic.tile_rows[s] = cv_default_tile_rows(pic.sw[s], pic.sh[s], tiles0);
+            tiles += scale_tiles(pic, s);
             const size_t m = (size_t)pic.sw[s] * pic.sh[s];
             pic.words[s].reset(m);
             pic.lists[s].reset(m);
@@ -207,6 +216,10 @@ void init_cambi(es_batch &b)
         b.max_pad = std::max(b.max_pad, pic.p.pad);
     }
     b.slots.reset(init.size());
+    if (tiles >= kCvBusyTiles) {
+        b.busy.reset(2 + 2 * tiles);
+        for (auto &pic : b.pictures) pic->strips.reset(prep0_strips(pic->w, pic->h));
+    }
     b.slot_n.reset(n.size());
     b.slot_k.reset(k.size());
     cuda_check(cudaMemcpy(b.slots.ptr, init.data(), sizeof(CvSlot) * init.size(), cudaMemcpyHostToDevice), "batch set-up");
@@ -369,6 +382,10 @@ void record_cambi(es_batch &b, long f, uint32_t skip, cudaStream_t s)
     }
     if (run.empty()) return;
     const Band band = band_of(b.pictures[0]->p);
+    size_t run_tiles = 0;
+    for (int i : run)
+        for (int sc = 0; sc < kScales; sc++) run_tiles += scale_tiles(*b.pictures[i], sc);
+    const bool busy = !b.net && run_tiles >= kCvBusyTiles;  // c-values from a list of the busy tiles
     Prep0Batch pb{};
     int pred_tiles = 0;  // with the proposal, scale 0 also makes the feature maps and the tiles' need flags
     for (int i : run) {
@@ -384,6 +401,7 @@ void record_cambi(es_batch &b, long f, uint32_t skip, cudaStream_t s)
         j.word1 = pic.words[1].ptr;
         j.w1 = pic.sw[1];
         j.h1 = pic.sh[1];
+        if (busy) j.strips = pic.strips.ptr;
         if (b.net) {
             j.feat = b.feat.ptr + b.feat_at[i];
             j.need = b.need.ptr + pred_tiles;
@@ -396,6 +414,7 @@ void record_cambi(es_batch &b, long f, uint32_t skip, cudaStream_t s)
     pb.nslots = nslots;
     pb.slot_n = b.slot_n.ptr;
     pb.slot_k = b.slot_k.ptr;
+    pb.clear = busy ? b.busy.ptr : nullptr;
     cuda_check(launch_prep0(pb, s), "batch scales 0 and 1");
     CvBatch cb{};
     int tiles = 0;
@@ -412,6 +431,8 @@ void record_cambi(es_batch &b, long f, uint32_t skip, cudaStream_t s)
             j.slot = i * kScales + sc;
             j.plane = pic.cv_plane[sc];
             j.tile_rows = (b.net && sc < 2) ? 64 : pic.tile_rows[sc];  // the proposal maps 64-row tiles of scales 0, 1
+            j.scale = sc;
+            if (busy && sc < 2) j.strips = pic.strips.ptr + sc * (pic.strips.count / 2);
             tiles += j.tiles_x * ((j.h + j.tile_rows - 1) / j.tile_rows);
         }
     }
@@ -446,6 +467,7 @@ void record_cambi(es_batch &b, long f, uint32_t skip, cudaStream_t s)
     }
     cuda_check(launch_decimate_mode(db, s), "batch scales");
     if (!b.net) {
+        if (busy) cb.busy = b.busy.ptr;
         cuda_check(launch_cvalues(cb, s), "batch c-values");
     } else {
         if (split) cuda_check(cudaStreamWaitEvent(s, b.join_aux.e, 0), "event");

@@ -122,6 +122,8 @@ __device__ __forceinline__ uint4 plane8(const uint16_t *img, int pitch, int w, i
     return make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
 }
 
+// kStrips: every job has strips (a branch on them instead cost 12 of 267 us for 16 uneven pairs without any).
+template <bool kStrips>
 __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ Prep0Batch b)
 {
     if ((int)blockIdx.x >= b.total_tiles) {  // the blocks after the tiles clear the counters, a slot each
@@ -133,6 +135,7 @@ __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ P
             S.n = b.slot_n[i];
             S.k = b.slot_k[i];
             S.above_fx = S.above_n = 0;
+            if (i == 0 && b.clear) b.clear[0] = b.clear[1] = 0;
         }
         return;
     }
@@ -284,6 +287,22 @@ __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ P
     const uint32_t lo2 = (uint32_t)(b.need_lo & 0x7FFF) * 0x10001u;
     uint32_t dmin = 0xFFFFFFFFu;
     bool need = false;
+    // the strip, per half: the least masked value (unmasked words count as 0x8000 and more) and the greatest (with the mask
+    // bit; without it for none)
+    uint32_t smin = 0xFFFFFFFFu, smax = 0;
+    auto strip_word = [&](uint32_t word) {
+        smin = vmin_u16x2(smin, word ^ 0x80008000u);
+        smax = vmax_u16x2(smax, word);
+    };
+    // the warp's strip, from the halves of columns inside the picture
+    auto strip_out = [&](unsigned *to, bool in0, bool in1) {
+        const unsigned lo = min(in0 ? smin & 0xFFFFu : 0xFFFFu, in1 ? smin >> 16 : 0xFFFFu);
+        const unsigned hi = max(in0 ? smax & 0xFFFFu : 0u, in1 ? smax >> 16 : 0u);
+        const unsigned wlo = __reduce_min_sync(0xffffffffu, lo), whi = __reduce_max_sync(0xffffffffu, hi);
+        if (lane == 0) *to = wlo | (whi & 0x7FFFu) << 16;
+        smin = 0xFFFFFFFFu;
+        smax = 0;
+    };
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int y = yb + i;
@@ -294,6 +313,7 @@ __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ P
         const uint32_t mk = ((mb << 15) & 0x8000u) | ((mb << 30) & 0x80000000u);
         const uint32_t word2 = v2 | mk;
         if (y < h) {
+            if (kStrips) strip_word(word2);
             if (vec_store && x + 1 < w) {
                 *(uint32_t *)(J.word + (size_t)y * w + x) = word2;
             } else {
@@ -352,6 +372,7 @@ __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ P
         if (tid == 0) J.need[t] = need ? 1u : 0u;
     }
     if (!J.word1) return;  // the same for the whole block
+    if (kStrips) strip_out(J.strips + 8 * t + g, x < w, x + 1 < w);
 
     // the ring of scale-0 words one step outside the tile that scale 1 reads: rows y0-2 and y0+64 (X = 0 .. 33), then
     // columns x0-2 and x0+64 (Y = 1 .. 32)
@@ -400,6 +421,7 @@ __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ P
                 const uint32_t word = *(const uint32_t *)&dw[2 * q + i + 1][2 * p + 2];
                 const uint32_t v = (Y1 == 0 || Y1 == h1 - 1) ? word & 0x7FFF7FFFu : mode3x2(hm[i], hm[i + 1], hm[i + 2]);
                 const uint32_t out = v | (word & 0x80008000u);
+                if (kStrips) strip_word(out);
                 uint16_t *dst = J.word1 + (size_t)Y1 * w1 + X1;
                 if (vec1) {
                     *(uint32_t *)dst = out;
@@ -409,6 +431,7 @@ __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ P
                 }
             }
         }
+        if (kStrips) strip_out(J.strips + 8 * (J.tiles_x * ((h + kP0T - 1) / kP0T) + t) + warp, X1 < w1, X1 + 1 < w1);
     }
 }
 
@@ -749,7 +772,10 @@ cudaError_t launch_prep0(Prep0Batch &b, cudaStream_t s)
     b.need_lo = lo < 0 ? 0 : lo + b.band.band_base;
     b.need_span = !one_range ? -1 : lo < 0 ? -1 : hi - lo;
     LaunchTimer t("cambi_prep0", s);
-    prep0_kernel<<<b.total_tiles + b.nslots, 256, 0, s>>>(b);
+    bool strips = true;
+    for (int j = 0; j < b.njobs; j++) strips = strips && b.job[j].strips && b.job[j].word1;
+    if (strips) prep0_kernel<true><<<b.total_tiles + b.nslots, 256, 0, s>>>(b);
+    else prep0_kernel<false><<<b.total_tiles + b.nslots, 256, 0, s>>>(b);
     return after_launch();
 }
 
@@ -788,7 +814,7 @@ cudaError_t launch_score(const ScoreBatch &b, cudaStream_t s)
     return after_launch();
 }
 
-const void *kernel_entry_prep0() { return (const void *)prep0_kernel; }
+const void *kernel_entry_prep0() { return (const void *)prep0_kernel<false>; }
 const void *kernel_entry_decimate_mode() { return (const void *)decimate_mode_kernel; }
 
 }  // namespace es

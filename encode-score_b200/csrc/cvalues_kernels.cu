@@ -3,7 +3,8 @@
 //
 // One 256-thread block per tile of 64 columns by 64, 32 or 16 rows of any scale of any picture (a table of jobs):
 //  1. the tile's own pixels give the range of band codes (value - band_base of a masked pixel in the band) whose
-//     c-value is needed; tiles without one -- most tiles of most pictures -- leave after reading them;
+//     c-value is needed; tiles without one -- most tiles of most pictures -- leave after reading them. (A launch of many
+//     tiles has a kernel list the others first, and blocks that stay take tiles from the list);
 //  2. the tile and its window margins are staged as one byte per pixel (the code relative to that range), and every
 //     code seen sets a byte flag; the codes that can matter -- occurring within kDiffs of a code whose c-value is not
 //     trivially 0 -- are ranked in order. The plane holds ranks: as it is when the codes are consecutive, else through
@@ -117,6 +118,13 @@ __device__ __forceinline__ uint32_t min2(uint32_t a, uint32_t b)
     return r;
 }
 
+__device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b)
+{
+    uint32_t r;
+    asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+
 // The words of row y, pixels x .. x + 7 (x a multiple of 8), 0 (unmasked) outside the picture: one 16-byte load, or 4-
 // or 2-byte loads where the rows are not 16-byte aligned (align: 0, 1, 2).
 __device__ __forceinline__ uint4 load8(const CvJob &J, int align, int y, int x)
@@ -153,9 +161,18 @@ struct CvShared {
     unsigned next_tile;
 };
 
-// One tile, gt its global number; all threads return together. N: k-steps of the job's pad.
+// How a job's rows may be read: load8's align.
+__device__ __forceinline__ int row_align(const CvJob &J)
+{
+    return (J.w & 7) == 0 && (((uintptr_t)J.word) & 15) == 0 ? 0 : (J.w & 1) == 0 && (((uintptr_t)J.word) & 3) == 0 ? 1 : 2;
+}
+
+constexpr unsigned kNoRange = 0xFFFFFFFFu;  // a tile whose code range is not known
+
+// One tile, gt its global number; all threads return together. N: k-steps of the job's pad. known: a range of band codes
+// that holds the tile's needed ones, or kNoRange.
 template <int N>
-__device__ __forceinline__ void tile_cvalues(const CvBatch &b, const CvJob &J, const int gt, unsigned char *smem, CvShared &sh)
+__device__ __forceinline__ void tile_cvalues(const CvBatch &b, const CvJob &J, const int gt, const unsigned known, unsigned char *smem, CvShared &sh)
 {
     constexpr int kCols = cv_cols(N), kCstr = cv_cstr(N), kWords = kCols / 4, kVecs = kCols / 8;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -165,7 +182,7 @@ __device__ __forceinline__ void tile_cvalues(const CvBatch &b, const CvJob &J, c
     const int x0 = (tile % J.tiles_x) * kCvTX, y0 = (tile / J.tiles_x) * th;
     const int w = J.w, h = J.h, P = J.pad;
     const int rows = min(th, h - y0), cols = min(kCvTX, w - x0);
-    const int align = (w & 7) == 0 && (((uintptr_t)J.word) & 15) == 0 ? 0 : (w & 1) == 0 && (((uintptr_t)J.word) & 3) == 0 ? 1 : 2;
+    const int align = row_align(J);
     const CvLayout L = cv_layout(P);
     uint8_t *plane = smem + L.plane;           // [RH][kCols]: code or rank of pixel (xs + j, y0 - P + r)
     uint8_t *seen = smem + L.seen;             // byte flags: [0, 256) codes in the margins, [256, 512) in the tile itself
@@ -175,7 +192,7 @@ __device__ __forceinline__ void tile_cvalues(const CvBatch &b, const CvJob &J, c
     // 1. the range of needed codes among the tile's pixels
     unsigned mlo = 0xFFFFu, mhi = 0xFFFFu;
     const bool range = b.need_span >= 0;
-    {
+    if (known == kNoRange) {
         const uint32_t clo = (uint32_t)((0x10000 - 0x8000 - b.need_lo) & 0xFFFF) * 0x10001u;
         const uint32_t chi = (uint32_t)((0x8000 + b.need_lo + b.need_span + 1) & 0xFFFF) * 0x10001u;
         uint32_t lo2 = 0xFFFFFFFFu, hi2 = 0xFFFFFFFFu;
@@ -219,12 +236,12 @@ __device__ __forceinline__ void tile_cvalues(const CvBatch &b, const CvJob &J, c
         mlo = min(mlo, sh.redlo[k]);
         mhi = min(mhi, sh.redhi[k]);
     }
-    if (mlo == 0xFFFFu || (range && mlo > (unsigned)b.need_span)) {
+    if (known == kNoRange && (mlo == 0xFFFFu || (range && mlo > (unsigned)b.need_span))) {
         if (b.tile_mass && tid == 0) b.tile_mass[gt] = 0;
         return;
     }
-    const int own_lo = range ? b.need_lo + (int)mlo - bd.band_base : (int)mlo;
-    const int own_hi = range ? b.need_lo + b.need_span - (int)mhi - bd.band_base : 0xFFFE - (int)mhi;
+    const int own_lo = known != kNoRange ? (int)(known & 0xFFFFu) : range ? b.need_lo + (int)mlo - bd.band_base : (int)mlo;
+    const int own_hi = known != kNoRange ? (int)(known >> 16) : range ? b.need_lo + b.need_span - (int)mhi - bd.band_base : 0xFFFE - (int)mhi;
 
     const int RH = rows + 2 * P, xs = x0 - P - cv_ox(P), px = P + cv_ox(P);  // plane column of tile column 0
     const int rpw = th / kWarps;  // rows of a warp: 8, 4 or 2
@@ -623,20 +640,20 @@ __global__ void __launch_bounds__(kCvThreads, kMaxN == 3 ? 3 : 2) cvalues_kernel
         }
         __syncthreads();
     }
-    auto tile_body = [&](int gt) {
+    auto tile_body = [&](int gt, unsigned known) {
         const CvJob &J = b.job[find_job(b.njobs, gt, [&](int k) { return b.job[k].first_tile; })];
         if (b.run && !b.run[J.run_index]) return;
         const int n = cv_ksteps(J.pad);
-        if (n == 2) tile_cvalues<2>(b, J, gt, smem, sh);
-        else if (kMaxN == 3 || n == 3) tile_cvalues<3>(b, J, gt, smem, sh);
-        else if (kMaxN > 3 && n == 4) tile_cvalues<4>(b, J, gt, smem, sh);
-        else if (kMaxN > 3) tile_cvalues<5>(b, J, gt, smem, sh);
+        if (n == 2) tile_cvalues<2>(b, J, gt, known, smem, sh);
+        else if (kMaxN == 3 || n == 3) tile_cvalues<3>(b, J, gt, known, smem, sh);
+        else if (kMaxN > 3 && n == 4) tile_cvalues<4>(b, J, gt, known, smem, sh);
+        else if (kMaxN > 3) tile_cvalues<5>(b, J, gt, known, smem, sh);
     };
     // tiles are numbered by job, a picture's scales in order; they are taken from the last one on, because the small
     // scales' few tiles hold the most ranks (several passes): taken last, they were a tail in which most SMs idled
     // (a quarter of the launch on one 4K picture)
     if (!b.tiles) {
-        tile_body(b.total_tiles - 1 - (int)blockIdx.x);
+        tile_body(b.total_tiles - 1 - (int)blockIdx.x, kNoRange);
         return;
     }
     const unsigned count = *b.tile_count;
@@ -645,18 +662,85 @@ __global__ void __launch_bounds__(kCvThreads, kMaxN == 3 ? 3 : 2) cvalues_kernel
         __syncthreads();
         const unsigned i = sh.next_tile;
         if (i >= count) break;
-        tile_body((int)b.tiles[count - 1 - i]);
+        tile_body((int)b.tiles[count - 1 - i], b.tile_range ? b.tile_range[count - 1 - i] : kNoRange);
         __syncthreads();
     }
 }
 
+// The list of the tiles that can hold a needed code, each with a range of its codes: a warp per tile, from the strips of
+// scales 0 and 1 or the words of the others. (From the words of all scales it took 70 us for 16 uneven pairs, which have
+// 210 MB of them, now about 18; the strips add 19 us to the 269 of the kernel that makes the words.)
+__global__ void __launch_bounds__(kCvThreads) cv_list_kernel(const __grid_constant__ CvBatch b, unsigned *tiles, unsigned *ranges)
+{
+    __shared__ unsigned found[kWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int first = blockIdx.x * kWarps, gt = first + warp;
+    unsigned range = kNoRange;  // (no band code is 0xFFFF)
+    if (gt < b.total_tiles) {
+        const CvJob &J = b.job[find_job(b.njobs, gt, [&](int k) { return b.job[k].first_tile; })];
+        const int tile = gt - J.first_tile, th = J.tile_rows ? J.tile_rows : kCvTY;
+        const int x0 = (tile % J.tiles_x) * kCvTX, y0 = (tile / J.tiles_x) * th, rows = min(th, J.h - y0);
+        unsigned lo = 0xFFFFu, hi = 0;
+        if (J.strips) {
+            // 8 rows x 64 columns each (scale 0) or 4 x 32 (scale 1): at most 32, a lane each
+            const int sc = J.scale, col = (x0 >> (6 - sc)) + (lane & sc), r = (lane >> sc) * (8 >> sc), row = y0 + r;
+            const int bx = (J.w + (64 >> sc) - 1) >> (6 - sc);
+            if (r < rows && col < bx) {
+                const unsigned v = __ldg(J.strips + 8 * ((row >> (6 - sc)) * bx + col) + ((row >> (3 - sc)) & 7));
+                lo = v & 0xFFFFu;
+                hi = v >> 16;
+            }
+        } else {
+            const int align = row_align(J);
+            uint32_t lo2 = 0xFFFFFFFFu, hi2 = 0;  // as prep0_kernel's strips
+#pragma unroll 8
+            for (int i = lane; i < rows * (kCvTX / 8); i += 32) {
+                const uint4 q = load8(J, align, y0 + (i >> 3), x0 + 8 * (i & 7));
+                const uint32_t v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    lo2 = min2(lo2, v[k] ^ 0x80008000u);
+                    hi2 = max2(hi2, v[k]);
+                }
+            }
+            lo = min(lo2 & 0xFFFFu, lo2 >> 16);
+            hi = max(hi2 & 0xFFFFu, hi2 >> 16) & 0x7FFFu;
+        }
+        const int least = max((int)__reduce_min_sync(kFull, lo), b.need_first), greatest = min((int)__reduce_max_sync(kFull, hi), b.need_last);
+        if (least <= greatest) range = (unsigned)(least - b.band.band_base) | (unsigned)(greatest - b.band.band_base) << 16;
+        else if (b.tile_mass && lane == 0) b.tile_mass[gt] = 0;
+    }
+    if (lane == 0) found[warp] = range;
+    __syncthreads();
+    if (warp == 0) {
+        const unsigned r = lane < kWarps ? found[lane] : kNoRange, set = __ballot_sync(kFull, r != kNoRange);
+        unsigned at = 0;
+        if (lane == 0 && set) at = atomicAdd(b.busy, (unsigned)__popc(set));
+        at = __shfl_sync(kFull, at, 0) + __popc(set & ((1u << lane) - 1u));
+        if (r != kNoRange) {
+            tiles[at] = (unsigned)(first + lane);
+            ranges[at] = r;
+        }
+    }
+}
+
 template <int kMaxN>
-cudaError_t launch_cvalues_n(const CvBatch &b, cudaStream_t s)
+cudaError_t launch_cvalues_n(CvBatch &b, cudaStream_t s)
 {
     const size_t smem = cvalues_smem_bytes(b.max_pad);
-    const cudaError_t e = cudaFuncSetAttribute(cvalues_kernel<kMaxN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(cvalues_kernel<kMaxN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     LaunchTimer t("cambi_cvalues", s);
+    if (!b.tiles && b.busy) {
+        unsigned *tiles = b.busy + 2, *ranges = tiles + b.total_tiles;
+        cv_list_kernel<<<(b.total_tiles + kWarps - 1) / kWarps, kCvThreads, 0, s>>>(b, tiles, ranges);
+        e = after_launch();
+        if (e != cudaSuccess) return e;
+        b.tiles = tiles;
+        b.tile_range = ranges;
+        b.tile_count = b.busy;
+        b.tile_next = b.busy + 1;
+    }
     const int grid = b.tiles && b.total_tiles > kCvListBlocks ? kCvListBlocks : b.total_tiles;
     cvalues_kernel<kMaxN><<<grid, kCvThreads, smem, s>>>(b);
     return after_launch();
@@ -685,6 +769,8 @@ cudaError_t launch_cvalues(const CvBatch &batch, cudaStream_t s)
     }
     b.need_lo = lo < 0 ? 0 : lo + b.band.band_base;
     b.need_span = !one_range ? -1 : lo < 0 ? -1 : hi - lo;
+    b.need_first = lo < 0 ? 1 : lo + b.band.band_base;
+    b.need_last = lo < 0 ? 0 : hi + b.band.band_base;
     int n = 2;
     for (int j = 0; j < b.njobs; j++) n = n > cv_ksteps(b.job[j].pad) ? n : cv_ksteps(b.job[j].pad);
     return n <= 3 ? launch_cvalues_n<3>(b, s) : launch_cvalues_n<5>(b, s);

@@ -105,7 +105,13 @@ struct Prep0Job {
     // optional: scale 1 (w1 x h1 = the halved size, rounded up) made in the same pass; nullptr: scale 0 only
     uint16_t *word1;
     int w1, h1;
+    // optional, with word1: strips[8 t + g], t a 64 x 64 tile of scale 0: the least and (<< 16) the greatest masked value of
+    // rows 8 g .. 8 g + 7 of the tile, a least above the greatest where there is none. After all tiles, the same for 4 rows
+    // of each tile's 32 x 32 words of scale 1.
+    unsigned *strips;
 };
+// Words of a w x h picture's strips, both scales.
+inline size_t prep0_strips(int w, int h) { return (size_t)((w + 63) / 64) * ((h + 63) / 64) * 16; }
 constexpr int kPrep0MaxJobs = kMaxPictures;
 struct Prep0Batch {
     Prep0Job job[kPrep0MaxJobs];
@@ -117,6 +123,7 @@ struct Prep0Batch {
     CvSlot *slots;
     int nslots;
     const unsigned long long *slot_n, *slot_k;
+    unsigned *clear;  // optional, with slots: two words set to 0
 };
 cudaError_t launch_prep0(Prep0Batch &b, cudaStream_t s);
 
@@ -144,6 +151,8 @@ struct CvJob {
     float *plane;   // optional: every computed c-value at its pixel
     int run_index;  // the entry of CvBatch::run that gates this job (with a run table)
     int tile_rows;  // rows of this job's tiles: 64 (0 means 64), 32 or 16; tiles are numbered row by row
+    int scale;      // with strips: 0 or 1
+    const unsigned *strips;  // optional, scales 0 and 1, for the busy tiles' list: this scale's part of Prep0Job::strips
 };
 struct CvBatch {
     CvJob job[kMaxJobs];
@@ -156,12 +165,23 @@ struct CvBatch {
     const unsigned *tiles;
     const unsigned *tile_count;
     unsigned *tile_next;
+    const unsigned *tile_range;  // optional, by list entry: a range of band codes, least | greatest << 16, that holds the tile's
+                                 // needed ones
+    // Optional, without a list: 2 + 2 total_tiles words, the first two 0 at launch (Prep0Batch::clear). A kernel of its own
+    // then first lists the tiles that can hold needed codes.
+    unsigned *busy;
     // Optional: per global tile, the exact sum of its positive c-values in 2^-24 units (0 for a tile with none).
     unsigned long long *tile_mass;
     // Optional: run[job.run_index] == 0 skips the job's tiles.
     const int *run;
-    int need_lo, need_span;  // set by the launcher: as Prep0Batch's
+    int need_lo, need_span;      // set by the launcher: as Prep0Batch's
+    int need_first, need_last;   // set by the launcher: the least and greatest needed value
 };
+// A launch of at least this many tiles lists its busy tiles first (CvBatch::busy). Most tiles of most pictures need no
+// c-value, but a block of their own costs 2 to 4 us of a place on an SM to find that out: 16 uneven pairs (26.6 thousand
+// tiles) took 706 us and take 588, a step of a 3840 x 2160 pair (5.5 thousand) 388 and 375; below, the launch more costs what it
+// saves: a step of a 1920 x 1080 pair (2.3 thousand) 170 and 173.
+constexpr int kCvBusyTiles = 4096;
 // Blocks of a tile-list launch.
 constexpr int kCvListBlocks = 148 * 3;
 constexpr int kCvTX = 64, kCvTY = 64, kCvThreads = 256, kCvBins = 32;

@@ -227,3 +227,33 @@ def test_host_frames_in_three_slots_equal_the_device_run(cuda, module, steps):
             assert results[f][k:k + n] == dev[s][0][f], (f, s)
             k += n
     assert [accum_bytes(x) for x in accs] == [accum_bytes(x) for x in dacc]
+
+
+@pytest.mark.parametrize("depth", [8, 10])
+def test_large_batch_of_listed_tiles_equals_frames_of_their_own(cuda, module, depth):
+    """A step of over 4096 c-value tiles lists the tiles that can hold banding from what the words' kernel noted of each
+    strip; a source of its own has every tile searched. Sizes one strip, one tile and an odd half past a boundary."""
+    sizes = [(254, 190), (258, 194), (256, 192), (322, 130), (318, 142), (382, 158), (390, 202), (446, 136)] * 4
+    stream = cuda.cuda.current_stream().cuda_stream
+    steps = [[es_synth.c3_step(f, s, w, h, depth) for s, (w, h) in enumerate(sizes)] for f in range(2)]
+    b = es_b200.Batch(module, [(w, h, depth, 1) for w, h in sizes], tuning=False)
+    got = []
+    for f in range(2):
+        keep, views = [], []
+        for s in range(len(sizes)):
+            k, sv, ev = step_to_dev(cuda, es_b200, steps[f][s])
+            keep.append(k)
+            views += [sv] + ev
+        b.queue(f, views, stream)
+        got.append([(r.cambi, r.cambi_source) for r in b.collect(f)])
+    b.close()
+    for s, (w, h) in enumerate(sizes):
+        fr = es_b200.Frame(module, w, h, depth, 1)
+        for f in range(2):
+            keep, sv, ev = step_to_dev(cuda, es_b200, steps[f][s])
+            fr.queue(f, sv, ev, stream)
+            acc = [es_b200.new_accum()]
+            r = fr.collect(f, acc, acc)[0]
+            assert (r.cambi, r.cambi_source) == got[f][s], (s, f)
+        fr.close()
+    assert max(max(c) for c in got[0]) > 0 and min(min(c) for c in got[0]) == 0
