@@ -308,7 +308,7 @@ struct PairSumsJob {
     unsigned long long *sse;       // [nenc][3]
     unsigned long long *color;     // [nenc + 1][3]: sum U, sum V, strength in 2^-30 units; source last
     int nenc, w, h, up;
-    int first_pic;  // set by the launcher: this job's pictures are grid rows first_pic .. first_pic + nenc
+    int first_block;  // set by the launcher
 };
 struct PairSumsBatch {
     PairSumsJob job[kMaxSources];
