@@ -85,11 +85,9 @@ struct CvSlot {
     float *list;                       // c-values, zeros among them (capacity n): every positive one is there once
     unsigned pad_[2];
     alignas(16) unsigned hist[2048];   // counts of the first radix digit
-    // counts of the second and the last digit, and the sums (2^-24 units) of the values of each last digit: clear between
-    // launches (the score kernel clears what a selection used)
+    // counts of the second and the last digit: clear between launches (the score kernel clears what a selection used)
     alignas(16) unsigned hist1[2048];
     alignas(16) unsigned hist2[1024];
-    alignas(16) unsigned long long dsum[1024];
 };
 
 // ---- scales 0 and 1: preprocessing, zero-derivative mask and mode filter of one plane, then its first decimation --

@@ -81,10 +81,7 @@ __global__ void noalloc_setup_kernel(CvSlot *slots, float *lut, const __grid_con
     }
     CvSlot &S = slots[blockIdx.x];
     for (int i = threadIdx.x; i < 2048; i += blockDim.x) S.hist[i] = S.hist1[i] = 0;
-    for (int i = threadIdx.x; i < 1024; i += blockDim.x) {
-        S.hist2[i] = 0;
-        S.dsum[i] = 0;
-    }
+    for (int i = threadIdx.x; i < 1024; i += blockDim.x) S.hist2[i] = 0;
     if (threadIdx.x == 0) {
         S.sum_fx = S.count = S.list_n = 0;
         S.n = st.n[blockIdx.x];
