@@ -473,7 +473,7 @@ void record_cambi(es_batch &b, long f, uint32_t skip, cudaStream_t s)
         if (split) cuda_check(cudaStreamWaitEvent(s, b.join_aux.e, 0), "event");
         record_proposal_cvalues(b, cb, ab, s);
     }
-    cuda_check(launch_topk(b.slots.ptr, nslots, s), "batch top-k");
+    cuda_check(launch_topk(b.slots.ptr, nslots, s, false), "batch top-k");
     ScoreBatch sb{};
     for (int i : run) {
         ScoreJob &j = sb.job[sb.njobs++];

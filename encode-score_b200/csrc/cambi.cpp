@@ -143,10 +143,12 @@ void queue_cambi(es_cambi *c, uint64_t img, int pitch, cudaStream_t caller)
     {
         static_assert(sizeof(CvSlot) % 8 == 0, "slot layout");
     }
+    cb.chained = 1;
     cuda_check(launch_cvalues(cb, s), "cambi c-values");
-    cuda_check(launch_topk(c->slots.ptr, kScales, s), "cambi top-k");
+    cuda_check(launch_topk(c->slots.ptr, kScales, s, true), "cambi top-k");
     ScoreBatch sb{};
     sb.njobs = 1;
+    sb.chained = 1;
     sb.job[0].first_slot = 0;
     sb.job[0].window = p.window;
     sb.job[0].score = c->score.ptr;

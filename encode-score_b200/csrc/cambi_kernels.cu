@@ -126,6 +126,7 @@ __device__ __forceinline__ uint4 plane8(const uint16_t *img, int pitch, int w, i
 template <bool kStrips>
 __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ Prep0Batch b)
 {
+    if (b.chained) let_next_start();
     if ((int)blockIdx.x >= b.total_tiles) {  // the blocks after the tiles clear the counters, a slot each
         const int i = blockIdx.x - b.total_tiles;
         CvSlot &S = b.slots[i];
@@ -471,6 +472,8 @@ __device__ __forceinline__ void mode_column(const uint16_t *d, int stride, int x
 
 __global__ void __launch_bounds__(256) decimate_mode_kernel(const __grid_constant__ DecBatch b)
 {
+    wait_for_previous();
+    let_next_start();
     __shared__ uint16_t d2[kD2H][kD2W], f2[kF2H][kF2W], d3[kF3H + 2][kF3W + 2], f3[kF3H][kF3W], d4[kDTH / 4 + 2][kDTW / 4 + 2];
     const int j = find_job(b.njobs, (int)blockIdx.x, [&](int k) { return b.job[k].first_block; });
     const DecJob &J = b.job[j];
@@ -586,6 +589,8 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(CvSlot *slots, int 
     __shared__ unsigned long long groups[kMaxJobs];  // of 4 values, in the slot's list
     __shared__ int warp_n[kSelThreads / 32];
     static_assert(kMaxJobs <= kSelThreads, "a thread per slot");
+    wait_for_previous();
+    let_next_start();
     const int tid = threadIdx.x;
     const bool mine = tid < nslots && slots[tid].count > slots[tid].k;
     if (!__syncthreads_or(mine)) return;
@@ -686,6 +691,7 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(CvSlot *slots, int 
 __global__ void __launch_bounds__(32 * kScales) score_kernel(const __grid_constant__ ScoreBatch b)
 {
     __shared__ double part[kScales];
+    wait_for_previous();
     const ScoreJob &J = b.job[blockIdx.x];
     const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
     CvSlot &S = b.slots[J.first_slot + s];
@@ -794,30 +800,26 @@ cudaError_t launch_decimate_mode(DecBatch &b, cudaStream_t s)
     }
     if (blocks <= 0) return cudaSuccess;
     LaunchTimer t("cambi_decimate_mode", s);
-    decimate_mode_kernel<<<blocks, 256, 0, s>>>(b);
-    return after_launch();
+    return launch_kernel(b.chained, decimate_mode_kernel, dim3(blocks), 256, 0, s, b);
 }
 
-cudaError_t launch_topk(CvSlot *slots, int nslots, cudaStream_t s)
+cudaError_t launch_topk(CvSlot *slots, int nslots, cudaStream_t s, bool chained)
 {
     if (nslots <= 0) return cudaSuccess;
     {
         LaunchTimer t("cambi_select", s);
-        select_kernel<1><<<kSelBlocks, kSelThreads, 0, s>>>(slots, nslots);
+        const cudaError_t e = launch_kernel(chained, select_kernel<1>, dim3(kSelBlocks), kSelThreads, 0, s, slots, nslots);
+        if (e != cudaSuccess) return e;
     }
-    const cudaError_t e = after_launch();
-    if (e != cudaSuccess) return e;
     LaunchTimer t("cambi_select", s);
-    select_kernel<2><<<kSelBlocks, kSelThreads, 0, s>>>(slots, nslots);
-    return after_launch();
+    return launch_kernel(chained, select_kernel<2>, dim3(kSelBlocks), kSelThreads, 0, s, slots, nslots);
 }
 
 cudaError_t launch_score(const ScoreBatch &b, cudaStream_t s)
 {
     if (b.njobs <= 0) return cudaSuccess;
     LaunchTimer t("cambi_score", s);
-    score_kernel<<<b.njobs, 32 * kScales, 0, s>>>(b);
-    return after_launch();
+    return launch_kernel(b.chained, score_kernel, dim3(b.njobs), 32 * kScales, 0, s, b);
 }
 
 const void *kernel_entry_prep0() { return (const void *)prep0_kernel<false>; }

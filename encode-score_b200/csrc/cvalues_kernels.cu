@@ -631,6 +631,7 @@ __global__ void __launch_bounds__(kCvThreads, kMaxN == 3 ? 3 : 2) cvalues_kernel
 {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ CvShared sh;
+    wait_for_previous();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (b.need_span < 0) {  // the codes whose c-value is needed, when they are no single range
         for (int word = warp; word < 32; word += kWarps) {
@@ -742,8 +743,7 @@ cudaError_t launch_cvalues_n(CvBatch &b, cudaStream_t s)
         b.tile_next = b.busy + 1;
     }
     const int grid = b.tiles && b.total_tiles > kCvListBlocks ? kCvListBlocks : b.total_tiles;
-    cvalues_kernel<kMaxN><<<grid, kCvThreads, smem, s>>>(b);
-    return after_launch();
+    return launch_kernel(b.chained, cvalues_kernel<kMaxN>, dim3(grid), kCvThreads, smem, s, b);
 }
 }  // namespace
 

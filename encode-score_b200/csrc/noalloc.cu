@@ -148,6 +148,7 @@ extern "C" int es_cambi_score_noalloc(uint64_t img, int pitch, int w, int h, int
         pj.word1 = (uint16_t *)(base + c.words[1]);
         pj.w1 = c.sw[1];
         pj.h1 = c.sh[1];
+        pb.chained = 1;
         cuda_check(launch_prep0(pb, s), "cambi scales 0 and 1");
         DecBatch db{};
         db.njobs = 1;
@@ -158,6 +159,7 @@ extern "C" int es_cambi_score_noalloc(uint64_t img, int pitch, int w, int h, int
             db.job[0].w[k - 2] = c.sw[k];
             db.job[0].h[k - 2] = c.sh[k];
         }
+        db.chained = 1;
         cuda_check(launch_decimate_mode(db, s), "cambi scales");
         CvBatch cb{};
         cb.njobs = kScales;
@@ -181,10 +183,12 @@ extern "C" int es_cambi_score_noalloc(uint64_t img, int pitch, int w, int h, int
                        {p.weight[0], p.weight[1], p.weight[2], p.weight[3]}};
         cb.lut = (const float *)(base + c.lut);
         cb.slots = slots;
+        cb.chained = 1;
         cuda_check(launch_cvalues(cb, s), "cambi c-values");
-        cuda_check(launch_topk(slots, kScales, s), "cambi top-k");
+        cuda_check(launch_topk(slots, kScales, s, true), "cambi top-k");
         ScoreBatch sb{};
         sb.njobs = 1;
+        sb.chained = 1;
         sb.job[0].first_slot = 0;
         sb.job[0].window = p.window;
         sb.job[0].score = rec;

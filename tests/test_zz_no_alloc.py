@@ -109,3 +109,26 @@ def test_no_alloc_in_a_created_context_matches_the_primary_one(cuda, module):
         ok(cu.cuCtxDestroy_v2(ctx), "cuCtxDestroy")  # pops it: the primary context is current again
     assert got == [want, want]
     assert primary_score() == want
+
+
+def test_no_alloc_in_a_captured_graph_matches_the_direct_call(cuda, module):
+    """The chain's launches overlap the kernels before them; captured, the graph's edges have to keep that order."""
+    torch = cuda
+    pictures = [banded(640, 360, 33 + k, lo=80, hi=200, step=2 + k) for k in range(2)]
+    h, w = pictures[0].shape
+    want = [allocating_score(torch, module, img, 10) for img in pictures]
+    plane = to_dev(torch, pictures[0])
+    out = torch.zeros(1, dtype=torch.float64, device="cuda")
+    stream = torch.cuda.Stream()
+    es_b200.cambi_score_noalloc(plane.data_ptr(), w, w, h, 10, out.data_ptr(), stream.cuda_stream)
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        es_b200.cambi_score_noalloc(plane.data_ptr(), w, w, h, 10, out.data_ptr(), stream.cuda_stream)
+    got = []
+    for img in pictures * 2:
+        plane.copy_(to_dev(torch, img))
+        graph.replay()
+        torch.cuda.synchronize()
+        got.append(float(from_dev(out, np.float64)[0]))
+    assert got == want * 2 and want[0] != want[1]
