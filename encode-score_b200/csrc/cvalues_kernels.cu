@@ -23,8 +23,9 @@
 // What bounds it: instruction issue and, on pictures with few busy tiles, one block's latency. The block-wide form this
 // replaces (two block barriers per row, every warp stepping through every row) issued 130 thousand warp instructions per
 // busy 4K tile, this one 60 thousand; three blocks per SM (80 registers) against two (128): 245 against 270 us on the
-// dense 4K picture. C-values of one picture, before / now: 3840x2160 10-bit dense 520 / 245 us, the same size bright with
-// steps of 8 codes 557 / 107 us, 1920x1080 8-bit 176 / 57 us, 640x360 8-bit 90 / 24 us.
+// dense 4K picture. C-values of one picture, before / now: 3840x2160 10-bit dense 520 / 225 us, the same size bright with
+// steps of 8 codes 557 / 105 us, 1920x1080 8-bit 176 / 55 us, 640x360 8-bit 90 / 24 us. (Of the 225, 23 fewer since the
+// counts move by atomics without a result and the four differences are computed without branches.)
 #include "cambi_codes.h"
 #include "es_kernels.h"
 
@@ -417,9 +418,15 @@ __device__ __forceinline__ void tile_cvalues(const CvBatch &b, const CvJob &J, c
                 const int row = kk + (int)nib - kDiffs;
                 ((uint16_t *)(smem + L.tab))[tid] = (nib == 15u || row < 0 || row >= kCvBins) ? 0 : (uint16_t)cv_row(row + 1);
             }
+            // a count on or off, as an addition to the word of its four columns (a lane's own): no byte ends below 0 or
+            // above 255, so the carries between the bytes cancel. An atomic without a result is one instruction that
+            // nothing waits for, where the byte's load, addition and store made a chain of eight per word.
+            const uint32_t cw_at = (uint32_t)__cvta_generic_to_shared(cw);
             auto count_rank = [&](uint32_t word, int wi, int e, int delta) {
                 const unsigned k = ((word >> (8 * e)) & 0xFFu) - off;
-                if (k < (unsigned)npos) cw[k * kCstr + 4 * wi + e] += (uint8_t)delta;
+                asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.u32 p, %0, %1;\n\t@p red.shared.add.u32 [%2], %3;\n\t}\n" ::"r"(k), "r"(npos),
+                             "r"(cw_at + k * kCstr + 4 * wi), "r"((unsigned)delta << (8 * e))
+                             : "memory");
             };
             // moves counts on from tile row r to r + 1: region row r leaves, r + 2 P + 1 enters
             auto slide = [&](int r) {
@@ -560,10 +567,10 @@ __device__ __forceinline__ void tile_cvalues(const CvBatch &b, const CvJob &J, c
                                     const unsigned p1 = lds_u16((up[d >> 1] >> (16 * (d & 1))) & 0xFFFFu);
                                     const unsigned p2 = lds_u16((dn[d >> 1] >> (16 * (d & 1))) & 0xFFFFu);
                                     const unsigned pm = p1 > p2 ? p1 : p2;
-                                    if (pm) {  // a diff with no neighbour gives 0, which never raises the c-value
-                                        const float val = __fmul_rn(__uint2float_rn((unsigned)bd.weight[d] * p0 * pm), __ldg(b.lut + p0 + pm));
-                                        if (val > cval) cval = val;
-                                    }
+                                    // (a diff with no neighbour gives 0; without a branch around it the four loads of
+                                    // the table are in flight together)
+                                    const float val = __fmul_rn(__uint2float_rn((unsigned)bd.weight[d] * p0 * pm), __ldg(b.lut + p0 + pm));
+                                    cval = fmaxf(cval, val);
                                 }
                                 if (J.plane) J.plane[(size_t)(y0 + r) * w + x0 + lane + 32 * half] = cval;
                             }
