@@ -415,6 +415,7 @@ void record_cambi(es_batch &b, long f, uint32_t skip, cudaStream_t s)
     pb.slot_n = b.slot_n.ptr;
     pb.slot_k = b.slot_k.ptr;
     pb.clear = busy ? b.busy.ptr : nullptr;
+    pb.chained = 1;
     cuda_check(launch_prep0(pb, s), "batch scales 0 and 1");
     CvBatch cb{};
     int tiles = 0;
@@ -465,9 +466,11 @@ void record_cambi(es_batch &b, long f, uint32_t skip, cudaStream_t s)
             dj.h[sc - 2] = pic.sh[sc];
         }
     }
+    db.chained = !b.net;
     cuda_check(launch_decimate_mode(db, s), "batch scales");
     if (!b.net) {
         if (busy) cb.busy = b.busy.ptr;
+        cb.chained = 1;
         cuda_check(launch_cvalues(cb, s), "batch c-values");
     } else {
         if (split) cuda_check(cudaStreamWaitEvent(s, b.join_aux.e, 0), "event");

@@ -110,6 +110,7 @@ void queue_cambi(es_cambi *c, uint64_t img, int pitch, cudaStream_t caller)
         dj.w[sc - 2] = c->sw[sc];
         dj.h[sc - 2] = c->sh[sc];
     }
+    db.early = 1;
     cuda_check(launch_decimate_mode(db, s), "cambi scales");
     CvBatch cb{};
     cb.njobs = kScales;
@@ -148,7 +149,6 @@ void queue_cambi(es_cambi *c, uint64_t img, int pitch, cudaStream_t caller)
     cuda_check(launch_topk(c->slots.ptr, kScales, s, true), "cambi top-k");
     ScoreBatch sb{};
     sb.njobs = 1;
-    sb.chained = 1;
     sb.job[0].first_slot = 0;
     sb.job[0].window = p.window;
     sb.job[0].score = c->score.ptr;

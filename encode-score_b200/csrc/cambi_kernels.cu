@@ -126,7 +126,7 @@ __device__ __forceinline__ uint4 plane8(const uint16_t *img, int pitch, int w, i
 template <bool kStrips>
 __global__ void __launch_bounds__(256, 5) prep0_kernel(const __grid_constant__ Prep0Batch b)
 {
-    if (b.chained) let_next_start();
+    wait_for_previous();
     if ((int)blockIdx.x >= b.total_tiles) {  // the blocks after the tiles clear the counters, a slot each
         const int i = blockIdx.x - b.total_tiles;
         CvSlot &S = b.slots[i];
@@ -473,7 +473,7 @@ __device__ __forceinline__ void mode_column(const uint16_t *d, int stride, int x
 __global__ void __launch_bounds__(256) decimate_mode_kernel(const __grid_constant__ DecBatch b)
 {
     wait_for_previous();
-    let_next_start();
+    if (b.early) let_next_start();
     __shared__ uint16_t d2[kD2H][kD2W], f2[kF2H][kF2W], d3[kF3H + 2][kF3W + 2], f3[kF3H][kF3W], d4[kDTH / 4 + 2][kDTW / 4 + 2];
     const int j = find_job(b.njobs, (int)blockIdx.x, [&](int k) { return b.job[k].first_block; });
     const DecJob &J = b.job[j];
@@ -578,7 +578,7 @@ __device__ Picked pick_digit(const unsigned *hist, unsigned long long remaining,
 // instructions than one atomic per matching value) a round took 29 us for a dense 3840 x 2160 picture and for four of them
 // with fewer values; now 19 us.
 template <int kRound>
-__global__ void __launch_bounds__(kSelThreads) select_kernel(CvSlot *slots, int nslots)
+__global__ void __launch_bounds__(kSelThreads) select_kernel(CvSlot *slots, int nslots, bool early)
 {
     constexpr bool last = kRound == 2;
     constexpr int shift = last ? 0 : 10, nb = last ? 1024 : 2048;
@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(kSelThreads) select_kernel(CvSlot *slots, int 
     __shared__ int warp_n[kSelThreads / 32];
     static_assert(kMaxJobs <= kSelThreads, "a thread per slot");
     wait_for_previous();
-    let_next_start();
+    if (early) let_next_start();
     const int tid = threadIdx.x;
     const bool mine = tid < nslots && slots[tid].count > slots[tid].k;
     if (!__syncthreads_or(mine)) return;
@@ -786,9 +786,7 @@ cudaError_t launch_prep0(Prep0Batch &b, cudaStream_t s)
     LaunchTimer t("cambi_prep0", s);
     bool strips = true;
     for (int j = 0; j < b.njobs; j++) strips = strips && b.job[j].strips && b.job[j].word1;
-    if (strips) prep0_kernel<true><<<b.total_tiles + b.nslots, 256, 0, s>>>(b);
-    else prep0_kernel<false><<<b.total_tiles + b.nslots, 256, 0, s>>>(b);
-    return after_launch();
+    return launch_kernel(b.chained, strips ? prep0_kernel<true> : prep0_kernel<false>, dim3(b.total_tiles + b.nslots), 256, 0, s, b);
 }
 
 cudaError_t launch_decimate_mode(DecBatch &b, cudaStream_t s)
@@ -803,23 +801,23 @@ cudaError_t launch_decimate_mode(DecBatch &b, cudaStream_t s)
     return launch_kernel(b.chained, decimate_mode_kernel, dim3(blocks), 256, 0, s, b);
 }
 
-cudaError_t launch_topk(CvSlot *slots, int nslots, cudaStream_t s, bool chained)
+cudaError_t launch_topk(CvSlot *slots, int nslots, cudaStream_t s, bool early)
 {
     if (nslots <= 0) return cudaSuccess;
     {
         LaunchTimer t("cambi_select", s);
-        const cudaError_t e = launch_kernel(chained, select_kernel<1>, dim3(kSelBlocks), kSelThreads, 0, s, slots, nslots);
+        const cudaError_t e = launch_kernel(true, select_kernel<1>, dim3(kSelBlocks), kSelThreads, 0, s, slots, nslots, early);
         if (e != cudaSuccess) return e;
     }
     LaunchTimer t("cambi_select", s);
-    return launch_kernel(chained, select_kernel<2>, dim3(kSelBlocks), kSelThreads, 0, s, slots, nslots);
+    return launch_kernel(true, select_kernel<2>, dim3(kSelBlocks), kSelThreads, 0, s, slots, nslots, early);
 }
 
 cudaError_t launch_score(const ScoreBatch &b, cudaStream_t s)
 {
     if (b.njobs <= 0) return cudaSuccess;
     LaunchTimer t("cambi_score", s);
-    return launch_kernel(b.chained, score_kernel, dim3(b.njobs), 32 * kScales, 0, s, b);
+    return launch_kernel(true, score_kernel, dim3(b.njobs), 32 * kScales, 0, s, b);
 }
 
 const void *kernel_entry_prep0() { return (const void *)prep0_kernel<false>; }

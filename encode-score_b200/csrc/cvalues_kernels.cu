@@ -681,6 +681,7 @@ __global__ void __launch_bounds__(kCvThreads, kMaxN == 3 ? 3 : 2) cvalues_kernel
 __global__ void __launch_bounds__(kCvThreads) cv_list_kernel(const __grid_constant__ CvBatch b, unsigned *tiles, unsigned *ranges)
 {
     __shared__ unsigned found[kWarps];
+    wait_for_previous();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int first = blockIdx.x * kWarps, gt = first + warp;
     unsigned range = kNoRange;  // (no band code is 0xFFFF)
@@ -741,13 +742,13 @@ cudaError_t launch_cvalues_n(CvBatch &b, cudaStream_t s)
     LaunchTimer t("cambi_cvalues", s);
     if (!b.tiles && b.busy) {
         unsigned *tiles = b.busy + 2, *ranges = tiles + b.total_tiles;
-        cv_list_kernel<<<(b.total_tiles + kWarps - 1) / kWarps, kCvThreads, 0, s>>>(b, tiles, ranges);
-        e = after_launch();
+        e = launch_kernel(b.chained, cv_list_kernel, dim3((b.total_tiles + kWarps - 1) / kWarps), kCvThreads, 0, s, b, tiles, ranges);
         if (e != cudaSuccess) return e;
         b.tiles = tiles;
         b.tile_range = ranges;
         b.tile_count = b.busy;
         b.tile_next = b.busy + 1;
+        b.chained = 1;
     }
     const int grid = b.tiles && b.total_tiles > kCvListBlocks ? kCvListBlocks : b.total_tiles;
     return launch_kernel(b.chained, cvalues_kernel<kMaxN>, dim3(grid), kCvThreads, smem, s, b);

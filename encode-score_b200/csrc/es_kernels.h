@@ -47,12 +47,10 @@ constexpr int kMaxJobs = kMaxPictures * 5;  // pictures x scales in one c-value 
 constexpr int kWin = 16;               // detail window side (src/kernels.cu:331)
 
 #ifdef __CUDACC__
-// A launch that may begin while the kernel before it on the stream ends (programmatic dependent launch): `kernel` calls
-// wait_for_previous() before it reads or writes memory, and what comes before the launch on the stream is a kernel. The
-// blocks' start and the launch's latency, 1 to 2 us, then lie beside the kernel before. Only a chain with the GPU to itself
-// is launched so, CAMBI of one picture (640x360 77 -> 68 us, 1920x1080 121 -> 112): beside another chain, the waiting
-// blocks hold places that it could use (a step of a 1920 x 800 pair in one batch 161 -> 171 us, of a 3840 x 2160 one
-// 372 -> 378).
+// A launch that is made ready while the kernel before it on the stream runs, and begins when that kernel's last block leaves
+// (programmatic dependent launch): `kernel` calls wait_for_previous() before it reads or writes memory, and what comes
+// before the launch on the stream is a kernel. CAMBI of one 640x360 picture 77 -> 68 us, of 1920x1080 121 -> 112; a step of
+// a 1920x1080 pair, whose kernels are launched one by one, 160 -> 152 us.
 // chained = false: a plain launch.
 template <typename... P, typename... A>
 cudaError_t launch_kernel(bool chained, void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, const A &...args)
@@ -73,7 +71,10 @@ cudaError_t launch_kernel(bool chained, void (*kernel)(P...), dim3 grid, int thr
 }
 // Until the kernels this one was launched to follow are complete and their writes visible (at once in a plain launch).
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-// Once every block of this kernel has said so or left, the next kernel's blocks may take free places and wait there.
+
+// Once every block of this kernel has said so or left, the next kernel's blocks may take free places and wait there: 1 us
+// more for CAMBI of one picture. Only where a chain has the GPU to itself: beside another chain, the waiting blocks hold
+// places that it could use (a step of a 1920 x 800 pair 161 -> 171 us).
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::); }
 
 // The job whose range of blocks or tiles holds t: the last job j with first(j) <= t, by binary search over a job
@@ -151,7 +152,7 @@ struct Prep0Batch {
     int nslots;
     const unsigned long long *slot_n, *slot_k;
     unsigned *clear;  // optional, with slots: two words set to 0
-    int chained;      // launch_decimate_mode follows at once on the same stream, chained
+    int chained;      // what comes before on the stream is the kernel that makes the planes (launch_kernel)
 };
 cudaError_t launch_prep0(Prep0Batch &b, cudaStream_t s);
 
@@ -168,6 +169,7 @@ struct DecBatch {
     DecJob job[kDecMaxJobs];
     int njobs;
     int chained;  // what comes before on the stream is the kernel of scales 0 and 1
+    int early;    // let the next kernel start early (let_next_start)
 };
 cudaError_t launch_decimate_mode(DecBatch &b, cudaStream_t s);
 
@@ -237,8 +239,8 @@ cudaError_t launch_cvalues(const CvBatch &b, cudaStream_t s);
 // exceeds k, after the c-value launches (which leave the first digit's counts in each slot): radix rounds of 11, 11 and
 // 10 bits, the second and third over the slots' lists, the last one also summing what lies above the selected value. The
 // score kernel makes the last pick.
-// chained: what comes before on the stream is the c-value kernel (launch_kernel).
-cudaError_t launch_topk(CvSlot *slots, int nslots, cudaStream_t s, bool chained);
+// Follows the c-value kernel on the stream (launch_kernel). early: let_next_start.
+cudaError_t launch_topk(CvSlot *slots, int nslots, cudaStream_t s, bool early);
 struct ScoreJob {
     int first_slot;  // kScales consecutive slots
     int window;
@@ -249,9 +251,9 @@ constexpr int kScoreMaxJobs = kMaxPictures;
 struct ScoreBatch {
     ScoreJob job[kScoreMaxJobs];
     int njobs;
-    int chained;  // what comes before on the stream is the last top-k round
     CvSlot *slots;
 };
+// Follows the last top-k round on the stream.
 cudaError_t launch_score(const ScoreBatch &b, cudaStream_t s);
 
 // ---- frame unpacking ---------------------------------------------------------------------------------------------
@@ -311,6 +313,7 @@ struct WindowBatch {
     WindowJob job[kMaxSources];
     int njobs;
 };
+// Follows the squared errors on the stream (launch_kernel).
 cudaError_t launch_window_stats(WindowBatch &b, cudaStream_t s);
 
 // ---- lasting texture ------------------------------------------------------------------------------------------------
@@ -331,6 +334,7 @@ struct PersistBatch {
     PersistJob job[kMaxSources];
     int njobs;
 };
+// Follows the window figures on the stream (launch_kernel).
 cudaError_t launch_persist(PersistBatch &b, cudaStream_t s);
 
 // ---- PSNR squared errors and color sums --------------------------------------------------------------------------

@@ -421,6 +421,7 @@ __global__ void __launch_bounds__(kWThreads, 4) window_stats_kernel(const __grid
             o[7] = oriented_of((long long)sxx, (long long)syy, sxy);
         }
     };
+    wait_for_previous();
     stage_raw_async(ws.raw[0], J.yr, w, h, x0, y0);
     for (int p = 0; p <= J.nenc; p++) {
         const Region &raw = ws.raw[p & 1];
@@ -465,6 +466,7 @@ constexpr int kAdvPixels = 8 * kAdvThreads;  // per block
 
 __global__ void __launch_bounds__(kAdvThreads) advance_kernel(const __grid_constant__ AdvanceBatch B)
 {
+    wait_for_previous();
     const int jb = find_job(B.njobs, (int)blockIdx.x, [&](int k) { return B.job[k].first_block; });
     const AdvanceJob &J = B.job[jb];
     const size_t at = (size_t)(blockIdx.x - J.first_block) * kAdvPixels + 8 * threadIdx.x;
@@ -531,6 +533,7 @@ __global__ void __launch_bounds__(kWThreads, 4) persist_kernel(const __grid_cons
     const bool inside = wx < ww && wy < wh;
     // pictures in turn: E, O, the centre frame, the encodes at the centre frame
     const int last = J.nenc + 2;
+    wait_for_previous();
     auto stage = [&](int p) {
         const uint16_t *src = p == 0 ? J.e_new : p == 1 ? J.o_new : p == 2 ? J.y_c : J.yd[p - 3];
         stage_raw_async(ps.raw[p & 1], src, w, h, x0, y0);
@@ -898,6 +901,7 @@ __global__ void __launch_bounds__(kCW) collect_windows_kernel(const __grid_const
 // cleared. (As three copies and two memory clears per source they cost the step 15 us of waiting on one another.)
 __global__ void __launch_bounds__(32 * kCollectSums) collect_final_kernel(const __grid_constant__ CollectBatch B)
 {
+    wait_for_previous();
     int jb = 0;
     while (jb + 1 < B.njobs && (int)blockIdx.x >= B.job[jb + 1].first_enc) jb++;
     const CollectJob &J = B.job[jb];
@@ -957,8 +961,7 @@ cudaError_t launch_window_stats(WindowBatch &b, cudaStream_t s)
                                                (int)sizeof(WinStatsSmem));
     if (e != cudaSuccess) return e;
     LaunchTimer t("window_stats", s);
-    window_stats_kernel<<<blocks, kWThreads, sizeof(WinStatsSmem), s>>>(b);
-    return after_launch();
+    return launch_kernel(true, window_stats_kernel, dim3(blocks), kWThreads, sizeof(WinStatsSmem), s, b);
 }
 
 cudaError_t launch_persist(PersistBatch &b, cudaStream_t s)
@@ -976,13 +979,11 @@ cudaError_t launch_persist(PersistBatch &b, cudaStream_t s)
     }
     if (advance == 0) return cudaSuccess;
     LaunchTimer t("persist_stats", s);
-    advance_kernel<<<(unsigned)advance, kAdvThreads, 0, s>>>(ab);
-    cudaError_t e = after_launch();
+    cudaError_t e = launch_kernel(true, advance_kernel, dim3((unsigned)advance), kAdvThreads, 0, s, ab);
     if (e != cudaSuccess || blocks == 0) return e;
     e = cudaFuncSetAttribute(persist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PersistSmem));
     if (e != cudaSuccess) return e;
-    persist_kernel<<<blocks, kWThreads, sizeof(PersistSmem), s>>>(b);
-    return after_launch();
+    return launch_kernel(true, persist_kernel, dim3(blocks), kWThreads, sizeof(PersistSmem), s, b);
 }
 
 cudaError_t launch_pair_sums(PairSumsBatch &b, cudaStream_t s)
@@ -1040,8 +1041,7 @@ cudaError_t launch_collect_sums(CollectBatch &b, cudaStream_t s)
     e = after_launch();
     if (e != cudaSuccess) return e;
     LaunchTimer t("frame_collect_final", s);
-    collect_final_kernel<<<encs, 32 * kCollectSums, 0, s>>>(b);
-    return after_launch();
+    return launch_kernel(true, collect_final_kernel, dim3(encs), 32 * kCollectSums, 0, s, b);
 }
 
 // ---------------------------------------------------------------------------------------------------------------

@@ -160,6 +160,7 @@ extern "C" int es_cambi_score_noalloc(uint64_t img, int pitch, int w, int h, int
             db.job[0].h[k - 2] = c.sh[k];
         }
         db.chained = 1;
+        db.early = 1;
         cuda_check(launch_decimate_mode(db, s), "cambi scales");
         CvBatch cb{};
         cb.njobs = kScales;
@@ -188,7 +189,6 @@ extern "C" int es_cambi_score_noalloc(uint64_t img, int pitch, int w, int h, int
         cuda_check(launch_topk(slots, kScales, s, true), "cambi top-k");
         ScoreBatch sb{};
         sb.njobs = 1;
-        sb.chained = 1;
         sb.job[0].first_slot = 0;
         sb.job[0].window = p.window;
         sb.job[0].score = rec;
