@@ -69,8 +69,8 @@ def algorithmic_bytes(name: str, wl: dict) -> float | None:
     sp = scale_pixels(w, h)
     table = {
         "cambi_cvalues": 2.0 * sum(sp) * pics,              # every picture's 5 scale planes (16-bit words)
-        "cambi_prep0": (2.0 * n + 2.0 * n) * pics,          # plane in, scale-0 words out
-        "cambi_decimate_mode": 4.0 * sum(sp[1:]) * pics,    # scale s - 1's even rows in, scale s out
+        "cambi_prep0": (2.0 * n + 2.0 * (sp[0] + sp[1])) * pics,        # plane in, words of scales 0 and 1 out
+        "cambi_decimate_mode": (1.0 * sp[1] + 2.0 * sum(sp[2:])) * pics,  # scale 1's even rows in, scales 2 to 4 out
         "window_stats": 2.0 * n * (1 + e) + 32.0 * windows * e,
         "persist_stats": 2.0 * n * (2 + 4 + 2 + e) + 20.0 * windows * e,
         "pair_sums": 3.0 * n * (1 + e),
@@ -536,7 +536,7 @@ def main() -> None:
 
     # ---- device-resident legs: the plain form (es_frame) and the batched form (es_batch, CUDA graphs) -------------
     class PlainForm:
-        name = "plain (es_frame queue/collect, one launch set per picture, CAMBI on per-picture streams)"
+        name = "plain (es_frame queue/collect: one source per step, every kernel launched by itself)"
 
         def __init__(self):
             self.fr = es_b200.Frame(module, w, h, pd, n_enc)
