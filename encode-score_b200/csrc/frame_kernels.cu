@@ -240,10 +240,23 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 // Queues the copy of `src`'s region at tile (x0, y0) into raw (unshifted; rows clamped): 8-byte asynchronous copies
 // where the columns lie inside the picture and the rows are 8-byte aligned, else plain loads and stores now. Every
-// thread commits one group of copies (possibly empty).
+// thread commits one group of copies (possibly empty). kUnroll: a tile without a row to clamp takes its copies without a
+// loop, 5 % of persist_kernel's time (window_stats has no registers left for their addresses: 174 against 171 us).
+template <bool kUnroll>
 __device__ __forceinline__ void stage_raw_async(Region &raw, const uint16_t *src, int w, int h, int x0, int y0)
 {
-    if (x0 >= kM && x0 + kWT + kM <= w && (w & 3) == 0 && ((uintptr_t)src & 7) == 0) {
+    const bool vec = x0 >= kM && x0 + kWT + kM <= w && (w & 3) == 0 && ((uintptr_t)src & 7) == 0;
+    if (kUnroll && vec && y0 >= kM && y0 + kWT + kM <= h) {
+        // no row to clamp: thread (q, r) copies group q of rows r, r + 7, ...
+        const int r = threadIdx.x / 18, q = threadIdx.x - 18 * r;
+        if (r < 7) {
+            const uint16_t *p = src + (size_t)(y0 - kM + r) * w + (x0 - kM) + 4 * q;
+            uint16_t *to = &raw[r][4 * q];
+#pragma unroll
+            for (int k = 0; k < kWR / 7; k++) cp_async8(to + 7 * k * kWS, p + (size_t)(7 * k) * w);
+            if (r < kWR % 7) cp_async8(to + kWR / 7 * 7 * kWS, p + (size_t)(kWR / 7 * 7) * w);
+        }
+    } else if (vec) {
         for (int i = threadIdx.x; i < kWR * 18; i += kWThreads) {
             const int r = i / 18, q = i - r * 18;
             const int y = min(max(y0 - kM + r, 0), h - 1);
@@ -422,12 +435,12 @@ __global__ void __launch_bounds__(kWThreads, 4) window_stats_kernel(const __grid
         }
     };
     wait_for_previous();
-    stage_raw_async(ws.raw[0], J.yr, w, h, x0, y0);
+    stage_raw_async<false>(ws.raw[0], J.yr, w, h, x0, y0);
     for (int p = 0; p <= J.nenc; p++) {
         const Region &raw = ws.raw[p & 1];
         __syncthreads();  // the walk of picture p - 1 is done with the buffer picture p + 1 goes to
         if (p < J.nenc) {
-            stage_raw_async(ws.raw[(p + 1) & 1], J.yd[p], w, h, x0, y0);
+            stage_raw_async<false>(ws.raw[(p + 1) & 1], J.yd[p], w, h, x0, y0);
             cp_async_wait<1>();  // picture p's copies are in; p + 1's may still be in flight
         } else {
             cp_async_wait<0>();
@@ -449,7 +462,7 @@ __global__ void __launch_bounds__(kWThreads, 4) window_stats_kernel(const __grid
 // columns 2 c and 2 c + 1 down window row g with running vertical sums of the mid-detail numerators. When each tile
 // advanced its own region of the sums first, the scattered 8-byte loads of that part alone took 59 of 98 us for a 3840 x
 // 2160 pair at 20 % of the memory's rate. One kernel with a column per thread took 82 us for that pair, 107 us with three
-// encodes and 317 us for 16 uneven pairs; the two now take 78, 104 and 296 us, of which 26, 26 and 93 us advance.
+// encodes and 317 us for 16 uneven pairs; the two now take 75, 99 and 280 us, of which 26, 26 and 93 us advance.
 // ---------------------------------------------------------------------------------------------------------------
 struct AdvanceJob {
     const uint16_t *e_old, *o_old, *y_m13, *y_m7, *y_c, *y_f;
@@ -536,7 +549,7 @@ __global__ void __launch_bounds__(kWThreads, 4) persist_kernel(const __grid_cons
     wait_for_previous();
     auto stage = [&](int p) {
         const uint16_t *src = p == 0 ? J.e_new : p == 1 ? J.o_new : p == 2 ? J.y_c : J.yd[p - 3];
-        stage_raw_async(ps.raw[p & 1], src, w, h, x0, y0);
+        stage_raw_async<true>(ps.raw[p & 1], src, w, h, x0, y0);
     };
     auto sums = [&](int p) {  // horizontal sums of picture p; picture p + 1's copies go on meanwhile
         __syncthreads();      // the sums of picture p - 1 are read, and its buffer takes picture p + 1
