@@ -675,6 +675,7 @@ int es_batch_create(const es_module *m, int n_sources, const es_batch_source *so
                     "es_batch_create: every picture must be even and at least 16 x 16");
             require(d.pd == 8 || d.pd == 10, "es_batch_create: pipeline depth must be 8 or 10");
             require(d.n_encodes >= 1 && d.n_encodes <= kMaxEncodes, "es_batch_create: 1 to 16 encodes per source");
+            check_cambi(d.w, d.h, d.pd, derive_params(d.w, d.h));
             pictures += 1 + d.n_encodes;
         }
         require(pictures <= kMaxBatchPictures, "es_batch_create: at most 64 pictures (sources and encodes) per batch");

@@ -10,6 +10,18 @@
 
 namespace es {
 const void *kernel_entry_cvalues();
+
+// A column's count of one code, at most the window's 2 pad + 1 rows, shares a word with three others; the c-value kernel
+// has a form for windows of up to 129 (5 k-steps of 32 columns).
+void check_cambi(int w, int h, int depth, const es_cambi_params &p)
+{
+    require(w > 1 && h > 1, "CAMBI needs a picture of at least 2 x 2 pixels");
+    require(depth == 8 || depth == 10, "CAMBI takes 8- or 10-bit planes");
+    require(p.pad >= 0 && p.pad <= kMaxPad && p.window == 2 * p.pad + 1, "CAMBI window must be odd and at most 129");
+    require(p.band_size > 0 && p.band_size <= kMaxBand && p.band_base >= 0 && p.band_base + p.band_size <= kMaxBand + 8,
+            "CAMBI band out of range");
+    require(p.topk > 0 && p.topk <= 1, "CAMBI topk must be in (0, 1]");
+}
 }
 
 using namespace es;
@@ -36,12 +48,7 @@ namespace {
 
 void init_cambi(es_cambi *c, int w, int h, int depth, const es_cambi_params &p)
 {
-    require(w > 1 && h > 1, "CAMBI needs a picture of at least 2 x 2 pixels");
-    require(depth == 8 || depth == 10, "CAMBI takes 8- or 10-bit planes");
-    require(p.pad >= 0 && p.pad <= kMaxPad && p.window == 2 * p.pad + 1, "CAMBI window must be odd and at most 129");
-    require(p.band_size > 0 && p.band_size <= kMaxBand && p.band_base >= 0 && p.band_base + p.band_size <= kMaxBand + 8,
-            "CAMBI band out of range");
-    require(p.topk > 0 && p.topk <= 1, "CAMBI topk must be in (0, 1]");
+    check_cambi(w, h, depth, p);
     c->w = w;
     c->h = h;
     c->depth = depth;

@@ -781,6 +781,7 @@ cudaError_t launch_cvalues(const CvBatch &batch, cudaStream_t s)
     b.need_last = lo < 0 ? 0 : hi + b.band.band_base;
     int n = 2;
     for (int j = 0; j < b.njobs; j++) n = n > cv_ksteps(b.job[j].pad) ? n : cv_ksteps(b.job[j].pad);
+    if (n > 5) return cudaErrorInvalidValue;  // a pad over kMaxPad: no kernel form reaches that far
     return n <= 3 ? launch_cvalues_n<3>(b, s) : launch_cvalues_n<5>(b, s);
 }
 

@@ -129,6 +129,8 @@ void check_device();
 
 // CAMBI's derived parameters (src/cambi.cpp:39-53).
 es_cambi_params derive_params(int w, int h);
+// Throws ES_ERR_INVALID unless CAMBI's kernels take a w x h picture with these parameters.
+void check_cambi(int w, int h, int depth, const es_cambi_params &p);
 // lut[i] = 1/i as float for i < (2 pad + 1)^2 + 1, lut[0] = 0.
 void reciprocal_table(int pad, float *lut, size_t n);
 // src/cambi.cpp:29: clip((int)(topk * n), 1, n).

@@ -217,7 +217,8 @@ typedef struct {
     uint32_t lasting_windows;   /* lasting-texture windows of frame f - 6 (when texture) */
 } es_frame_result;
 
-/* `w` x `h` is the common picture area (even), `pd` the pipeline depth (8 or 10, src/main.cpp:377-382). */
+/* `w` x `h` is the common picture area (even, at least 16 x 16, w + h below 12000: as es_cambi_create, it refuses
+ * pictures whose CAMBI window is over 129), `pd` the pipeline depth (8 or 10, src/main.cpp:377-382). */
 int es_frame_create(const es_module *m, int w, int h, int pd, int n_encodes, es_frame **out);
 /* Frame f (0, 1, 2, ... in order). source / encodes[i] are device frames cropped at (sx, sy) / (ex[i], ey[i]);
  * source_cambi = 0 skips the source's CAMBI (src/main.cpp:522-523, a cached value given to collect instead). */
@@ -306,7 +307,7 @@ void es_proposal_net_destroy(es_proposal_net *net);
  * --------------------------------------------------------------------------------------------------------------- */
 typedef struct es_batch es_batch;
 typedef struct {
-    int w, h;      /* common picture area of the source and its encodes (even) */
+    int w, h;      /* common picture area of the source and its encodes, as es_frame_create's */
     int pd;        /* pipeline depth, 8 or 10 */
     int n_encodes; /* 1 to 16 */
     int cv_tile_rows[5]; /* rows of the c-value tiles per scale: 64, 32 or 16 (0 = chosen by the scale's size); an

@@ -188,3 +188,28 @@ def test_score_known_answers():
     p = accum(0, 0, windows=3, vmaf=90.0)
     assert math.isnan(p.texture)
     assert p.score == pytest.approx((90 * 0.30 + 100 * 0.40) / 0.70)
+
+
+@pytest.mark.parametrize("w,h,refused", [(7680, 4320, True), (8192, 4320, True), (16, 11984, True), (7680, 4318, False), (16, 16, False)])
+@pytest.mark.parametrize("what", ["frame", "batch"])
+def test_pictures_whose_window_is_too_wide_are_refused(what, w, h, refused):
+    """CAMBI's window grows with the picture; over 129 its counts no longer fit the kernels. The refusal comes before the
+    device is looked for, so it shows here; an accepted size gets as far as the device (with one, the GPU tests create it)."""
+    import torch
+
+    lib, out, module = es_b200.lib(), ctypes.c_void_p(), ctypes.c_void_p(1)  # the module is only tested for NULL
+    if torch.cuda.is_available() and not refused:
+        pytest.skip("a GPU is present")
+    if what == "frame":
+        status = lib.es_frame_create(module, w, h, 10, 1, ctypes.byref(out))
+    else:
+        src = (es_b200.BatchSource * 2)()
+        for k, size in enumerate(((1920, 1080), (w, h))):
+            src[k].w, src[k].h = size
+            src[k].pd, src[k].n_encodes = 10, 1
+        status = lib.es_batch_create(module, 2, src, None, ctypes.byref(out))
+    assert not out.value
+    if refused:
+        assert status == es_b200.ES_ERR_INVALID and b"at most 129" in lib.es_last_error()
+    else:
+        assert status not in (es_b200.ES_OK, es_b200.ES_ERR_INVALID)
