@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <string>
 #include <vector>
 
 #include "es_internal.h"
@@ -26,10 +27,14 @@ struct es_frame {
 
 namespace {
 
-// a failed call of the batch beneath fails this one alike
+// A failed call of the batch beneath fails this one alike; its message names the call that was made.
 void pass(int status)
 {
-    if (status != ES_OK) throw Error(status, es_last_error());
+    if (status == ES_OK) return;
+    std::string what = es_last_error();
+    const std::string theirs = "es_batch_", ours = "es_frame_";
+    for (size_t at = 0; (at = what.find(theirs, at)) != std::string::npos; at += ours.size()) what.replace(at, theirs.size(), ours);
+    throw Error(status, what);
 }
 
 // the n bins the collect kernel wrote (only those that count)

@@ -243,3 +243,35 @@ def test_structure_threshold_at_large_sizes(cuda, module, w, h, kind):
         assert np.array_equal(np.array(acc[0].matching[k].bins), want.matching[k].bins)
     for name in ("st_r", "st_d", "sh_st_x"):
         assert np.allclose(np.array(list(getattr(acc[0], name))), getattr(want, name), rtol=1e-12, atol=0), name
+
+
+def test_errors_name_the_frame_call_that_was_made(cuda, module):
+    """A frame step is a batch of one source underneath; what it refuses is told as the frame call's own error."""
+    torch = cuda
+    step = es_synth.c2_step(0, w=64, h=48, n_encodes=1)
+    fr = es_b200.Frame(module, 64, 48, 10, 1)
+    devs = [DevFrame(torch, raw_frame(p, "planar16"), 10) for p in (step.source, step.encodes[0])]
+    src, enc = devs[0].view, [devs[1].view]
+
+    def error(status, call, *args, **kw):
+        with pytest.raises(es_b200.EsError) as e:
+            getattr(fr, call)(*args, **kw)
+        assert e.value.status == status and f"es_frame_{call}:" in str(e.value) and "es_batch" not in str(e.value), str(e.value)
+
+    error(es_b200.ES_ERR_INVALID, "queue", 1, src, enc)
+    error(es_b200.ES_ERR_INVALID, "queue", 0, src, enc, sx=1)
+    error(es_b200.ES_ERR_INVALID, "queue", 0, src, enc, ey=[-2])
+    error(es_b200.ES_ERR_STATE, "collect", 0, None, None)
+    error(es_b200.ES_ERR_STATE, "luma", 0, 0)
+    error(es_b200.ES_ERR_INVALID, "luma", 2, 0)
+    error(es_b200.ES_ERR_STATE, "read_windows", 0)
+    fr.queue(0, src, enc)
+    fr.queue(1, src, enc, source_cambi=False)
+    error(es_b200.ES_ERR_STATE, "queue", 2, src, enc)
+    fr.collect(0, None, None)
+    error(es_b200.ES_ERR_STATE, "collect", 0, None, None)
+    error(es_b200.ES_ERR_INVALID, "collect", 1, None, None)
+    error(es_b200.ES_ERR_INVALID, "read_windows", 0, persist=True)
+    error(es_b200.ES_ERR_INVALID, "read_windows", 1)
+    fr.collect(1, None, None, 0.25)
+    fr.close()
