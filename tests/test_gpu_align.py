@@ -229,3 +229,59 @@ def test_thumbnails_of_crops_that_start_and_end_anywhere(cuda, module, fmt, x0, 
         sums = np.add.reduceat(np.add.reduceat(v[k, :ys[-1], :xs[-1]], ys[:-1], axis=0), xs[:-1], axis=1)
         n = np.outer(np.diff(ys), np.diff(xs))
         assert np.array_equal(got[k], sums.astype(np.float32) / n.astype(np.float32)), k
+
+
+@pytest.mark.parametrize("n_ref,n_probe,inexact", [(3641, 3641, False), (3642, 3641, True), (2100, 24, False), (2072, 25, True)])
+def test_offset_totals_at_the_limits_of_the_exact_sums_and_the_fixed_array(cuda, module, n_ref, n_probe, inexact):
+    """Over 3640 probe frames the exact sums could leave 53 bits and every lag is added in order; over 2048 lags
+    es_find_offset allocates its totals. Both entries, values that are exact in any order and values that are not."""
+    rng = np.random.default_rng(n_ref)
+    ref = (rng.integers(8 * 900, 1023 * 900, (n_ref, 2304)) / 900).astype(np.float32)
+    at = (n_ref - n_probe) * 2 // 3
+    probe = np.clip(ref[at:at + n_probe] + rng.integers(-3, 4, (n_probe, 2304)).astype(np.float32), 0, 1023)
+    if inexact:
+        ref[at // 2, ::7] = np.float32(1) / np.float32(3)
+    lags = n_ref - n_probe + 1
+    d_ref, d_probe = cuda.from_numpy(ref.ravel()).cuda(), cuda.from_numpy(probe.ravel()).cuda()
+    totals = cuda.full((lags,), -1.0, dtype=cuda.float64, device="cuda")
+    es_b200.offset_totals(d_ref.data_ptr(), n_ref, d_probe.data_ptr(), n_probe, totals.data_ptr())
+    want = align.lag_totals(ref, probe)
+    assert np.array_equal(totals.cpu().numpy().view(np.uint64), want.view(np.uint64))
+    off, best = es_b200.find_offset(d_ref.data_ptr(), [k / 25.0 for k in range(n_ref)], d_probe.data_ptr(), [k / 25.0 for k in range(n_probe)])
+    lag = int(np.argmin(want))
+    assert lag == at and off == lag / 25.0 and best == want[lag] / (n_probe * 2304.0)
+
+
+def test_find_offset_from_many_threads(cuda, module):
+    """Twelve callers at once, each with a stream and an answer of its own: eight take a place in the library's array of
+    totals, the others allocate theirs."""
+    import threading
+
+    rng = np.random.default_rng(5)
+    ref = (rng.integers(8 * 900, 1023 * 900, (160, 2304)) / 900).astype(np.float32)
+    d_ref = cuda.from_numpy(ref.ravel()).cuda()
+    times = [k / 24.0 for k in range(160)]
+    callers, wrong = 12, []
+    host = [ref[9 * k:9 * k + 40] + np.float32(k % 3) for k in range(callers)]
+    want = [align.lag_totals(ref[9 * k:9 * k + 40], host[k])[0] / (40 * 2304.0) for k in range(callers)]
+    probes = [cuda.from_numpy(p.ravel()).cuda() for p in host]
+    streams = [cuda.cuda.Stream() for _ in range(callers)]
+    cuda.cuda.synchronize()
+    start = threading.Barrier(callers)
+
+    def caller(k):
+        try:
+            start.wait()
+            for _ in range(20):
+                off, best = es_b200.find_offset(d_ref.data_ptr(), times, probes[k].data_ptr(), times[:40], streams[k].cuda_stream)
+                if off != times[9 * k] or best != want[k]:
+                    wrong.append((k, off, best))
+        except Exception as e:  # told below, in the test's own thread
+            wrong.append((k, e))
+
+    threads = [threading.Thread(target=caller, args=(k,)) for k in range(callers)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong

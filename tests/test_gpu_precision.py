@@ -64,3 +64,28 @@ def test_sizes_around_the_table_bands_and_chunks(cuda, module, w, h):
         scale = np.maximum(np.abs(want), 1e-3 * np.abs(want).max(axis=0, keepdims=True))
         assert (np.abs(outs[1] - want) / scale).max() <= 1e-5
     win.close()
+
+
+@pytest.mark.parametrize("w,h,depth", [(16, 16, 10), (65, 33, 10), (130, 63, 8), (208, 144, 10), (191, 32, 8), (16, 16400, 10), (50, 16385, 10)])
+def test_fp32_figures_bit_for_bit(cuda, module, w, h, depth):
+    """The roundings of the FP32 forms are what the study is about: the compensated and the plain figures equal a
+    restatement that adds, multiplies and divides in FP32 in the same order, with whole and partial bands and chunks of the
+    tables and on both sides of the 16384 rows where their kernels change."""
+    rng = np.random.default_rng(w + h)
+    yy, xx = np.mgrid[0:h, 0:w]
+    top = 1023 if depth == 10 else 255
+    yr = np.clip(top * (0.65 + 0.2 * np.sin(xx / 9 + yy / 23)) + rng.normal(0, top / 50, (h, w)), 0, top).astype(np.uint16)
+    yd = np.clip(yr + rng.normal(0, top / 100, (h, w)), 0, top).astype(np.uint16)
+    up = 10 - depth
+    win = es_b200.Windows(w, h)
+    r, d = to_dev(cuda, yr), to_dev(cuda, yd)
+    win.compute(r.data_ptr(), d.data_ptr(), up)
+    for window in (16, 32, 48):
+        n = (w // window) * (h // window)
+        if not n:
+            continue
+        for mode in (1, 2):
+            o = zeros_dev(cuda, (n, 8), np.float64)
+            win.figures(window, mode, o.data_ptr())
+            assert np.array_equal(from_dev(o, np.float64), precision.fp32_window_figures(yr, yd, up, window, mode)), (window, mode)
+    win.close()
