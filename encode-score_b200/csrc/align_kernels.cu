@@ -174,7 +174,8 @@ __global__ void __launch_bounds__(256) thumb_rows_kernel(const __grid_constant__
 // for 256 differences (a float subtraction, a conversion and about one integer addition each). The loads bound it, 47
 // from L2 per 256 differences (conversions spread over other pipes changed nothing, sums in double were slower: 84
 // against 62 us); the in-order form issues about 40 instructions per difference and has one warp per lag. 483 lags of
-// 192 frames: 1027 us in order, 78 us for the three launches.
+// 192 frames: 1035 us in order, 76 us for the three launches; where no lag is exact (means below 8 code values) 1010 us, 1129
+// when offset_exact_kernel added marked lags all the same.
 constexpr double kFixed = 1048576.0;                     // units per code value
 constexpr unsigned long long kInexact = 1ull << 63;      // mark in a lag's integer sum
 constexpr int kExactMaxProbe = (1 << 23) / kThumbPixels;  // frames whose totals stay below 2^53 units
@@ -225,10 +226,12 @@ __global__ void __launch_bounds__(kExThreads, 2) offset_exact_kernel(const float
                                                                      unsigned long long *sums)
 {
     __shared__ unsigned long long total[kExLags];
+    wait_for_previous();
     const int l0 = blockIdx.x * kExLags, i0 = blockIdx.y * kExFrames, lane = threadIdx.x & 31;
     const int n_lags = min(kExLags, lags - l0), n_frames = min(kExFrames, n_probe - i0);
     if (threadIdx.x < kExLags) total[threadIdx.x] = 0;
-    __syncthreads();
+    // nothing to add where every lag is marked (other blocks' additions leave the marks as they are)
+    if (__syncthreads_and((int)threadIdx.x >= n_lags || (__ldcg(sums + l0 + threadIdx.x) & kInexact))) return;
     unsigned long long acc[kExLags];
 #pragma unroll
     for (int l = 0; l < kExLags; l++) acc[l] = 0;
@@ -273,14 +276,15 @@ __device__ __forceinline__ ParityMap compose(const ParityMap &a, const ParityMap
 
 // With kSums, totals[] holds the exact kernels' integer sums: a lag they marked is added as above, any other becomes its
 // sum's double.
-template <bool kVec>
+template <bool kVec, bool kSums>
 __global__ void __launch_bounds__(32 * kLagWarps) offset_totals_kernel(const float *ref, const float *probe, int n_probe, int lags,
-                                                                      double *totals, int sums)
+                                                                      double *totals)
 {
     __shared__ __align__(16) double serial[kLagWarps][kChunk];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, l = blockIdx.x * kLagWarps + w;
     if (l >= lags) return;  // whole warps: one lag per warp
-    if (sums) {
+    if (kSums) {
+        wait_for_previous();
         const unsigned long long v = ((const unsigned long long *)totals)[l];
         if (!(v & kInexact)) {
             __syncwarp();
@@ -420,15 +424,14 @@ cudaError_t launch_offset_totals(const float *ref, int n_ref, const float *probe
         {
             LaunchTimer t("align_offset_exact", s);
             const dim3 grid((lags + kExLags - 1) / kExLags, (n_probe + kExFrames - 1) / kExFrames, kThumbPixels / kExPixels);
-            offset_exact_kernel<<<grid, kExThreads, 0, s>>>(ref, probe, n_probe, lags, sums);
+            e = launch_kernel(true, offset_exact_kernel, grid, kExThreads, 0, s, ref, probe, n_probe, lags, sums);
         }
-        if ((e = after_launch()) != cudaSuccess) return e;
+        if (e != cudaSuccess) return e;
     }
     LaunchTimer t("align_offset_totals", s);
-    const int blocks = (lags + kLagWarps - 1) / kLagWarps;
-    if (vec) offset_totals_kernel<true><<<blocks, 32 * kLagWarps, 0, s>>>(ref, probe, n_probe, lags, totals, exact);
-    else offset_totals_kernel<false><<<blocks, 32 * kLagWarps, 0, s>>>(ref, probe, n_probe, lags, totals, exact);
-    return after_launch();
+    const auto kernel = vec ? exact ? offset_totals_kernel<true, true> : offset_totals_kernel<true, false>
+                            : exact ? offset_totals_kernel<false, true> : offset_totals_kernel<false, false>;
+    return launch_kernel(exact, kernel, dim3((lags + kLagWarps - 1) / kLagWarps), 32 * kLagWarps, 0, s, ref, probe, n_probe, lags, totals);
 }
 
 namespace {
