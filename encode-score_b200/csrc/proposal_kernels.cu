@@ -15,6 +15,8 @@
 //  * propose_kernel / audit_kernel: the per-step tile lists and the audit's estimate, all on the device.
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 #include "cambi_codes.h"
 #include "es_kernels.h"
 
@@ -222,8 +224,9 @@ __global__ void __launch_bounds__(128) conv_bwd_data_kernel(const float *gout, c
 // Weight and bias gradients. A block takes tiles of 8 x 36 output pixels in turn: both planes' tiles are staged in shared
 // memory and a thread holds the 9 taps of one (output, input) channel pair, reading 4 pixels of the gradient and the 6
 // input values of a new row per 36 multiply-adds. Its sums go to its own row of `parts`; net_grads_kernel adds the rows
-// in a fixed order. (One block per pair over every pixel, the form before, left 16 to 256 blocks walking 139 thousand
-// pixels each: 335 us a layer on average, with the data gradients, against 52.)
+// in a fixed order. Only output pixels inside the crop are multiplied: a tile's margin past it would cost time and turn an
+// infinite input into NaN in taps it has no part in. (One block per pair over every pixel, the form before, left 16 to 256
+// blocks walking 139 thousand pixels each: 335 us a layer on average, with the data gradients, against 52.)
 constexpr int kWgRows = 8, kWgCols = 36, kWgStride = 40;
 template <int CI, int CO>
 __global__ void __launch_bounds__(256) conv_bwd_weight_kernel(const float *gout, const float *in, int n, int h, int w,
@@ -243,6 +246,7 @@ __global__ void __launch_bounds__(256) conv_bwd_weight_kernel(const float *gout,
     for (int k = 0; k < 10; k++) acc[k] = 0.0f;
     for (int t = blockIdx.x; t < tiles; t += kNetGradBlocks) {
         const int nn = t / (ty * tx), r = t - nn * ty * tx, y0 = r / tx * kWgRows, x0 = r % tx * kWgCols;
+        const int rows = min(kWgRows, ho - y0), cols = min(kWgCols, wo - x0);  // output pixels inside the crop
         __syncthreads();
         for (int i = tid; i < CI * (kWgRows + 2) * kWgStride; i += 256) {
             const int c = i / ((kWgRows + 2) * kWgStride), q = i % ((kWgRows + 2) * kWgStride), y = y0 + q / kWgStride, x = x0 + q % kWgStride;
@@ -264,38 +268,56 @@ __global__ void __launch_bounds__(256) conv_bwd_weight_kernel(const float *gout,
             v[4] = p.x;
             v[5] = p.y;
         };
-        auto add = [&](const float (&v0)[6], const float (&v1)[6], const float (&v2)[6], int y, int x) {
+        // Whole: the four pixels' columns are inside the crop, else the first two are (crops have an even number of columns)
+        auto add = [&](auto whole, const float (&v0)[6], const float (&v1)[6], const float (&v2)[6], int y, int x) {
             const float4 q = *(const float4 *)(g + y * kWgCols + x);
             const float gv[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
             for (int k = 0; k < 3; k++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
+                for (int j = 0; j < (decltype(whole)::value ? 4 : 2); j++) {
                     acc[k] = __fmaf_rn(gv[j], v0[j + k], acc[k]);
                     acc[3 + k] = __fmaf_rn(gv[j], v1[j + k], acc[3 + k]);
                     acc[6 + k] = __fmaf_rn(gv[j], v2[j + k], acc[6 + k]);
                 }
             acc[9] += (gv[0] + gv[1]) + (gv[2] + gv[3]);
         };
-        if (kGroups == 1) {
-            for (int x = 0; x < kWgCols; x += 4) {
-                float v[3][6];
-                row6(v[0], 0, x);
-                row6(v[1], 1, x);
+        auto column = [&](auto whole, int x) {
+            float v[3][6];
+            row6(v[0], 0, x);
+            row6(v[1], 1, x);
+            if (rows == kWgRows) {
 #pragma unroll
                 for (int y = 0; y < kWgRows; y++) {
                     row6(v[(y + 2) % 3], y + 2, x);
-                    add(v[y % 3], v[(y + 1) % 3], v[(y + 2) % 3], y, x);
+                    add(whole, v[y % 3], v[(y + 1) % 3], v[(y + 2) % 3], y, x);
+                }
+            } else {
+                for (int y = 0; y < rows; y++) {
+                    row6(v[2], y + 2, x);
+                    add(whole, v[0], v[1], v[2], y, x);
+#pragma unroll
+                    for (int k = 0; k < 6; k++) {
+                        v[0][k] = v[1][k];
+                        v[1][k] = v[2][k];
+                    }
                 }
             }
+        };
+        if (kGroups == 1) {
+            int x = 0;
+            for (; x + 4 <= cols; x += 4) column(std::true_type{}, x);
+            if (x < cols) column(std::false_type{}, x);
         } else {
             for (int i = group; i < kWgRows * (kWgCols / 4); i += kGroups) {
                 const int y = i / (kWgCols / 4), x = 4 * (i % (kWgCols / 4));
+                if (y >= rows || x >= cols) continue;
                 float v[3][6];
                 row6(v[0], y, x);
                 row6(v[1], y + 1, x);
                 row6(v[2], y + 2, x);
-                add(v[0], v[1], v[2], y, x);
+                if (x + 4 <= cols) add(std::true_type{}, v[0], v[1], v[2], y, x);
+                else add(std::false_type{}, v[0], v[1], v[2], y, x);
             }
         }
     }

@@ -185,3 +185,28 @@ def test_gradients_of_crops_around_the_weight_kernels_tiles(cuda, module, n, th,
             got = grads[at:at + g.size].reshape(g.shape)
             assert np.abs(got - g).max() <= 1e-3 * np.abs(g).max() + 1e-9
             at += g.size
+
+
+@pytest.mark.parametrize("n,th,tw", [(1, 1, 1), (2, 2, 2), (1, 4, 4)])
+def test_an_infinite_input_reaches_only_the_taps_that_read_it(cuda, module, n, th, tw):
+    """The last pixel of a crop's first channel is read by one tap of the first layer. Infinite there (and masked by the
+    ReLU behind it, so that everything else stays finite), it makes that tap's weight gradients NaN (0 x inf) and leaves
+    every other gradient as a finite value in its place leaves it, whatever the weight kernel's tiles reach past a crop."""
+    rng = np.random.default_rng(n + th + tw)
+    h, w = 8 + 16 * th, 8 + 16 * tw
+    params = random_params(8)
+    params[0][0][:, 0, 2, 2] = 0.5
+    xd = rng.normal(0, 1, (n, 2, h, w)).astype(np.float32)
+    ld = to_dev(cuda, rng.normal(0.5, 0.5, (n, th, tw)).astype(np.float32))
+    grads = []
+    for corner in (-1e4, -np.inf):
+        xd[:, 0, h - 1, w - 1] = corner
+        net = es_b200.ProposalNet(proposal.flatten(params))
+        x = to_dev(cuda, xd)
+        _, g = net.train_step(x.data_ptr(), ld.data_ptr(), n, h, w, 0.0, want_grads=True)
+        grads.append(np.array(g))
+        net.close()
+    hit = np.zeros(grads[0].shape, bool)
+    hit[:16 * 2 * 9].reshape(16, 2, 3, 3)[:, 0, 2, 2] = True
+    assert np.isfinite(grads[0]).all() and np.isnan(grads[1][hit]).all()
+    assert np.array_equal(grads[1][~hit], grads[0][~hit])
