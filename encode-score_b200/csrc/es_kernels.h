@@ -448,20 +448,27 @@ inline size_t feature_map_size(int w, int h) { return (size_t)((w + 3) / 4) * ((
 cudaError_t launch_net_features(const uint16_t *word, int w, int h, const int *xy, int n, int fw, int fh, float *out,
                                 cudaStream_t s);
 // Training on crops (NCHW float, h even): forward of layer l (input n x ci x h x w, output n x co x (h - 2) x (w - 2),
-// ReLU for l < 3); backward of layer l (its weights' and biases' gradients in kNetGradBlocks parts of kNetParams floats
+// ReLU for l < 3); backward of layer l (its weights' and biases' gradients in net_grad_blocks parts of kNetParams floats
 // and, for l > 0, the gradient of its input times the ReLU mask of that input into gin); the tile loss of the last layer (n x 1 x 16a x 16b against
 // n x a x b labels: per-tile squared differences into loss_parts, the gradient of the last layer's output into gz);
 // and the gradients from every layer's parts, with Adam's step on them when lr > 0 (master weights, their
 // bfloat16-rounded copy, moments).
-constexpr int kNetGradBlocks = 148 * 2;
+constexpr int kNetGradBlocks = 148 * 2;                 // parts at most
+constexpr int kNetGradRows = 8, kNetGradCols = 36;      // output pixels of a block's tile
+// Parts of a layer with an n x h x w input.
+inline int net_grad_blocks(int n, int h, int w)
+{
+    const size_t tiles = (size_t)n * ((h - 2 + kNetGradRows - 1) / kNetGradRows) * ((w - 2 + kNetGradCols - 1) / kNetGradCols);
+    return tiles < (size_t)kNetGradBlocks ? (int)tiles : kNetGradBlocks;
+}
 cudaError_t launch_net_forward(int layer, const float *in, int n, int h, int w, const float *params, float *out,
                                cudaStream_t s);
 cudaError_t launch_net_backward(int layer, const float *gout, const float *in, int n, int h, int w, const float *params,
                                 float *gin, float *parts, cudaStream_t s);
 cudaError_t launch_net_loss(const float *z, const float *labels, int n, int ta, int tb, float *gz, float *loss_parts,
                             cudaStream_t s);
-cudaError_t launch_net_grads(const float *parts, float *params, float *rounded, float *grads, float *m, float *v, float lr, float b1,
-                             float b2, float eps, int t, cudaStream_t s);
+cudaError_t launch_net_grads(const float *parts, int n, int h, int w, float *params, float *rounded, float *grads, float *m, float *v,
+                             float lr, float b1, float b2, float eps, int t, cudaStream_t s);
 // The mma B fragments of layers 1 and 2 (kNetFrags words) from the bfloat16-rounded parameters.
 cudaError_t launch_net_pack(const float *rounded, uint32_t *frags, cudaStream_t s);
 

@@ -144,7 +144,7 @@ int es_proposal_net_train_step(es_proposal_net *net, const float *x, const float
             net->t++;
             net->frags_current = false;
         }
-        cuda_check(launch_net_grads(net->parts.ptr, net->params.ptr, net->rounded.ptr, net->grads.ptr, net->m.ptr, net->v.ptr, lr, 0.9f, 0.999f,
+        cuda_check(launch_net_grads(net->parts.ptr, n, h, w, net->params.ptr, net->rounded.ptr, net->grads.ptr, net->m.ptr, net->v.ptr, lr, 0.9f, 0.999f,
                                     1e-8f, net->t, s),
                    "training step");
         if (grads)

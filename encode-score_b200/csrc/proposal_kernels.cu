@@ -125,12 +125,13 @@ __global__ void __launch_bounds__(256) feature_map_kernel(const __grid_constant_
 // ---------------------------------------------------------------------------------------------------------------
 // Training: valid 3 x 3 convolutions on NCHW float crops, weights rounded to bfloat16. What bounds them is the FP32 fused
 // multiply-adds (2.1 G per step of 32 crops of 72 x 72: 58 us at the FP32 rate) and, beside them, the shared-memory reads
-// of the weights: a thread makes two pixels, one above the other, of all 16 channels, so one 16-byte read of four weights
-// serves eight multiply-adds. Per step of 32 crops, before / now: forward 142 / 89 us, backward 1339 / 209 us.
+// of the weights: a thread makes one or two pixels (net_two_pixels), one above the other, of all 16 channels, so one 16-byte
+// read of four weights serves four or eight multiply-adds. Per step of 32 crops, before / now: forward 142 / 85 us, backward
+// 1339 / 215 us.
 // ---------------------------------------------------------------------------------------------------------------
-// acc[j][c] += v[j] w[c] for the N channels of one tap
-template <int N>
-__device__ __forceinline__ void tap_fma(float (&acc)[2][N], float v0, float v1, const float *w)
+// acc[j][c] += v[j] w[c] for the N channels of one tap and J pixels
+template <int N, int J>
+__device__ __forceinline__ void tap_fma(float (&acc)[J][N], const float (&v)[J], const float *w)
 {
     if constexpr (N % 4 == 0) {
 #pragma unroll
@@ -138,22 +139,21 @@ __device__ __forceinline__ void tap_fma(float (&acc)[2][N], float v0, float v1, 
             const float4 q = *(const float4 *)(w + c);
             const float wv[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                acc[0][c + k] = __fmaf_rn(v0, wv[k], acc[0][c + k]);
-                acc[1][c + k] = __fmaf_rn(v1, wv[k], acc[1][c + k]);
-            }
+            for (int k = 0; k < 4; k++)
+#pragma unroll
+                for (int j = 0; j < J; j++) acc[j][c + k] = __fmaf_rn(v[j], wv[k], acc[j][c + k]);
         }
     } else {
 #pragma unroll
-        for (int c = 0; c < N; c++) {
-            acc[0][c] = __fmaf_rn(v0, w[c], acc[0][c]);
-            acc[1][c] = __fmaf_rn(v1, w[c], acc[1][c]);
-        }
+        for (int c = 0; c < N; c++)
+#pragma unroll
+            for (int j = 0; j < J; j++) acc[j][c] = __fmaf_rn(v[j], w[c], acc[j][c]);
     }
 }
 
-// A thread makes output pixels (y, x) and (y + 1, x), y even (crops have an even number of rows), of every channel.
-template <int CI, int CO>
+// A thread makes output pixels (y, x) .. (y + J - 1, x), y a multiple of J (crops have an even number of rows), of every
+// channel.
+template <int CI, int CO, int J>
 __global__ void __launch_bounds__(128) conv_fwd_kernel(const float *in, int n, int h, int w, const float *P, int woff, int boff,
                                                        bool relu, float *out)
 {
@@ -162,30 +162,37 @@ __global__ void __launch_bounds__(128) conv_fwd_kernel(const float *in, int n, i
     for (int i = threadIdx.x; i < CO * CI * 9; i += 128) W[(i % (CI * 9)) * CO + i / (CI * 9)] = bf16r(P[woff + i]);
     for (int i = threadIdx.x; i < CO; i += 128) B[i] = bf16r(P[boff + i]);
     __syncthreads();
-    const int ho = h - 2, wo = w - 2, pairs = ho / 2 * wo, idx = blockIdx.x * 128 + threadIdx.x;
-    if (idx >= pairs * n) return;
-    const int nn = idx / pairs, r = idx - nn * pairs, y = 2 * (r / wo), x = r % wo;
-    float acc[2][CO];
+    const int ho = h - 2, wo = w - 2, groups = ho / J * wo, idx = blockIdx.x * 128 + threadIdx.x;
+    if (idx >= groups * n) return;
+    const int nn = idx / groups, r = idx - nn * groups, y = J * (r / wo), x = r % wo;
+    float acc[J][CO];
 #pragma unroll
-    for (int co = 0; co < CO; co++) acc[0][co] = acc[1][co] = B[co];
+    for (int co = 0; co < CO; co++)
+#pragma unroll
+        for (int j = 0; j < J; j++) acc[j][co] = B[co];
     const float *src = in + ((size_t)nn * CI * h + y) * w + x;
     for (int ci = 0; ci < CI; ci++, src += (size_t)h * w) {
-        float v[4][3];
+        float v[J + 2][3];
 #pragma unroll
-        for (int k = 0; k < 12; k++) v[k / 3][k % 3] = __ldg(src + (k / 3) * w + k % 3);
+        for (int k = 0; k < 3 * (J + 2); k++) v[k / 3][k % 3] = __ldg(src + (k / 3) * w + k % 3);
 #pragma unroll
-        for (int k = 0; k < 9; k++) tap_fma<CO>(acc, v[k / 3][k % 3], v[k / 3 + 1][k % 3], W + (ci * 9 + k) * CO);
+        for (int k = 0; k < 9; k++) {
+            float t[J];
+#pragma unroll
+            for (int j = 0; j < J; j++) t[j] = v[k / 3 + j][k % 3];
+            tap_fma(acc, t, W + (ci * 9 + k) * CO);
+        }
     }
 #pragma unroll
     for (int co = 0; co < CO; co++)
 #pragma unroll
-        for (int j = 0; j < 2; j++)
+        for (int j = 0; j < J; j++)
             out[((size_t)(nn * CO + co) * ho + y + j) * wo + x] = relu ? fmaxf(acc[j][co], 0.0f) : acc[j][co];
 }
 
 // gin = (full correlation of gout with the flipped kernel) x (in > 0): the gradient of the layer's input, through the
-// ReLU that produced it, two input pixels per thread as above.
-template <int CI, int CO>
+// ReLU that produced it, J input pixels per thread as above.
+template <int CI, int CO, int J>
 __global__ void __launch_bounds__(128) conv_bwd_data_kernel(const float *gout, const float *in, int n, int h, int w,
                                                             const float *P, int woff, float *gin)
 {
@@ -195,27 +202,34 @@ __global__ void __launch_bounds__(128) conv_bwd_data_kernel(const float *gout, c
         W[(co * 9 + r % 9) * CI + r / 9] = bf16r(P[woff + i]);
     }
     __syncthreads();
-    const int ho = h - 2, wo = w - 2, pairs = h / 2 * w, idx = blockIdx.x * 128 + threadIdx.x;
-    if (idx >= pairs * n) return;
-    const int nn = idx / pairs, r = idx - nn * pairs, y = 2 * (r / w), x = r % w;
-    float acc[2][CI];
+    const int ho = h - 2, wo = w - 2, groups = h / J * w, idx = blockIdx.x * 128 + threadIdx.x;
+    if (idx >= groups * n) return;
+    const int nn = idx / groups, r = idx - nn * groups, y = J * (r / w), x = r % w;
+    float acc[J][CI];
 #pragma unroll
-    for (int ci = 0; ci < CI; ci++) acc[0][ci] = acc[1][ci] = 0.0f;
+    for (int ci = 0; ci < CI; ci++)
+#pragma unroll
+        for (int j = 0; j < J; j++) acc[j][ci] = 0.0f;
     for (int co = 0; co < CO; co++) {
         const float *src = gout + (size_t)(nn * CO + co) * ho * wo;
-        float g[4][3];  // gout rows y - 2 .. y + 1, columns x - 2 .. x; 0 outside
+        float g[J + 2][3];  // gout rows y - 2 .. y + J - 1, columns x - 2 .. x; 0 outside
 #pragma unroll
-        for (int k = 0; k < 12; k++) {
+        for (int k = 0; k < 3 * (J + 2); k++) {
             const int oy = y - 2 + k / 3, ox = x - 2 + k % 3;
             g[k / 3][k % 3] = (oy >= 0 && oy < ho && ox >= 0 && ox < wo) ? __ldg(src + oy * wo + ox) : 0.0f;
         }
 #pragma unroll
-        for (int k = 0; k < 9; k++) tap_fma<CI>(acc, g[2 - k / 3][2 - k % 3], g[3 - k / 3][2 - k % 3], W + (co * 9 + k) * CI);
+        for (int k = 0; k < 9; k++) {
+            float t[J];
+#pragma unroll
+            for (int j = 0; j < J; j++) t[j] = g[2 - k / 3 + j][2 - k % 3];
+            tap_fma(acc, t, W + (co * 9 + k) * CI);
+        }
     }
 #pragma unroll
     for (int ci = 0; ci < CI; ci++)
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
+        for (int j = 0; j < J; j++) {
             const size_t at = ((size_t)(nn * CI + ci) * h + y + j) * w + x;
             gin[at] = in[at] > 0.0f ? acc[j][ci] : 0.0f;
         }
@@ -227,7 +241,7 @@ __global__ void __launch_bounds__(128) conv_bwd_data_kernel(const float *gout, c
 // in a fixed order. Only output pixels inside the crop are multiplied: a tile's margin past it would cost time and turn an
 // infinite input into NaN in taps it has no part in. (One block per pair over every pixel, the form before, left 16 to 256
 // blocks walking 139 thousand pixels each: 335 us a layer on average, with the data gradients, against 52.)
-constexpr int kWgRows = 8, kWgCols = 36, kWgStride = 40;
+constexpr int kWgRows = kNetGradRows, kWgCols = kNetGradCols, kWgStride = 40;
 template <int CI, int CO>
 __global__ void __launch_bounds__(256) conv_bwd_weight_kernel(const float *gout, const float *in, int n, int h, int w,
                                                               float *parts, int woff, int boff)
@@ -366,7 +380,7 @@ __global__ void __launch_bounds__(256) net_loss_kernel(const float *z, const flo
 
 // The gradients from the blocks' parts, 32 parameters per block in a fixed order (warp g adds blocks g q .. g q + q - 1,
 // the 8 warps' sums are added in turn), then, with lr > 0, Adam's step on them.
-__global__ void __launch_bounds__(256) net_grads_kernel(const float *parts, float *P, float *R, float *G, float *M, float *V, float lr,
+__global__ void __launch_bounds__(256) net_grads_kernel(const float *parts, const int4 blocks, float *P, float *R, float *G, float *M, float *V, float lr,
                                                         float b1, float b2, float eps, int t)
 {
     constexpr int kPer = kNetGradBlocks / 8;
@@ -376,8 +390,13 @@ __global__ void __launch_bounds__(256) net_grads_kernel(const float *parts, floa
     float a = 0.0f;
     if (i < kNetParams) {
         const float *p = parts + (size_t)warp * kPer * kNetParams + i;
+        const int n = i < net_w(1) ? blocks.x : i < net_w(2) ? blocks.y : i < net_w(3) ? blocks.z : blocks.w;  // of i's layer
+        if (n == kNetGradBlocks) {
 #pragma unroll 8
-        for (int k = 0; k < kPer; k++) a += __ldg(p + (size_t)k * kNetParams);
+            for (int k = 0; k < kPer; k++) a += __ldg(p + (size_t)k * kNetParams);
+        } else {
+            for (int k = 0; k < min(kPer, n - warp * kPer); k++) a += __ldg(p + (size_t)k * kNetParams);
+        }
     }
     sum[warp][lane] = a;
     __syncthreads();
@@ -926,17 +945,29 @@ cudaError_t launch_net_features(const uint16_t *word, int w, int h, const int *x
     return after_launch();
 }
 
+namespace {
+// Whether the convolutions' threads make two pixels each: half the reads of the weights, but half the threads, each with
+// twice the work in a row. One pixel each is faster until the threads fill 4 (forward) or 8 (backward) blocks of an SM. Crops
+// of 72 x 72, one / two pixels a thread, forward: 16 crops 72 / 70 us, 28 crops 95 / 83; of 40 x 40, 32 crops 63 / 66.
+// Backward (with the weights): 16 crops 134 / 146, 28 crops 202 / 210, 32 crops 216 / 214. A whole step of one crop of
+// 24 x 24: 169 / 193 us (187 to 195 with one block per pair of channels for the weights).
+bool net_two_pixels(size_t pixels, int blocks) { return pixels > (size_t)148 * blocks * 128; }
+}  // namespace
+
 cudaError_t launch_net_forward(int layer, const float *in, int n, int h, int w, const float *params, float *out, cudaStream_t s)
 {
-    const size_t total = (size_t)(h - 2) / 2 * (w - 2) * n;
+    const size_t total = (size_t)(h - 2) * (w - 2) * n;
     if (!total) return cudaSuccess;
     LaunchTimer t("proposal_train_forward", s);
-    const unsigned g = (unsigned)((total + 127) / 128);
+    const bool two = net_two_pixels(total, 4);
+    const unsigned g = (unsigned)((total / (two ? 2 : 1) + 127) / 128);
+    const int wo = net_w(layer), bo = net_b(layer);
+    auto run = [&](auto kernel2, auto kernel1) { (two ? kernel2 : kernel1)<<<g, 128, 0, s>>>(in, n, h, w, params, wo, bo, layer < 3, out); };
     switch (layer) {
-    case 0: conv_fwd_kernel<2, 16><<<g, 128, 0, s>>>(in, n, h, w, params, net_w(0), net_b(0), true, out); break;
-    case 1: conv_fwd_kernel<16, 16><<<g, 128, 0, s>>>(in, n, h, w, params, net_w(1), net_b(1), true, out); break;
-    case 2: conv_fwd_kernel<16, 16><<<g, 128, 0, s>>>(in, n, h, w, params, net_w(2), net_b(2), true, out); break;
-    case 3: conv_fwd_kernel<16, 1><<<g, 128, 0, s>>>(in, n, h, w, params, net_w(3), net_b(3), false, out); break;
+    case 0: run(conv_fwd_kernel<2, 16, 2>, conv_fwd_kernel<2, 16, 1>); break;
+    case 1:
+    case 2: run(conv_fwd_kernel<16, 16, 2>, conv_fwd_kernel<16, 16, 1>); break;
+    case 3: run(conv_fwd_kernel<16, 1, 2>, conv_fwd_kernel<16, 1, 1>); break;
     default: return cudaErrorInvalidValue;
     }
     return after_launch();
@@ -946,23 +977,24 @@ cudaError_t launch_net_backward(int layer, const float *gout, const float *in, i
                                 float *gin, float *parts, cudaStream_t s)
 {
     LaunchTimer t("proposal_train_backward", s);
-    const unsigned g = (unsigned)(((size_t)h / 2 * w * n + 127) / 128);
+    const size_t total = (size_t)h * w * n;
+    const bool two = net_two_pixels(total, 8);
+    const unsigned g = (unsigned)((total / (two ? 2 : 1) + 127) / 128), gw = (unsigned)net_grad_blocks(n, h, w);
+    const int wo = net_w(layer), bo = net_b(layer);
+    auto data = [&](auto kernel2, auto kernel1) {
+        count_launch();
+        (two ? kernel2 : kernel1)<<<g, 128, 0, s>>>(gout, in, n, h, w, params, wo, gin);
+    };
     switch (layer) {
-    case 0: conv_bwd_weight_kernel<2, 16><<<kNetGradBlocks, 256, 0, s>>>(gout, in, n, h, w, parts, net_w(0), net_b(0)); break;
+    case 0: conv_bwd_weight_kernel<2, 16><<<gw, 256, 0, s>>>(gout, in, n, h, w, parts, wo, bo); break;
     case 1:
-        conv_bwd_weight_kernel<16, 16><<<kNetGradBlocks, 256, 0, s>>>(gout, in, n, h, w, parts, net_w(1), net_b(1));
-        count_launch();
-        conv_bwd_data_kernel<16, 16><<<g, 128, 0, s>>>(gout, in, n, h, w, params, net_w(1), gin);
-        break;
     case 2:
-        conv_bwd_weight_kernel<16, 16><<<kNetGradBlocks, 256, 0, s>>>(gout, in, n, h, w, parts, net_w(2), net_b(2));
-        count_launch();
-        conv_bwd_data_kernel<16, 16><<<g, 128, 0, s>>>(gout, in, n, h, w, params, net_w(2), gin);
+        conv_bwd_weight_kernel<16, 16><<<gw, 256, 0, s>>>(gout, in, n, h, w, parts, wo, bo);
+        data(conv_bwd_data_kernel<16, 16, 2>, conv_bwd_data_kernel<16, 16, 1>);
         break;
     case 3:
-        conv_bwd_weight_kernel<16, 1><<<kNetGradBlocks, 256, 0, s>>>(gout, in, n, h, w, parts, net_w(3), net_b(3));
-        count_launch();
-        conv_bwd_data_kernel<16, 1><<<g, 128, 0, s>>>(gout, in, n, h, w, params, net_w(3), gin);
+        conv_bwd_weight_kernel<16, 1><<<gw, 256, 0, s>>>(gout, in, n, h, w, parts, wo, bo);
+        data(conv_bwd_data_kernel<16, 1, 2>, conv_bwd_data_kernel<16, 1, 1>);
         break;
     default: return cudaErrorInvalidValue;
     }
@@ -977,11 +1009,13 @@ cudaError_t launch_net_loss(const float *z, const float *labels, int n, int ta, 
     return after_launch();
 }
 
-cudaError_t launch_net_grads(const float *parts, float *params, float *rounded, float *grads, float *m, float *v, float lr, float b1,
-                             float b2, float eps, int t, cudaStream_t s)
+cudaError_t launch_net_grads(const float *parts, int n, int h, int w, float *params, float *rounded, float *grads, float *m, float *v,
+                             float lr, float b1, float b2, float eps, int t, cudaStream_t s)
 {
     LaunchTimer tm("proposal_train_adam", s);
-    net_grads_kernel<<<(kNetParams + 31) / 32, 256, 0, s>>>(parts, params, rounded, grads, m, v, lr, b1, b2, eps, t);
+    const int4 blocks = make_int4(net_grad_blocks(n, h, w), net_grad_blocks(n, h - 2, w - 2), net_grad_blocks(n, h - 4, w - 4),
+                                  net_grad_blocks(n, h - 6, w - 6));
+    net_grads_kernel<<<(kNetParams + 31) / 32, 256, 0, s>>>(parts, blocks, params, rounded, grads, m, v, lr, b1, b2, eps, t);
     return after_launch();
 }
 

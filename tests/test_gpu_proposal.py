@@ -210,3 +210,26 @@ def test_an_infinite_input_reaches_only_the_taps_that_read_it(cuda, module, n, t
     hit[:16 * 2 * 9].reshape(16, 2, 3, 3)[:, 0, 2, 2] = True
     assert np.isfinite(grads[0]).all() and np.isnan(grads[1][hit]).all()
     assert np.array_equal(grads[1][~hit], grads[0][~hit])
+
+
+@pytest.mark.parametrize("n,th,tw", [(16, 4, 4), (40, 2, 5), (32, 4, 4)])
+def test_gradients_of_batches_around_two_pixels_a_thread(cuda, module, n, th, tw):
+    """The convolutions' threads make two pixels each in large batches: batches where the forward layers do and the backward
+    ones do not, and where both do. Tolerances as above."""
+    rng = np.random.default_rng(n)
+    h, w = 8 + 16 * th, 8 + 16 * tw
+    x = rng.normal(0, 1, (n, 2, h, w)).astype(np.float32)
+    labels = rng.normal(0.5, 0.5, (n, th, tw)).astype(np.float32)
+    params = random_params(7)
+    net = es_b200.ProposalNet(proposal.flatten(params))
+    xd, ld = to_dev(cuda, x), to_dev(cuda, labels)
+    loss, grads = net.train_step(xd.data_ptr(), ld.data_ptr(), n, h, w, 0.0, want_grads=True)
+    net.close()
+    want_loss, want = proposal.loss_and_grads(x.astype(np.float64), labels.astype(np.float64), params)
+    assert abs(loss - want_loss) <= 1e-5 * abs(want_loss)
+    at = 0
+    for gw, gb in want:
+        for g in (gw, gb):
+            got = grads[at:at + g.size].reshape(g.shape)
+            assert np.abs(got - g).max() <= 1e-3 * np.abs(g).max() + 1e-9
+            at += g.size
