@@ -86,6 +86,7 @@ struct es_batch {
     long queued[2] = {-1, -1};
     long next = 0, last_collected = -1;
     uint64_t graph_launches = 0;
+    bool unsettled = false;  // a step failed half-way (settle)
 
     // learned tile proposal (off while net is null)
     es_proposal_net *net = nullptr;
@@ -658,6 +659,19 @@ void queue_step(es_batch &b, long f, uint32_t skip)
     b.graph_launches++;
 }
 
+// After a step that failed half-way: what its kernels would have left clear (the digit counts of the top-k selection, the
+// squared errors and colors, the bin counts) is cleared, so that the same frame can be queued again. Everything else of a
+// step is written anew before it is read.
+void settle(es_batch &b)
+{
+    cudaStream_t s = b.main.s;
+    clear_selection(b.slots.ptr, (int)b.slots.count, s);
+    for (auto &S : b.sources) {
+        for (int i = 0; i < 2; i++) cuda_check(cudaMemsetAsync(S->sums[i].ptr, 0, S->sums[i].bytes(), s), "clearing");
+        cuda_check(cudaMemsetAsync(S->bin_n.ptr, 0, S->bin_n.bytes(), s), "clearing");
+    }
+}
+
 }  // namespace
 
 extern "C" {
@@ -736,17 +750,25 @@ int es_batch_queue(es_batch *b, long f, const es_frame_view *views, const int *c
         for (int s = 0; s < (int)b->sources.size(); s++)
             if (source_cambi && !source_cambi[s]) skip |= 1u << s;
         cudaStream_t caller = (cudaStream_t)stream;
-        cuda_check(cudaEventRecord(b->start.e, caller), "event");
-        cuda_check(cudaStreamWaitEvent(b->main.s, b->start.e, 0), "event");
-        cuda_check(cudaMemcpyAsync(b->views.ptr, b->h_views[at].ptr, sizeof(UnpackView) * P, cudaMemcpyHostToDevice, b->main.s),
-                   "input addresses");
-        if (b->net) {
-            b->h_frame[at].ptr[0] = (unsigned long long)f;
-            cuda_check(cudaMemcpyAsync(b->frame.ptr, b->h_frame[at].ptr, 8, cudaMemcpyHostToDevice, b->main.s), "frame number");
+        if (b->unsettled) settle(*b);
+        b->unsettled = true;
+        try {
+            cuda_check(cudaEventRecord(b->start.e, caller), "event");
+            cuda_check(cudaStreamWaitEvent(b->main.s, b->start.e, 0), "event");
+            cuda_check(cudaMemcpyAsync(b->views.ptr, b->h_views[at].ptr, sizeof(UnpackView) * P, cudaMemcpyHostToDevice, b->main.s),
+                       "input addresses");
+            if (b->net) {
+                b->h_frame[at].ptr[0] = (unsigned long long)f;
+                cuda_check(cudaMemcpyAsync(b->frame.ptr, b->h_frame[at].ptr, 8, cudaMemcpyHostToDevice, b->main.s), "frame number");
+            }
+            queue_step(*b, f, skip);
+            cuda_check(cudaEventRecord(b->done[at].e, b->main.s), "event");
+            cuda_check(cudaStreamWaitEvent(caller, b->done[at].e, 0), "event");
+        } catch (...) {  // nothing of it may run beside the next step, or after the caller's frames are gone
+            for (cudaStream_t s : {b->main.s, b->side.s, b->side2.s, b->aux.s}) wait_quietly(s);
+            throw;
         }
-        queue_step(*b, f, skip);
-        cuda_check(cudaEventRecord(b->done[at].e, b->main.s), "event");
-        cuda_check(cudaStreamWaitEvent(caller, b->done[at].e, 0), "event");
+        b->unsettled = false;
         b->skipped[at] = skip;
         b->queued[at] = f;
         b->next = f + 1;

@@ -11,6 +11,12 @@
 namespace es {
 const void *kernel_entry_cvalues();
 
+void clear_selection(CvSlot *slots, int n, cudaStream_t s)
+{
+    static_assert(offsetof(CvSlot, hist2) == offsetof(CvSlot, hist1) + sizeof(CvSlot::hist1) && sizeof(CvSlot::hist2) % 16 == 0, "one run of counts");
+    cuda_check(cudaMemset2DAsync(slots->hist1, sizeof(CvSlot), 0, sizeof(CvSlot::hist1) + sizeof(CvSlot::hist2), n, s), "clearing");
+}
+
 // A column's count of one code, at most the window's 2 pad + 1 rows, shares a word with three others; the c-value kernel
 // has a form for windows of up to 129 (5 k-steps of 32 columns).
 void check_cambi(int w, int h, int depth, const es_cambi_params &p)
@@ -42,6 +48,7 @@ struct es_cambi {
     float *planes[kScales] = {};
     unsigned long long *tile_mass = nullptr;
     bool pending = false, done = false;
+    bool unsettled = false;  // a launch failed half-way: the next one starts from cleared counts
 };
 
 namespace {
@@ -220,7 +227,19 @@ int es_cambi_launch(es_cambi *c, uint64_t img, int pitch, void *stream)
         require(img != 0, "es_cambi_launch: NULL plane");
         require(pitch >= c->w, "es_cambi_launch: pitch is smaller than the width");
         if (c->pending) throw Error(ES_ERR_STATE, "es_cambi_launch: the previous launch has not been finished");
-        queue_cambi(c, img, pitch, (cudaStream_t)stream);
+        if (c->unsettled) {
+            clear_selection(c->slots.ptr, kScales, c->stream.s);
+            cuda_check(cudaStreamSynchronize(c->stream.s), "cambi");
+        }
+        c->unsettled = true;
+        try {
+            queue_cambi(c, img, pitch, (cudaStream_t)stream);
+        } catch (...) {  // nothing of it may run beside the next launch, or after the caller's plane is gone
+            wait_quietly((cudaStream_t)stream);
+            wait_quietly(c->stream.s);
+            throw;
+        }
+        c->unsettled = false;
         c->pending = true;
     });
 }

@@ -124,6 +124,14 @@ struct Event {
     Event(const Event &) = delete;
 };
 
+// Waits for a stream after a failed call (errors are the failed call's to tell), unless it is being captured.
+inline void wait_quietly(cudaStream_t s)
+{
+    cudaStreamCaptureStatus st;
+    if (cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone) cudaStreamSynchronize(s);
+    cudaGetLastError();
+}
+
 // The current device must be an sm_100 part whose kernels load; throws ES_ERR_DEVICE otherwise.
 void check_device();
 
@@ -131,6 +139,8 @@ void check_device();
 es_cambi_params derive_params(int w, int h);
 // Throws ES_ERR_INVALID unless CAMBI's kernels take a w x h picture with these parameters.
 void check_cambi(int w, int h, int depth, const es_cambi_params &p);
+// Clears the digit counts that a slot's selection leaves clear (CvSlot::hist1, hist2) after one that was not finished.
+void clear_selection(CvSlot *slots, int n, cudaStream_t s);
 // lut[i] = 1/i as float for i < (2 pad + 1)^2 + 1, lut[0] = 0.
 void reciprocal_table(int pad, float *lut, size_t n);
 // src/cambi.cpp:29: clip((int)(topk * n), 1, n).

@@ -15,10 +15,13 @@ void count_launch();
 // Adds n (which may be negative) to the launch count: a graph replay counts its kernel nodes, a capture takes back
 // the launches its recording counted.
 void count_launches(long long n);
+// The launch that es_fail_launch asked to fail (once).
+bool launch_fails();
 inline cudaError_t after_launch()
 {
     count_launch();
-    return cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
+    return launch_fails() ? cudaErrorUnknown : e;
 }
 
 // Brackets a launcher's kernel launch with CUDA events on its stream while kernel timing is switched on

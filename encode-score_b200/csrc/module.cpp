@@ -16,9 +16,11 @@ namespace es {
 
 namespace {
 thread_local std::string g_last_error;
+thread_local int g_fail_launch = 0;
 std::atomic<unsigned long long> g_launches{0};
 }  // namespace
 
+bool launch_fails() { return g_fail_launch > 0 && --g_fail_launch == 0; }
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 void count_launches(long long n) { g_launches.fetch_add((unsigned long long)n, std::memory_order_relaxed); }
 
@@ -214,6 +216,14 @@ const char *es_last_error(void) { return g_last_error.c_str(); }
 int es_version(void) { return 10000; }
 
 uint64_t es_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
+
+int es_fail_launch(int n)
+{
+    return guarded([&] {
+        require(n >= 0, "es_fail_launch: n must be >= 0");
+        g_fail_launch = n;
+    });
+}
 
 int es_kernel_timing(int on)
 {

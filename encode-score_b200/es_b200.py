@@ -23,7 +23,7 @@ SCALES = 5
 
 # every symbol include/es_b200.h declares, for the load check
 SYMBOLS = (
-    "es_last_error", "es_version", "es_launch_count", "es_kernel_timing", "es_kernel_times", "es_module_load", "es_module_unload", "es_module_get", "es_module_launch",
+    "es_last_error", "es_version", "es_launch_count", "es_fail_launch", "es_kernel_timing", "es_kernel_times", "es_module_load", "es_module_unload", "es_module_get", "es_module_launch",
     "es_cambi_create", "es_cambi_create_with", "es_cambi_derive_params", "es_cambi_get_params", "es_cambi_launch",
     "es_cambi_finish", "es_cambi_destroy", "es_cambi_scale_stats", "es_cambi_read_scale", "es_cambi_set_cvalue_planes",
     "es_cambi_score_noalloc", "es_cambi_tile_count", "es_cambi_set_tile_mass", "es_cambi_scale_words",
@@ -133,6 +133,7 @@ def lib() -> ctypes.CDLL:
         P, I, U64 = ctypes.c_void_p, ctypes.c_int, ctypes.c_uint64
         L.es_last_error.restype = ctypes.c_char_p
         L.es_launch_count.restype = U64
+        L.es_fail_launch.argtypes = [I]
         L.es_kernel_timing.argtypes = [I]
         L.es_kernel_times.argtypes = [P, P, P, I, ctypes.POINTER(I)]
         L.es_module_load.argtypes = [ctypes.POINTER(P)]
@@ -218,6 +219,11 @@ def check(status: int) -> None:
 
 def launch_count() -> int:
     return int(lib().es_launch_count())
+
+
+def fail_launch(n: int) -> None:
+    """For tests: the n-th kernel this thread launches from now on is told as failed (0: none)."""
+    check(lib().es_fail_launch(n))
 
 
 def kernel_timing(on: bool, serial: bool = False) -> None:

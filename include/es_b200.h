@@ -40,6 +40,9 @@ int es_version(void);
 /* Diagnostics with no counterpart in the reference: the number of kernels this library has launched in this process
  * (all threads), so a caller can check how many GPU launches a piece of work took. */
 uint64_t es_launch_count(void);
+/* Diagnostics with no counterpart in the reference, for tests of what follows an error: the n-th kernel that the calling
+ * thread launches from now on runs but is told as failed (ES_ERR_CUDA from the call that launched it); 0 takes it back. */
+int es_fail_launch(int n);
 /* Diagnostics with no counterpart in the reference: with on != 0, each later kernel launch of the library is
  * bracketed by CUDA events on the stream it is launched on (and earlier totals are cleared); 0 stops it. With on == 2
  * the CAMBI work of es_cambi_launch and es_frame_queue also stays on the caller's stream instead of each instance's
