@@ -3,26 +3,23 @@
 // Some callers must not allocate device memory when they score a picture: plugins whose host application owns the
 // device memory budget, and latency-critical paths where cudaMalloc's implicit device synchronization is not
 // acceptable. This entry point runs the same kernels as es_cambi_launch / es_cambi_finish, but every buffer they use
-// -- the five scale planes, the per-scale lists of positive c-values, the counters and the reciprocal table -- lives
-// in one file-scope device array of kScratchBytes (20 MiB), which every GPU that loads the library holds until the
-// process exits. The caller passes the input plane and a device double for the output.
+// lives in two file-scope device arrays of 20 MiB together, which every GPU that loads the library holds until the
+// process exits: the five scale planes, the per-scale lists of c-values and the reciprocal table in g_scratch, the
+// counters in g_slots. The caller passes the input plane and a device double for the output.
 //
-// Host code cannot use the array's name as a device address (in host code it names a host-side stand-in). A device
+// Host code cannot use an array's name as a device address (in host code it names a host-side stand-in). A device
 // symbol's address belongs to a CUDA context, and a program may call from more than one context on a device (the
-// primary one, or one it made with cuCtxCreate), so every call looks the address up again with cudaGetSymbolAddress in
+// primary one, or one it made with cuCtxCreate), so every call looks the addresses up again with cudaGetSymbolAddress in
 // the context current on the calling thread, and every call rewrites the reciprocal table in its first kernel: no
 // address or table state is kept on the host. A context's first call may load the library's kernels into it, so make
-// it before any stream capture. Every call shares the array: each call clears what must start at zero, and calls whose
+// it before any stream capture. Every call shares the arrays: each call clears what must start at zero, and calls whose
 // work overlaps on the GPU race.
 #include "es_internal.h"
 
 namespace es {
 namespace {
 
-constexpr size_t kScratchBytes = (size_t)20 << 20;
-// What the array holds before the planes: pictures are refused by what 20 MiB leave beside it. (The counters have an
-// array of their own.)
-constexpr size_t kScratchHead = 82432;
+constexpr size_t kScratchBytes = ((size_t)20 << 20) - 82432;  // with the counters about 20 MiB; pictures that need more are refused
 constexpr int kNoAllocMaxPad = 32;                                                  // windows up to 65
 constexpr int kLutEntries = (2 * kNoAllocMaxPad + 1) * (2 * kNoAllocMaxPad + 1) + 1;  // 4226
 
@@ -39,7 +36,7 @@ struct Carve {
 Carve carve(int w, int h)
 {
     Carve c{};
-    size_t at = kScratchHead;
+    size_t at = 0;
     c.score = at;
     at = align256(at + (1 + kScales) * sizeof(double));
     c.lut = at;

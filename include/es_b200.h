@@ -45,8 +45,8 @@ uint64_t es_launch_count(void);
 int es_fail_launch(int n);
 /* Diagnostics with no counterpart in the reference: with on != 0, each later kernel launch of the library is
  * bracketed by CUDA events on the stream it is launched on (and earlier totals are cleared); 0 stops it. With on == 2
- * the CAMBI work of es_cambi_launch and es_frame_queue also stays on the caller's stream instead of each instance's
- * own, so kernels run one at a time and each event pair times one kernel alone. */
+ * the work of es_cambi_launch stays on the caller's stream and that of es_frame_queue and es_batch_queue on one stream of
+ * the object's, so kernels run one at a time and each event pair times one kernel alone. */
 int es_kernel_timing(int on);
 /* Waits for the device, then writes per kernel (up to `max` kernels): its name in names[32 i .. 32 i + 31]
  * (NUL-terminated), the summed event time in total_ms[i] and the number of timed launches in launches[i];
@@ -121,14 +121,14 @@ int es_cambi_scale_words(const es_cambi *c, int s, uint64_t *address);
 /* No counterpart in the reference. The CAMBI score of one plane, like es_cambi_create + es_cambi_launch +
  * es_cambi_finish, for callers that must not allocate device memory when they score a picture: plugins whose host
  * application owns the device memory budget, and latency-critical paths where cudaMalloc's implicit device
- * synchronization is not acceptable. It allocates nothing: its scratch is one fixed 20 MiB device array inside the
+ * synchronization is not acceptable. It allocates nothing: its scratch is 20 MiB of fixed device arrays inside the
  * library, which every GPU that loads the library holds until the process exits, so it takes pictures up to about
  * 1920 x 1080 (larger ones fail with ES_ERR_INVALID and the size they would need). `img` is a device plane of w x h
  * values at `depth` bits (8 or 10), `pitch` in pixels; the score is written to the device double `score`; all work is
  * queued on `stream` and the call returns without waiting. It runs in the CUDA context current on the calling thread
- * (the primary context, or one made with cuCtxCreate): each call looks the array's address up in that context and
+ * (the primary context, or one made with cuCtxCreate): each call looks the arrays' addresses up in that context and
  * rewrites its reciprocal table, so nothing is cached across contexts or device resets. A context's first call may
- * load the library's kernels into it, so it should come before any stream capture. Every call shares the array: calls
+ * load the library's kernels into it, so it should come before any stream capture. Every call shares the arrays: calls
  * whose work overlaps on the GPU race, so serialize them (one stream, or events). */
 int es_cambi_score_noalloc(uint64_t img, int pitch, int w, int h, int depth, double *score, void *stream);
 
@@ -261,8 +261,8 @@ int es_to_pictures(const es_picture_copy *copies, int n, void *stream);
 /* ---------------------------------------------------------------------------------------------------------------
  * Texture window energies on larger windows, in three arithmetics (the precision study; no counterpart in the
  * reference, which sums FP32 box means over fixed 16 x 16 windows, src/kernels.cu:331-428). The 3 x 3 and 9 x 9 box
- * sums (edge pixels repeated) come from summed-area tables of each luma plane kept as int64, as FP32 with two-sum
- * compensation, and as plain FP32; pixel terms and their per-16 x 16-block sums follow in the same arithmetic (exact
+ * sums (edge pixels repeated) are made exactly from the pixels as integers, and from summed-area tables of each luma
+ * plane in FP32 with two-sum compensation and in plain FP32; pixel terms and their per-16 x 16-block sums follow in the same arithmetic (exact
  * int64 numerators; Neumaier-compensated FP32; plain FP32). A window of side 16 k sums k x k blocks and gives the
  * 8 figures of src/kernels.cu:340-341 (windows x 8 doubles, window (x, y) at index y * (w / window) + x).
  * --------------------------------------------------------------------------------------------------------------- */
@@ -270,7 +270,7 @@ typedef struct es_windows es_windows;
 int es_windows_create(int w, int h, es_windows **out);
 /* src / enc: device luma planes (w x h uint16 at the pipeline depth); up = 10 - depth (0 or 2). */
 int es_windows_compute(es_windows *p, uint64_t src, uint64_t enc, int up, void *stream);
-/* mode 0: integer tables (exact, rounded once to double); 1: compensated FP32; 2: plain FP32. out: device doubles. */
+/* mode 0: integers (exact, rounded once to double); 1: compensated FP32; 2: plain FP32. out: device doubles. */
 int es_windows_figures(es_windows *p, int window, int mode, double *out, void *stream);
 void es_windows_destroy(es_windows *p);
 

@@ -213,3 +213,18 @@ def test_pictures_whose_window_is_too_wide_are_refused(what, w, h, refused):
         assert status == es_b200.ES_ERR_INVALID and b"at most 129" in lib.es_last_error()
     else:
         assert status not in (es_b200.ES_OK, es_b200.ES_ERR_INVALID)
+
+
+@pytest.mark.parametrize("w,h", [(1920, 1360), (1280, 2040), (720, 3626)])
+def test_the_largest_pictures_of_the_no_allocation_call(w, h):
+    """What its fixed arrays hold, to the row: the refusal comes before the device is looked for."""
+    lib = es_b200.lib()
+    import torch
+
+    out = ctypes.c_double()
+    for rows, fits in ((h, True), (h + 1, False)):
+        if fits and torch.cuda.is_available():
+            continue  # (the plane is not one)
+        status = lib.es_cambi_score_noalloc(1, w, w, rows, 10, ctypes.addressof(out), None)
+        told = lib.es_last_error()
+        assert (b"bytes of scratch" not in told) == fits and (status == es_b200.ES_ERR_INVALID or fits), (rows, told)

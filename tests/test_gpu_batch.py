@@ -257,3 +257,23 @@ def test_large_batch_of_listed_tiles_equals_frames_of_their_own(cuda, module, de
             assert (r.cambi, r.cambi_source) == got[f][s], (s, f)
         fr.close()
     assert max(max(c) for c in got[0]) > 0 and min(min(c) for c in got[0]) == 0
+
+
+@pytest.mark.parametrize("rows", [[16, 64, 32, 0, 64], [16, 16, 64, 32, 0], [0, 32, 64, 64, 16]])
+def test_rows_of_listed_tiles_change_no_result(cuda, module, rows):
+    """Steps that list their busy tiles (over 4096 of them) with tiles of 16, 32 and 64 rows at different scales, some left
+    to the library, against the library's choice throughout; the strips the list is made from stay 8 and 4 rows high."""
+    sizes = [(256, 192), (390, 202), (318, 142), (446, 136)] * 8
+    stream = cuda.cuda.current_stream().cuda_stream
+    keep, views = [], []
+    for s, (w, h) in enumerate(sizes):
+        k, sv, ev = step_to_dev(cuda, es_b200, es_synth.c3_step(0, s, w, h, 10))
+        keep.append(k)
+        views += [sv] + ev
+    got = []
+    for tuning in (False, {size: rows for size in sizes}):
+        b = es_b200.Batch(module, [(w, h, 10, 1) for w, h in sizes], tuning=tuning)
+        b.queue(0, views, stream)
+        got.append([(r.cambi, r.cambi_source) for r in b.collect(0)])
+        b.close()
+    assert got[0] == got[1] and max(c[0] for c in got[0]) > 0
