@@ -2,15 +2,16 @@
 //
 // The reference scores one source per process, with one launch per kernel and picture and a host round trip per
 // top-k radix round (src/main.cpp:518-643, src/cambi.cpp:88-184). Here a frame step of every source is one launch per
-// stage for all pictures: unpacking, scale 0, the decimation of each scale, the c-values of every scale of every
-// picture, the top-k rounds of every slot and the scores form one chain; PSNR / color, window figures, lasting texture
-// and the per-frame reduction of every source form a second chain that runs beside it. Once a source's rings are full
+// stage for all pictures: unpacking, scales 0 and 1, scales 2 to 4, the c-values of every scale of every picture, the
+// top-k rounds of every slot and the scores form one chain; PSNR / color, window figures, lasting texture and the
+// per-frame reduction of every source form a second chain that runs beside it. Once a source's rings are full
 // (frame 14 on), a step is replayed from a CUDA graph captured per ring phase, so queueing a step costs one small copy
 // of the input addresses and one graph launch.
 //
 // Per source the device state is that of es_frame (luma rings, running texture sums, structure masks, figures); per
-// picture the CAMBI state is one word plane and one positive c-value list per scale. The figures of step f are copied
-// to page-locked memory indexed by f % 2, so collect(f) reads them while step f + 1 runs.
+// picture the CAMBI state is one word plane and one c-value list per scale. The last kernels of step f write its scores
+// and figures to page-locked memory indexed by f % 2, so collect(f) reads them while step f + 1 runs, and clear the counts
+// that they have read: those are clear when a step begins.
 #include <cstring>
 #include <map>
 #include <memory>
@@ -251,7 +252,7 @@ uint16_t *luma_of(const es_batch &b, int picture, long f)
 // and audited tiles, the audit, then the skipped tiles of the pictures whose audit asks for the fallback. `run` lists
 // the pictures whose CAMBI runs; cb is the step's c-value job table (scales 0-4 of each, in that order).
 // The proposal of a step up to its tile lists: features come with scale 0, then the prediction, the optional budget
-// and the lists. Needs scale 0 only, so it runs beside the decimation of scales 1-4. Returns the audit's table.
+// and the lists. Needs scale 0 only, so it runs beside the decimation of scales 2-4. Returns the audit's table.
 AuditBatch record_proposal_lists(es_batch &b, const std::vector<int> &run, CvBatch &cb, cudaStream_t s)
 {
     const int np = (int)run.size();

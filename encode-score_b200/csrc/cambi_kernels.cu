@@ -12,8 +12,8 @@
 //  * two launches of select_kernel and the score kernel find the exact k-th largest value, and the sum above it, on the
 //    device when more than k values are positive (no host round trips; the first radix digit is counted by the c-value
 //    kernel); the score kernel also pools and weights the scales and writes the score to the host's memory.
-// A picture is five launches after the last one's input is there. They were twelve and a copy: a launch takes 2.5 to 5 us
-// of host time and 3 to 5 us on the GPU here, as long as the work of most of them.
+// A picture is six launches: scales 0 and 1, scales 2-4, the c-values, two top-k rounds, the score. They were twelve and a
+// copy: a launch takes 2.5 to 5 us of host time and 3 to 5 us on the GPU here, as long as the work of most of them.
 #include "cambi_codes.h"
 #include "es_kernels.h"
 

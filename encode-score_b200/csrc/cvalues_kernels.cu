@@ -632,7 +632,9 @@ __device__ __forceinline__ void tile_cvalues(const CvBatch &b, const CvJob &J, c
     }
 }
 
-// kMaxN: the most k-steps of a job of the launch (3 covers pads up to 32, pictures up to 4K; 5 every pad).
+// kMaxN: the most k-steps of a job of the launch (3 covers pads up to 32, w + h up to 6092; 5 every pad). Above pad 32 a block's
+// buffers take 87 KB and more, so two share an SM whatever its registers. Launch to finished score, the block-wide form / this
+// one: 4096x2160 10-bit dense (pad 33) 815 / 455 us, 5120x2880 (43) 1437 / 724, 7680x4318 (64) 3730 / 1732.
 template <int kMaxN>
 __global__ void __launch_bounds__(kCvThreads, kMaxN == 3 ? 3 : 2) cvalues_kernel(const __grid_constant__ CvBatch b)
 {

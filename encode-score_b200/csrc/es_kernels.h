@@ -52,8 +52,9 @@ constexpr int kWin = 16;               // detail window side (src/kernels.cu:331
 #ifdef __CUDACC__
 // A launch that is made ready while the kernel before it on the stream runs, and begins when that kernel's last block leaves
 // (programmatic dependent launch): `kernel` calls wait_for_previous() before it reads or writes memory, and what comes
-// before the launch on the stream is a kernel. CAMBI of one 640x360 picture 77 -> 68 us, of 1920x1080 121 -> 112; a step of
-// a 1920x1080 pair, whose kernels are launched one by one, 160 -> 152 us.
+// before the launch on the stream is a kernel. Launch to finished score through Python, in the build that brought it: CAMBI
+// of one 640x360 picture 77 -> 68 us, of 1920x1080 121 -> 112; a step of a 1920x1080 pair, whose kernels are launched one
+// by one, 160 -> 152 us.
 // chained = false: a plain launch.
 template <typename... P, typename... A>
 cudaError_t launch_kernel(bool chained, void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, const A &...args)
@@ -106,7 +107,8 @@ struct Band {
 // Per picture-scale counters in device memory. The c-values are exact multiples of 2^-24 (they are at least 0.5), so
 // their sum is kept exactly as an integer in those units; the order of additions does not matter.
 // The c-value kernel also counts the positive values by the top 11 bits of their floats (the first radix digit of the
-// top-k selection): at least 0.5 and below 2^13, so those digits lie in kCvDigit0 .. kCvDigit0 + 55.
+// top-k selection): at least 0.5 and, for windows of up to 129 and weights of up to 4, below 2^15 (4 x 129^2 / 4 = 16641 at
+// most), so those digits lie in kCvDigit0 .. kCvDigit0 + 60; larger ones, of other weights, are counted one by one.
 constexpr unsigned kCvDigit0 = 0x3F000000u >> 21, kCvDigits = 64;
 struct CvSlot {
     unsigned long long sum_fx, count;  // positive c-values: sum in 2^-24 units, number
@@ -213,9 +215,9 @@ struct CvBatch {
     int need_first, need_last;   // set by the launcher: the least and greatest needed value
 };
 // A launch of at least this many tiles lists its busy tiles first (CvBatch::busy). Most tiles of most pictures need no
-// c-value, but a block of their own costs 2 to 4 us of a place on an SM to find that out: 16 uneven pairs (26.6 thousand
-// tiles) took 706 us and take 588, a step of a 3840 x 2160 pair (5.5 thousand) 388 and 375; below, the launch more costs what it
-// saves: a step of a 1920 x 1080 pair (2.3 thousand) 170 and 173.
+// c-value, but a block of their own costs 2 to 4 us of a place on an SM to find that out. Without and with the list, in the
+// build that brought it: 16 uneven pairs (26.6 thousand tiles) 706 and 588 us of c-values, a step of a 3840 x 2160 pair (5.5
+// thousand) 388 and 375; below, the launch more costs what it saves: a step of a 1920 x 1080 pair (2.3 thousand) 170 and 173.
 constexpr int kCvBusyTiles = 4096;
 // Blocks of a tile-list launch.
 constexpr int kCvListBlocks = 148 * 3;
@@ -228,7 +230,9 @@ inline int cv_tiles(int w, int h) { return ((w + kCvTX - 1) / kCvTX) * ((h + kCv
 // done sooner, which decides where the tiles do not fill the chip's 444 places or hold many ranks (several passes),
 // as the small scales' do. Measured, c-values of one picture, 64 rows everywhere / by this rule: 640x360 8-bit 55 / 24
 // us, 1920x1080 8-bit 96 / 57 us, 3840x2160 10-bit 190 / 108 us; 32 rows for scale 1 of a dense 4K picture instead of 64:
-// 260 against 247 us, 64 rows for scale 0 of the 1080p one instead of 32: 69 against 57 us.
+// 260 against 247 us, 64 rows for scale 0 of the 1080p one instead of 32: 69 against 57 us. The line at 592 tiles was drawn
+// from these three; just above it 64 rows are too many: a 1920x800 pair (780 tiles) takes 36 us, with 32 rows at scale 0 29
+// us, with the autotuned rows 28.
 inline int cv_default_tile_rows(int w, int h, int tiles0)
 {
     const int tiles = cv_tiles(w, h);

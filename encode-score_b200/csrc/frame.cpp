@@ -5,8 +5,9 @@
 // frame's figures are read from comes in two, used by f % 2.
 //
 // It had one CAMBI instance per picture and parity, each with its own chain of launches: 31 launches and 242 us a frame of
-// one 1080p encode, now 13 launches and 192 us. The steps are launched, not replayed from graphs: replays take 183 us
-// here, but capturing a frame's graph takes another 170 us in each of the first 14 ring phases.
+// one 1080p encode, as a batch 13 launches and 192 us (152 since, with faster kernels). The steps are launched, not replayed
+// from graphs: replays took 183 us then, but capturing a frame's graph takes another 170 us in each of the first 14 ring
+// phases.
 #include <cmath>
 #include <cstring>
 #include <memory>
