@@ -233,3 +233,27 @@ def test_gradients_of_batches_around_two_pixels_a_thread(cuda, module, n, th, tw
             got = grads[at:at + g.size].reshape(g.shape)
             assert np.abs(got - g).max() <= 1e-3 * np.abs(g).max() + 1e-9
             at += g.size
+
+
+@pytest.mark.parametrize("n,th,tw", [(1, 2, 2), (4, 2, 2), (2, 4, 4)])
+def test_gradients_of_a_flat_crop_round_like_short_chains(cuda, module, n, th, tw):
+    """On a flat crop every product of a tap is the same number and additions in one long chain all round the same way. The
+    network passes its first input through (middle taps 1), input, labels and number of tiles are such that everything up to
+    the products is exact in FP32, so a gradient's only errors are its additions': 36 products in a row at most, then
+    FP64 and three roundings to FP32 on the way, 40 half-steps of 2^-23 in all."""
+    h, w = 8 + 16 * th, 8 + 16 * tw
+    c, d = 507 / 512, 15347 / 16384
+    params = [(np.zeros_like(a), np.zeros_like(b)) for a, b in random_params(1)]
+    for weights, _ in params:
+        weights[0, 0, 1, 1] = 1.0
+    x = np.zeros((n, 2, h, w), np.float32)
+    x[:, 0] = c
+    labels = np.full((n, th, tw), c - d, np.float32)
+    net = es_b200.ProposalNet(proposal.flatten(params))
+    xd, ld = to_dev(cuda, x), to_dev(cuda, labels)
+    _, grads = net.train_step(xd.data_ptr(), ld.data_ptr(), n, h, w, 0.0, want_grads=True)
+    net.close()
+    _, want = proposal.loss_and_grads(x.astype(np.float64), labels.astype(np.float64), params)
+    want = np.concatenate([g.ravel() for pair in want for g in pair])
+    assert want.min() >= 0 and (want > 0).sum() >= 40
+    assert (np.abs(np.array(grads, np.float64) - want) <= 40 * 2.0 ** -24 * want).all()
