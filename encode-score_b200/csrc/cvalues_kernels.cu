@@ -739,7 +739,11 @@ template <int kMaxN>
 cudaError_t launch_cvalues_n(CvBatch &b, cudaStream_t s)
 {
     const size_t smem = cvalues_smem_bytes(b.max_pad);
-    cudaError_t e = cudaFuncSetAttribute(cvalues_kernel<kMaxN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the most a launch of this form takes, not this launch's size: the attribute is the kernel's, and another thread's
+    // smaller picture may set it between here and the launch
+    static_assert(cv_ksteps(32) == 3 && cv_ksteps(kMaxPad) == 5, "the pads of the two forms");
+    cudaError_t e = cudaFuncSetAttribute(cvalues_kernel<kMaxN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)cvalues_smem_bytes(kMaxN == 3 ? 32 : kMaxPad));
     if (e != cudaSuccess) return e;
     LaunchTimer t("cambi_cvalues", s);
     if (!b.tiles && b.busy) {

@@ -168,3 +168,40 @@ def test_bad_sizes_are_refused(cuda, module):
     p.window, p.pad = 131, 65
     with pytest.raises(es_b200.EsError):
         es_b200.Cambi(module, 100, 100, 10, p)
+
+
+def test_pictures_of_different_windows_from_several_threads(cuda, module):
+    """Eight threads score pictures whose windows, and so whose blocks' shared memory, differ: each gets its own scores."""
+    import threading
+
+    sizes = [(320, 180), (640, 360), (960, 540), (1280, 720), (1600, 900), (1920, 1080), (2560, 1440), (3200, 1800)]
+    planes = [to_dev(cuda, banded(w, h, 7, step=4)) for w, h in sizes]
+    instances = [es_b200.Cambi(module, w, h, 10) for w, h in sizes]
+    streams = [cuda.cuda.Stream() for _ in sizes]
+    cuda.cuda.synchronize()
+
+    def score(k):
+        instances[k].launch(planes[k].data_ptr(), sizes[k][0], streams[k].cuda_stream)
+        return instances[k].finish()
+
+    want = [score(k) for k in range(len(sizes))]
+    wrong, start = [], threading.Barrier(len(sizes))
+
+    def caller(k):
+        start.wait()
+        for _ in range(300):
+            try:
+                got = score(k)
+            except es_b200.EsError as e:
+                got = str(e)
+            if got != want[k]:
+                wrong.append((k, got))
+
+    threads = [threading.Thread(target=caller, args=(k,)) for k in range(len(sizes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for c in instances:
+        c.close()
+    assert not wrong, (len(wrong), wrong[:3])
