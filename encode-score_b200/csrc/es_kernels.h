@@ -33,8 +33,8 @@ struct LaunchTimer {
     ~LaunchTimer();
     LaunchTimer(const LaunchTimer &) = delete;
 };
-// True while es_kernel_timing(2) is in force: CAMBI instances then queue all their work on the caller's stream, so
-// that nothing runs beside a timed kernel and its events bracket that kernel alone.
+// True while es_kernel_timing(2) is in force: CAMBI instances then queue all their work on the caller's stream and frame
+// steps theirs on one stream, so that nothing runs beside a timed kernel and its events bracket that kernel alone.
 bool serial_streams();
 // True while es_kernel_timing is on (its events need plain launches, so graphs are not used then).
 bool kernel_timing_on();

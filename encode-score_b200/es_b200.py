@@ -227,8 +227,8 @@ def fail_launch(n: int) -> None:
 
 
 def kernel_timing(on: bool, serial: bool = False) -> None:
-    """Brackets each later kernel launch with CUDA events; with serial=True the CAMBI work also stays on the caller's
-    stream, so each event pair times one kernel running alone."""
+    """Brackets each later kernel launch with CUDA events; with serial=True a call's work also stays on one stream, so each
+    event pair times one kernel running alone."""
     check(lib().es_kernel_timing(2 if (on and serial) else int(bool(on))))
 
 
